@@ -1131,15 +1131,15 @@ int msplat_cuda_knn3_mean_dist(msplat_cuda_ctx *ctx, const float *points, uint32
     if (n == 0) return MSPLAT_CUDA_OK;
     if (!points || !mean_dist) return fail(MSPLAT_CUDA_EINVAL, "null buffer");
     if (n > (uint32_t)INT32_MAX) return fail(MSPLAT_CUDA_EINVAL, "too many points");
-    const int nb = knn_boxes((int)n);
+    const int nodes = knn_nodes((int)n);
     ENSURE(ctx->k_bounds, 8, unsigned int, bounds);
-    ENSURE(ctx->keys[0], n, uint64_t, k0);
-    ENSURE(ctx->keys[1], n, uint64_t, k1);
+    ENSURE(ctx->keys[0], n, uint32_t, k0);
+    ENSURE(ctx->keys[1], n, uint32_t, k1);
     ENSURE(ctx->vals[0], n, uint32_t, v0);
     ENSURE(ctx->vals[1], n, uint32_t, v1);
     ENSURE(ctx->radix_scratch, radix_scratch_bytes((int)n), unsigned char, rs);
     ENSURE(ctx->k_sorted, n, float4, sorted);
-    ENSURE(ctx->k_box, 2 * (size_t)nb, float4, boxes);
+    ENSURE(ctx->k_box, 2 * (size_t)nodes, float4, boxes);
     ENSURE(ctx->k_evals, 1, unsigned long long, evals);
     KnnScratch s;
     s.evals = evals;
@@ -1151,7 +1151,7 @@ int msplat_cuda_knn3_mean_dist(msplat_cuda_ctx *ctx, const float *points, uint32
     s.radix_scratch = rs;
     s.sorted = sorted;
     s.bmin = boxes;
-    s.bmax = boxes + nb;
+    s.bmax = boxes + nodes;
     launch_knn3(points, (int)n, mean_dist, s, ctx->stream);
     CUDA_TRY(cudaGetLastError());
     return MSPLAT_CUDA_OK;

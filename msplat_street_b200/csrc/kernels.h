@@ -346,13 +346,15 @@ void launch_needle_cap(float *scales, int n, float log_max, cudaStream_t st);
 
 struct KnnScratch {
     unsigned int *bounds;  // 6 ordered-bit floats: min xyz, max xyz
-    uint64_t *keys[2];
+    uint32_t *keys[2];
     uint32_t *vals[2];
     void *radix_scratch;
-    float4 *sorted, *bmin, *bmax;
+    float4 *sorted;
+    float4 *bmin, *bmax;  // knn_nodes(n) bounds each: boxes, groups, supergroups
     unsigned long long *evals;  // (may be null) point distances the search computed
 };
 int knn_boxes(int n);
+int knn_nodes(int n);  // boxes, groups and supergroups
 int launch_knn3(const float *pts, int n, float *out, KnnScratch &s, cudaStream_t st);
 void launch_init_gaussians(const float *md, const uint8_t *rgb, int n, uint32_t seed, float logit, float *scales,
                            float *quats, float *dc, float *opac, cudaStream_t st);

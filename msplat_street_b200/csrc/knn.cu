@@ -4,13 +4,16 @@
 // Metal backend sorts by Morton code and culls by box distance) returns, for every
 // point, the mean distance to its 3 nearest OTHER points (fewer if n < 4, 1.0 if
 // none). Here points are sorted by a 30-bit Morton code with the device radix sort and
-// cut into boxes of 32 consecutive points. One warp answers one box's 32 queries: its
-// lanes test 32 candidate boxes at a time, nearest Morton neighbours first, against
-// the query box's bounds; a box survives only if its lower-bound squared distance is
-// below the warp's worst current third-best, then its 32 points are streamed through
-// the warp with shuffles. The lower bound uses the same float subtractions and
-// squares as the point distances, and float rounding is monotonic, so a pruned box
-// can hold no point that would enter a lane's best three: the result is exact.
+// cut into boxes of 32 consecutive points, groups of 32 boxes and supergroups of 32
+// groups, each with its bounds. One warp answers one box's 32 queries: it searches its
+// own box, the rest of its own group, then every other group, descending from the
+// supergroups; its lanes test 32 nodes of a level at a time against the query box's
+// bounds, and a node survives only if its lower-bound squared distance is below the
+// warp's worst third-best so far. A surviving box is tested once more by every query
+// for itself before its 32 points are read. The lower bounds use the same float
+// subtractions and squares as the point distances, and float rounding is monotonic, so
+// a pruned node can hold no point that would enter a lane's best three: the result is
+// exact, whatever the order of the search.
 //
 // msplat_init_gaussians (:1582-1605): isotropic log-scale log(max(d, 1e-7)), a
 // uniformly random rotation from three PCG uniforms (Shoemake), DC colour from RGB
@@ -30,7 +33,12 @@ __device__ __forceinline__ float from_ordered(unsigned int u) {
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-__global__ void knn_bounds_kernel(const float *pts, int n, unsigned int *bb) {
+constexpr int KNN_BOUNDS_THREADS = 512;
+
+// One atomic per block and bound: with one per warp, the 57 k atomics of a 400 k-point
+// cloud on six addresses took 38 us.
+__global__ void __launch_bounds__(KNN_BOUNDS_THREADS) knn_bounds_kernel(const float *pts, int n, unsigned int *bb) {
+    __shared__ unsigned int part[6][KNN_BOUNDS_THREADS / 32];
     unsigned int mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         for (int a = 0; a < 3; a++) {
@@ -40,16 +48,22 @@ __global__ void knn_bounds_kernel(const float *pts, int n, unsigned int *bb) {
             mn[a] = min(mn[a], o);
             mx[a] = max(mx[a], o);
         }
-    for (int a = 0; a < 3; a++) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-            mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
+    for (int a = 0; a < 3; a++) {
+        const unsigned int lo = __reduce_min_sync(0xffffffffu, mn[a]), hi = __reduce_max_sync(0xffffffffu, mx[a]);
+        if (lane == 0) {
+            part[a][warp] = lo;
+            part[3 + a][warp] = hi;
         }
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&bb[a], mn[a]);
-            atomicMax(&bb[3 + a], mx[a]);
-        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int a = threadIdx.x;
+        unsigned int r = part[a][0];
+        for (int w = 1; w < KNN_BOUNDS_THREADS / 32; w++) r = a < 3 ? min(r, part[a][w]) : max(r, part[a][w]);
+        if (a < 3) atomicMin(&bb[a], r);
+        else atomicMax(&bb[a], r);
     }
 }
 
@@ -62,7 +76,7 @@ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
     return v;
 }
 
-__global__ void knn_morton_kernel(const float *pts, int n, const unsigned int *bb, uint64_t *keys, uint32_t *vals) {
+__global__ void knn_morton_kernel(const float *pts, int n, const unsigned int *bb, uint32_t *keys, uint32_t *vals) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t q[3];
@@ -74,7 +88,7 @@ __global__ void knn_morton_kernel(const float *pts, int n, const unsigned int *b
         t = fminf(fmaxf(t, 0.f), 1.f);
         q[a] = (uint32_t)(t * 1023.f);
     }
-    keys[i] = (uint64_t)(spread10(q[0]) | (spread10(q[1]) << 1) | (spread10(q[2]) << 2));
+    keys[i] = spread10(q[0]) | (spread10(q[1]) << 1) | (spread10(q[2]) << 2);
     vals[i] = (uint32_t)i;
 }
 
@@ -85,27 +99,72 @@ __global__ void knn_gather_kernel(const float *pts, int n, const uint32_t *order
     sp[j] = make_float4(pts[3 * (size_t)i], pts[3 * (size_t)i + 1], pts[3 * (size_t)i + 2], __uint_as_float(i));
 }
 
-__global__ void knn_boxes_kernel(const float4 *sp, int n, int nboxes, float4 *bmin, float4 *bmax) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nboxes) return;
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    const int end = min(n, (b + 1) * KNN_BOX);
-    for (int j = b * KNN_BOX; j < end; j++) {
-        const float4 p = sp[j];
-        const float c[3] = {p.x, p.y, p.z};
-        for (int a = 0; a < 3; a++)
-            if (isfinite(c[a])) {
-                lo[a] = fminf(lo[a], c[a]);
-                hi[a] = fmaxf(hi[a], c[a]);
-            }
-    }
-    bmin[b] = make_float4(lo[0], lo[1], lo[2], 0.f);
-    bmax[b] = make_float4(hi[0], hi[1], hi[2], 0.f);
+// Bounds over a warp's lanes, on every lane.
+struct Bounds {
+    float lo[3], hi[3];
+};
+__device__ __forceinline__ void warp_bounds(Bounds &b) {
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            b.lo[a] = fminf(b.lo[a], __shfl_xor_sync(0xffffffffu, b.lo[a], o));
+            b.hi[a] = fmaxf(b.hi[a], __shfl_xor_sync(0xffffffffu, b.hi[a], o));
+        }
+}
+__device__ __forceinline__ void store_bounds(float4 *mn, float4 *mx, int i, const Bounds &b) {
+    mn[i] = make_float4(b.lo[0], b.lo[1], b.lo[2], 0.f);
+    mx[i] = make_float4(b.hi[0], b.hi[1], b.hi[2], 0.f);
 }
 
-// best[0] <= best[1] <= best[2] (core/cpu/msplat_cpu.cpp:1522-1531)
+// One block per group: each warp takes one of its boxes, a lane per point, and warp 0
+// the group's bounds from the warps'. Non-finite coordinates bound nothing.
+__global__ void __launch_bounds__(KNN_BOX * KNN_BOX) knn_boxes_kernel(const float4 *sp, int n, int nboxes,
+                                                                      float4 *bmin, float4 *bmax, float4 *gmin,
+                                                                      float4 *gmax) {
+    __shared__ Bounds s[KNN_BOX];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int box = blockIdx.x * KNN_BOX + warp, j = box * KNN_BOX + lane;
+    Bounds b{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
+    if (box < nboxes && j < n) {
+        const float4 p = sp[j];
+        const float c[3] = {p.x, p.y, p.z};
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            if (isfinite(c[a])) b.lo[a] = b.hi[a] = c[a];
+    }
+    warp_bounds(b);
+    if (lane == 0) {
+        if (box < nboxes) store_bounds(bmin, bmax, box, b);
+        s[warp] = b;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        b = s[lane];
+        warp_bounds(b);
+        if (lane == 0) store_bounds(gmin, gmax, blockIdx.x, b);
+    }
+}
+
+// The supergroups' bounds, a warp each.
+__global__ void knn_super_kernel(const float4 *gmin, const float4 *gmax, int ngroups, int nsuper, float4 *smin,
+                                 float4 *smax) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= nsuper) return;  // warp-uniform
+    const int g = i * KNN_BOX + lane;
+    Bounds b{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
+    if (g < ngroups) {
+        const float4 lo = gmin[g], hi = gmax[g];
+        b = Bounds{{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}};
+    }
+    warp_bounds(b);
+    if (lane == 0) store_bounds(smin, smax, i, b);
+}
+
+// best[0] <= best[1] <= best[2] (core/cpu/msplat_cpu.cpp:1522-1531); a NaN distance
+// (a candidate with non-finite coordinates) is no neighbour
 __device__ __forceinline__ void keep3(float d, float &b0, float &b1, float &b2) {
-    if (d >= b2) return;
+    if (!(d < b2)) return;
     if (d < b1) {
         b2 = b1;
         if (d < b0) {
@@ -119,89 +178,150 @@ __device__ __forceinline__ void keep3(float d, float &b0, float &b1, float &b2) 
     }
 }
 
+// Lower bound of the squared distance between a point of [qlo, qhi] and one of [lo, hi].
 __device__ __forceinline__ float gap(float qlo, float qhi, float blo, float bhi) {
     return fmaxf(fmaxf(blo - qhi, qlo - bhi), 0.f);
 }
+__device__ __forceinline__ float gap2(const Bounds &q, const float4 lo, const float4 hi) {
+    const float gx = gap(q.lo[0], q.hi[0], lo.x, hi.x), gy = gap(q.lo[1], q.hi[1], lo.y, hi.y),
+                gz = gap(q.lo[2], q.hi[2], lo.z, hi.z);
+    return gx * gx + gy * gy + gz * gz;
+}
+
+// A warp's search state: its 32 queries (one per lane) and their three best distances.
+struct KnnSearch {
+    const float4 *sp;
+    int n;
+    float4 q;
+    uint32_t self;
+    bool fin;      // this lane has a query with finite coordinates
+    Bounds qb;     // bounds of the warp's finite queries
+    float b0, b1, b2;
+    unsigned boxes;  // boxes whose points were read
+
+    // the warp's largest third-best: no node at or beyond it matters
+    __device__ __forceinline__ float threshold() const {
+        return from_ordered(__reduce_max_sync(0xffffffffu, ordered_bits(fin ? b2 : -INFINITY)));
+    }
+    // whether node i (< count) may hold a neighbour of one of the warp's queries
+    __device__ __forceinline__ bool near(const float4 *mn, const float4 *mx, int i, int count, float thr) const {
+        if (i >= count) return false;
+        const float4 lo = mn[i], hi = mx[i];
+        return lo.x <= hi.x && gap2(qb, lo, hi) < thr;
+    }
+    // box c's points against every query; the loads are the same on every lane
+    __device__ __forceinline__ void scan_box(int c) {
+        boxes++;
+        const int j0 = c * KNN_BOX, cnt = min(KNN_BOX, n - j0);
+#pragma unroll 8
+        for (int k = 0; k < cnt; k++) {
+            const float4 p = sp[j0 + k];
+            const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+            const float d = dx * dx + dy * dy + dz * dz;
+            if (d < b2 && fin && __float_as_uint(p.w) != self) keep3(d, b0, b1, b2);
+        }
+    }
+    // the 32 boxes of group g, except box `skip`
+    __device__ __forceinline__ void scan_group(int g, int skip, const float4 *bmin, const float4 *bmax, int nboxes) {
+        const int lane = threadIdx.x & 31, c = g * KNN_BOX + lane;
+        const float thr = threshold();  // every lane takes part
+        unsigned m = __ballot_sync(0xffffffffu, c != skip && near(bmin, bmax, c, nboxes, thr));
+        while (m) {  // warp-uniform
+            const int cb = g * KNN_BOX + __ffs(m) - 1;
+            m &= m - 1;
+            const float4 lo = bmin[cb], hi = bmax[cb];
+            const Bounds me{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
+            if (__ballot_sync(0xffffffffu, fin && gap2(me, lo, hi) < b2)) scan_box(cb);
+        }
+    }
+};
 
 // evals (may be null): adds the point distances the warp computes (32 per query per
-// surviving box) -- the search's work, for throughput reports.
-__global__ void knn_query_kernel(const float4 *sp, int n, int nboxes, const float4 *bmin, const float4 *bmax,
-                                 float *out, unsigned long long *evals) {
+// box it reads) -- the search's work, for throughput reports.
+//
+// Bound by instruction issue: about 12 instructions a point of a box that is read. A
+// 400 k-point cloud: 4.34 -> 0.56 ms against the form in which every warp tested all
+// 12.5 k boxes, 32 at a time, and read all that passed the first test; the descent
+// through groups and supergroups leaves a few dozen node tests a warp.
+__global__ void __launch_bounds__(128) knn_query_kernel(const float4 *sp, int n, int nboxes, const float4 *bmin,
+                                                        const float4 *bmax, int ngroups, const float4 *gmin,
+                                                        const float4 *gmax, int nsuper, const float4 *smin,
+                                                        const float4 *smax, float *out, unsigned long long *evals) {
     const int lane = threadIdx.x & 31;
     const int own = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     if (own >= nboxes) return;  // warp-uniform
     const int j = own * KNN_BOX + lane;
     const bool valid = j < n;
-    const float4 q = valid ? sp[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint32_t self = __float_as_uint(q.w);
-    const bool fin = valid && isfinite(q.x) && isfinite(q.y) && isfinite(q.z);
-    // bounds of the warp's queries
-    float ql[3] = {fin ? q.x : INFINITY, fin ? q.y : INFINITY, fin ? q.z : INFINITY};
-    float qh[3] = {fin ? q.x : -INFINITY, fin ? q.y : -INFINITY, fin ? q.z : -INFINITY};
+    KnnSearch s;
+    s.sp = sp;
+    s.n = n;
+    s.q = valid ? sp[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    s.self = __float_as_uint(s.q.w);
+    s.fin = valid && isfinite(s.q.x) && isfinite(s.q.y) && isfinite(s.q.z);
+    const float c[3] = {s.q.x, s.q.y, s.q.z};
 #pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            ql[a] = fminf(ql[a], __shfl_xor_sync(0xffffffffu, ql[a], o));
-            qh[a] = fmaxf(qh[a], __shfl_xor_sync(0xffffffffu, qh[a], o));
-        }
-    float b0 = INFINITY, b1 = INFINITY, b2 = INFINITY;
-    const unsigned nq = __popc(__ballot_sync(0xffffffffu, fin));  // queries with a finite point
-    // candidate t visits own, own+1, own-1, own+2, own-2, ...
-    const int span = 2 * nboxes;
-    for (int t0 = 0; t0 < span; t0 += 32) {
-        const int t = t0 + lane;
-        const int c = own + ((t & 1) ? (t + 1) / 2 : -(t / 2));
-        float thr = fin ? b2 : -INFINITY;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) thr = fmaxf(thr, __shfl_xor_sync(0xffffffffu, thr, o));
-        bool pass = false;
-        if (t < span && c >= 0 && c < nboxes && ql[0] <= qh[0]) {
-            const float4 lo = bmin[c], hi = bmax[c];
-            const float gx = gap(ql[0], qh[0], lo.x, hi.x), gy = gap(ql[1], qh[1], lo.y, hi.y),
-                        gz = gap(ql[2], qh[2], lo.z, hi.z);
-            pass = gx * gx + gy * gy + gz * gz < thr && lo.x <= hi.x;
-        }
-        unsigned m = __ballot_sync(0xffffffffu, pass);
-        if (evals && lane == 0 && m) atomicAdd(evals, (unsigned long long)__popc(m) * nq * KNN_BOX);
-        while (m) {
-            const int src = __ffs(m) - 1;
-            m &= m - 1;
-            const int cb = __shfl_sync(0xffffffffu, c, src);
-            const int pj = cb * KNN_BOX + lane;
-            const float4 p = pj < n ? sp[pj] : make_float4(INFINITY, INFINITY, INFINITY, __uint_as_float(0xffffffffu));
-            for (int k = 0; k < KNN_BOX; k++) {
-                const float px = __shfl_sync(0xffffffffu, p.x, k), py = __shfl_sync(0xffffffffu, p.y, k),
-                            pz = __shfl_sync(0xffffffffu, p.z, k);
-                const uint32_t pi = __float_as_uint(__shfl_sync(0xffffffffu, p.w, k));
-                if (!fin || cb * KNN_BOX + k >= n || pi == self) continue;
-                const float dx = px - q.x, dy = py - q.y, dz = pz - q.z;
-                keep3(dx * dx + dy * dy + dz * dz, b0, b1, b2);
+    for (int a = 0; a < 3; a++) {
+        s.qb.lo[a] = s.fin ? c[a] : INFINITY;
+        s.qb.hi[a] = s.fin ? c[a] : -INFINITY;
+    }
+    warp_bounds(s.qb);
+    s.b0 = s.b1 = s.b2 = INFINITY;
+    s.boxes = 0;
+    const unsigned nq = __popc(__ballot_sync(0xffffffffu, s.fin));
+    if (nq) {  // warp-uniform
+        const int og = own / KNN_BOX, os = og / KNN_BOX;
+        s.scan_box(own);
+        s.scan_group(og, own, bmin, bmax, nboxes);
+        // supergroup 0 of the walk is the warp's own, then the others in order
+        for (int i0 = 0; i0 < nsuper; i0 += 32) {
+            const int i = i0 + lane, sg = i == 0 ? os : (i <= os ? i - 1 : i);
+            const float thr = s.threshold();
+            unsigned ms = __ballot_sync(0xffffffffu, i < nsuper && s.near(smin, smax, sg, nsuper, thr));
+            while (ms) {
+                const int sgi = __shfl_sync(0xffffffffu, sg, __ffs(ms) - 1);
+                ms &= ms - 1;
+                const int g = sgi * KNN_BOX + lane;
+                const float thrg = s.threshold();
+                unsigned mg = __ballot_sync(0xffffffffu, g != og && s.near(gmin, gmax, g, ngroups, thrg));
+                while (mg) {
+                    const int gi = sgi * KNN_BOX + __ffs(mg) - 1;
+                    mg &= mg - 1;
+                    s.scan_group(gi, -1, bmin, bmax, nboxes);
+                }
             }
         }
+        if (evals && lane == 0) atomicAdd(evals, (unsigned long long)s.boxes * nq * KNN_BOX);
     }
     if (!valid) return;
     float sum = 0.f, cnt = 0.f;
-    if (isfinite(b0)) { sum += sqrtf(b0); cnt += 1.f; }
-    if (isfinite(b1)) { sum += sqrtf(b1); cnt += 1.f; }
-    if (isfinite(b2)) { sum += sqrtf(b2); cnt += 1.f; }
-    out[self] = cnt > 0.f ? sum / cnt : 1.f;
+    if (isfinite(s.b0)) { sum += sqrtf(s.b0); cnt += 1.f; }
+    if (isfinite(s.b1)) { sum += sqrtf(s.b1); cnt += 1.f; }
+    if (isfinite(s.b2)) { sum += sqrtf(s.b2); cnt += 1.f; }
+    out[s.self] = cnt > 0.f ? sum / cnt : 1.f;
 }
 
 int knn_boxes(int n) { return (n + KNN_BOX - 1) / KNN_BOX; }
+int knn_nodes(int n) {
+    const int nb = knn_boxes(n), ng = knn_boxes(nb);
+    return nb + ng + knn_boxes(ng);
+}
 
 int launch_knn3(const float *pts, int n, float *out, KnnScratch &s, cudaStream_t st) {
     if (n <= 0) return 0;
     const unsigned int init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     cudaMemcpyAsync(s.bounds, init, sizeof init, cudaMemcpyHostToDevice, st);
     if (s.evals) cudaMemsetAsync(s.evals, 0, sizeof(unsigned long long), st);
-    knn_bounds_kernel<<<std::min((n + 255) / 256, 1184), 256, 0, st>>>(pts, n, s.bounds);
+    knn_bounds_kernel<<<std::min((n + KNN_BOUNDS_THREADS - 1) / KNN_BOUNDS_THREADS, 2 * 148), KNN_BOUNDS_THREADS, 0,
+                        st>>>(pts, n, s.bounds);
     knn_morton_kernel<<<(n + 255) / 256, 256, 0, st>>>(pts, n, s.bounds, s.keys[0], s.vals[0]);
-    const int cur = radix_sort_pairs(s.keys, s.vals, n, 30, s.radix_scratch, st);
+    const int cur = radix_sort_pairs32(s.keys, s.vals, n, 30, s.radix_scratch, st);
     knn_gather_kernel<<<(n + 255) / 256, 256, 0, st>>>(pts, n, s.vals[cur], s.sorted);
-    const int nb = knn_boxes(n);
-    knn_boxes_kernel<<<(nb + 127) / 128, 128, 0, st>>>(s.sorted, n, nb, s.bmin, s.bmax);
-    knn_query_kernel<<<(nb * 32 + 127) / 128, 128, 0, st>>>(s.sorted, n, nb, s.bmin, s.bmax, out, s.evals);
+    const int nb = knn_boxes(n), ng = knn_boxes(nb), ns = knn_boxes(ng);
+    float4 *gmin = s.bmin + nb, *gmax = s.bmax + nb, *smin = gmin + ng, *smax = gmax + ng;
+    knn_boxes_kernel<<<ng, KNN_BOX * KNN_BOX, 0, st>>>(s.sorted, n, nb, s.bmin, s.bmax, gmin, gmax);
+    knn_super_kernel<<<(ns + 7) / 8, 256, 0, st>>>(gmin, gmax, ng, ns, smin, smax);
+    knn_query_kernel<<<(int)(((int64_t)nb * 32 + 127) / 128), 128, 0, st>>>(
+        s.sorted, n, nb, s.bmin, s.bmax, ng, gmin, gmax, ns, smin, smax, out, s.evals);
     return 0;
 }
 

@@ -79,6 +79,20 @@ def test_gpu_knn_counts_its_distance_evaluations():
     assert int(ctx.frame("knn_evals").view(torch.int64)[0]) == 2 * 33 * 32
 
 
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 32 * 1024 - 1, 32 * 1024 + 1, 34 * 1024 + 5, 90_001])
+def test_gpu_knn_search_levels(n):
+    """Sizes around a group (1024 points) and a supergroup (32 groups) of the search, on a
+    cloud of tight clusters, copies of one point and strays far from both, against the
+    oracle's k-d tree: the same float distances, so exactly its values."""
+    rng = np.random.default_rng(n)
+    centres = rng.uniform(-50, 50, (12, 3))
+    pts = centres[rng.integers(0, 12, n)] + rng.normal(0, 0.05, (n, 3))
+    pts[: n // 10] = pts[0]
+    pts[-7:] = rng.uniform(-400, 400, (7, 3))
+    pts = rng.permutation(pts).astype(np.float32)
+    np.testing.assert_array_equal(_core._gpu_knn3_mean_dist(pts), Oracle("restatement").knn3_mean_dist(pts))
+
+
 def _f32_ulps(a, b):
     ia = np.asarray(a, np.float32).view(np.int32).astype(np.int64)
     ib = np.asarray(b, np.float32).view(np.int32).astype(np.int64)
