@@ -138,3 +138,38 @@ def test_autograd_stored_transmittance(capacity):
         ag.set_transmittance_mode("recompute")
     for t, b, nm in zip(p.tensors(), ref_grads, NAMES):
         assert rel_l2(t.grad.cpu().numpy(), b) <= GRAD_RTOL_L2, (nm, capacity, rel_l2(t.grad.cpu().numpy(), b))
+
+
+def _ssim_l1_fp64(img, gt, w):
+    """The training loss in float64 with torch convolutions: zero-padded 11-tap window."""
+    k = torch.exp(-(torch.arange(11, dtype=torch.float64) - 5) ** 2 / 4.5)
+    k = (k / k.sum()).cuda()
+
+    def blur(x):
+        y = torch.nn.functional.conv2d(x[:, None], k.view(1, 1, 1, 11), padding=(0, 5))
+        return torch.nn.functional.conv2d(y, k.view(1, 1, 11, 1), padding=(5, 0))[:, 0]
+
+    a, b = gt.permute(2, 0, 1), img.permute(2, 0, 1)
+    ma, mb = blur(a), blur(b)
+    va, vb, ab = blur(a * a) - ma * ma, blur(b * b) - mb * mb, blur(a * b) - ma * mb
+    ssim = (2 * ma * mb + 1e-4) * (2 * ab + 9e-4) / ((ma * ma + mb * mb + 1e-4) * (va + vb + 9e-4))
+    return w * (1 - ssim.mean()) + (1 - w) * (img - gt).abs().mean()
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (5, 200), (31, 33), (32, 32), (33, 64), (97, 65)])
+def test_ssim_loss_tile_edges(h, w):
+    """Sizes around the loss kernel's 32x32 tiles against a float64 torch loss. Tolerances
+    from the arithmetic: an 11-tap separable sum of values below 1 is off by at most about
+    22 roundings of 6e-8, which the variance terms divide by the window's variance
+    (above 0.01 for these images): 1.3e-6 / 0.01 at the worst pixel, a tenth of that in
+    the mean over pixels."""
+    rng = np.random.default_rng(h * 1000 + w)
+    gt = torch.from_numpy(rng.random((h, w, 3)).astype(np.float32)).cuda()
+    img = torch.from_numpy(rng.random((h, w, 3)).astype(np.float32)).cuda().requires_grad_(True)
+    loss = ag.ssim_l1_loss(img, gt, 0.2)
+    loss.backward()
+    ref = img.detach().double().requires_grad_(True)
+    loss64 = _ssim_l1_fp64(ref, gt.double(), 0.2)
+    loss64.backward()
+    assert abs(float(loss) - float(loss64)) <= 1e-5
+    assert rel_l2(img.grad.cpu().numpy(), ref.grad.cpu().numpy()) <= 2e-5
