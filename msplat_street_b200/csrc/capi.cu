@@ -1201,15 +1201,9 @@ int msplat_cuda_image_metrics(msplat_cuda_ctx *ctx, const float *rendered, const
     if (!rendered || !gt) return fail(MSPLAT_CUDA_EINVAL, "null image");
     const size_t npix = (size_t)h * w;
     MetricsScratch s;
-    ENSURE(ctx->img[0], npix * 15, float, hbuf);
-    ENSURE(ctx->img[1], npix * 3, float, ts);
-    ENSURE(ctx->img[2], npix * 3, float, tl);
-    ENSURE(ctx->img[3], npix * 3, double, tq);
-    ENSURE(ctx->img[4], (size_t)h * 3 + 3, double, rows);
-    s.hbuf = hbuf;
+    ENSURE(ctx->img[0], npix * 3, float, ts);
+    ENSURE(ctx->img[1], (size_t)h * 3 + 3, double, rows);
     s.t_ssim = ts;
-    s.t_l1 = tl;
-    s.t_sq = tq;
     s.rows = rows;
     double *dout = rows + (size_t)h * 3;
     launch_image_metrics(rendered, gt, h, w, s, dout, ctx->stream);
@@ -1222,7 +1216,7 @@ int msplat_cuda_pack_rgba8(msplat_cuda_ctx *ctx, const float *img, uint32_t n, u
     if (!ctx) return fail(MSPLAT_CUDA_EINVAL, "null context");
     if (n == 0) return MSPLAT_CUDA_OK;
     if (!img || !out) return fail(MSPLAT_CUDA_EINVAL, "null image");
-    ENSURE(ctx->img[5], (size_t)n * 4, uint8_t, packed);
+    ENSURE(ctx->img[2], (size_t)n * 4, uint8_t, packed);
     launch_pack_rgba8(img, n, packed, ctx->stream);
     CUDA_TRY(cudaMemcpyAsync(out, packed, (size_t)n * 4, cudaMemcpyDefault, ctx->stream));
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -1325,8 +1319,7 @@ int64_t msplat_cuda_ctx_device_bytes(msplat_cuda_ctx *ctx) {
                         &ctx->tcount, &ctx->bdesc, &ctx->bcounter, &ctx->tb.desc, &ctx->tb.pix_img,
                         &ctx->tb.pix_T, &ctx->tb.pix_idx, &ctx->tb.pix_v, &ctx->tb.partials, &ctx->tb.losses,
                         &ctx->tb.counters, &ctx->dkeys[0], &ctx->dkeys[1], &ctx->dvals[0], &ctx->dvals[1],
-                        &ctx->dcounts, &ctx->doff, &ctx->img[0], &ctx->img[1], &ctx->img[2], &ctx->img[3],
-                        &ctx->img[4], &ctx->img[5]};
+                        &ctx->dcounts, &ctx->doff, &ctx->img[0], &ctx->img[1], &ctx->img[2]};
     int64_t total = 0;
     for (const Buf *b : all) total += (int64_t)b->bytes;
     for (const Buf &b : ctx->pri) total += (int64_t)b.bytes;

@@ -207,8 +207,8 @@ struct msplat_cuda_ctx {
     Buf ch[CH_COUNT];
     // depth order of the Gaussians (or batch instances) before key emission
     Buf dkeys[2], dvals[2], dcounts, doff;
-    // image pipeline scratch: metrics (moments, terms, row sums) and RGBA8 packing
-    Buf img[6];
+    // image pipeline scratch: metrics (SSIM terms, row sums) and RGBA8 packing
+    Buf img[3];
     // prior-guided extras: the prior in force, whether the last frame ran in aux
     // mode, and their buffers
     bool has_prior = false, aux_frame = false;
@@ -235,7 +235,7 @@ struct msplat_cuda_ctx {
                       &isect_gid, &inv, &slots, &radix_scratch, &tile_start, &tile_end, &out_img, &final_T,
                       &final_idx, &v_rendered, &loss_part, &loss, &d_flags, &d_counts, &d_scratch, &k_bounds,
                       &k_sorted, &k_box, &k_md, &k_evals, &tstore, &tcount, &pairs, &bdesc, &bcounter, &dkeys[0], &dkeys[1],
-                      &dvals[0], &dvals[1], &dcounts, &doff, &img[0], &img[1], &img[2], &img[3], &img[4], &img[5]};
+                      &dvals[0], &dvals[1], &dcounts, &doff, &img[0], &img[1], &img[2]};
         for (Buf *b : all) {
             if (b->ptr) cudaFree(b->ptr);
             b->ptr = nullptr;

@@ -9,6 +9,8 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "ordered_sums.cuh"
+#include "ssim_window.cuh"
 
 namespace msplat {
 
@@ -80,92 +82,75 @@ __global__ void undistort_kernel(const float *in, int sw, int sh, float fx, floa
     }
 }
 
-__constant__ float kWinM[11] = {0.0010283801f, 0.0075987581f, 0.0360007721f, 0.1093606895f,
-                                0.2130055377f, 0.2660117249f, 0.2130055377f, 0.1093606895f,
-                                0.0360007721f, 0.0075987581f, 0.0010283801f};
+// Metrics pass 1: the SSIM term of every (pixel, channel) (msplat_cpu.cpp:1675-1712), a
+// 32x32 tile of one channel per block: inputs with a 5-pixel halo, clamped to the
+// image's edge, and their horizontal moments in shared memory; each thread computes a
+// run of consecutive outputs (ssim_window.cuh). 1297 x 840: 213 -> 54 us against two passes
+// through a 60-byte-a-pixel buffer of moments, read eleven times.
+constexpr int MT = 32, M_IN = MT + 10, M_PIN = M_IN + 1, M_PH = MT + 1;
+constexpr int M_RUN_H = 8, M_RUN_V = 4, METRICS_THREADS = 256;
+static_assert(MT * (MT / M_RUN_V) == METRICS_THREADS, "one vertical run a thread");
 
-// Metrics pass 1: horizontal 11-tap moments with clamp-to-edge columns, 15 floats per
-// pixel (5 per channel) (msplat_cpu.cpp:1675-1688).
-__global__ void metrics_h_kernel(const float *a, const float *b, int h, int w, float *hb) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= w || y >= h) return;
-    float *o = hb + ((size_t)y * w + x) * 15;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f, s4 = 0.f;
-        for (int k = 0; k < 11; k++) {
-            const int sx = min(max(x + k - 5, 0), w - 1);
-            const size_t i = ((size_t)y * w + sx) * 3 + c;
-            const float gk = kWinM[k], xa = a[i], yb = b[i];
-            s0 += gk * xa;
-            s1 += gk * yb;
-            s2 += gk * xa * xa;
-            s3 += gk * yb * yb;
-            s4 += gk * xa * yb;
-        }
-        o[5 * c] = s0;
-        o[5 * c + 1] = s1;
-        o[5 * c + 2] = s2;
-        o[5 * c + 3] = s3;
-        o[5 * c + 4] = s4;
-    }
-}
-
-// Metrics pass 2: vertical taps, the per-(pixel, channel) SSIM term, |d| and d^2
-// (msplat_cpu.cpp:1690-1712), stored for the ordered row sums.
-__global__ void metrics_v_kernel(const float *a, const float *b, int h, int w, const float *hb, float *t_ssim,
-                                 float *t_l1, double *t_sq) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= w || y >= h) return;
+__global__ void __launch_bounds__(METRICS_THREADS) metrics_ssim_kernel(const float *a, const float *b, int h, int w,
+                                                                        float *t_ssim) {
+    __shared__ float2 in[M_IN * M_PIN];
+    __shared__ Moments<M_IN * M_PH> hb;
     const float C1 = 0.0001f, C2 = 0.0009f;
+    const int tile = blockIdx.x / 3, c = blockIdx.x - 3 * tile, nbx = (w + MT - 1) / MT;
+    const int x0 = tile % nbx * MT, y0 = tile / nbx * MT;
+    for (int i = threadIdx.x; i < M_IN * M_IN; i += METRICS_THREADS) {
+        const int r = i / M_IN, q = i - r * M_IN;
+        const int gy = min(max(y0 - 5 + r, 0), h - 1), gx = min(max(x0 - 5 + q, 0), w - 1);
+        const size_t k = ((size_t)gy * w + gx) * 3 + c;
+        in[r * M_PIN + q] = make_float2(a[k], b[k]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < M_IN * (MT / M_RUN_H); i += METRICS_THREADS) {
+        const int seg = i / M_IN, r = i - seg * M_IN;
+        window_moments_h<M_RUN_H>(in + r * M_PIN + seg * M_RUN_H, hb, r * M_PH + seg * M_RUN_H);
+    }
+    __syncthreads();
+    const int q = threadIdx.x % MT, r0 = threadIdx.x / MT * M_RUN_V;
+    float2 mu[M_RUN_V], sq[M_RUN_V];
+    float xy[M_RUN_V];
+    window_moments_v<M_RUN_V, M_PH>(hb, r0 * M_PH + q, mu, sq, xy);
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        float s[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int k = 0; k < 11; k++) {
-            const int sy = min(max(y + k - 5, 0), h - 1);
-            const float *o = hb + ((size_t)sy * w + x) * 15 + c * 5;
-#pragma unroll
-            for (int q = 0; q < 5; q++) s[q] += kWinM[k] * o[q];
-        }
-        const float m12 = s[0] * s[1], m1 = s[0] * s[0], m2 = s[1] * s[1];
-        const float num = (2.f * m12 + C1) * (2.f * (s[4] - m12) + C2);
-        const float den = (m1 + m2 + C1) * ((s[2] - m1) + (s[3] - m2) + C2);
-        const size_t i = ((size_t)y * w + x) * 3 + c;
-        const float d = a[i] - b[i];
-        t_ssim[i] = num / den;
-        t_l1[i] = fabsf(d);
-        t_sq[i] = (double)d * d;
+    for (int t = 0; t < M_RUN_V; t++) {
+        const int y = y0 + r0 + t, x = x0 + q;
+        if (x >= w || y >= h) continue;
+        const float m12 = mu[t].x * mu[t].y, m1 = mu[t].x * mu[t].x, m2 = mu[t].y * mu[t].y;
+        const float num = (2.f * m12 + C1) * (2.f * (xy[t] - m12) + C2);
+        const float den = (m1 + m2 + C1) * ((sq[t].x - m1) + (sq[t].y - m2) + C2);
+        t_ssim[((size_t)y * w + x) * 3 + c] = num / den;
     }
 }
 
-// Metrics pass 3: one thread per row sums its terms in double in (x, channel) order.
-__global__ void metrics_rows_kernel(int h, int w, const float *t_ssim, const float *t_l1, const double *t_sq,
-                                    double *rows) {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= h) return;
-    double rs = 0.0, rl = 0.0, rq = 0.0;
-    const size_t o = (size_t)y * w * 3;
-    for (int i = 0; i < w * 3; i++) {
-        rs += t_ssim[o + i];
-        rl += t_l1[o + i];
-        rq += t_sq[o + i];
-    }
-    rows[3 * (size_t)y] = rs;
-    rows[3 * (size_t)y + 1] = rl;
-    rows[3 * (size_t)y + 2] = rq;
+// Metrics pass 2: each row's SSIM terms, |d| and d^2 summed in double in (x, channel)
+// order. Bound by the chain of 3 w dependent additions: 42.9 us at 1297 x 840 against
+// 951 with one thread a row, whose loads the chain waited for.
+__global__ void __launch_bounds__(32 * ORD_WARPS) metrics_rows_kernel(const float *a, const float *b, int h, int w,
+                                                                      const float *t_ssim, double *rows) {
+    const int n = 3 * w;
+    block_row_sums3(h, n, [&](int y, int i) {
+        const size_t k = (size_t)y * n + i;
+        return Raw3{{t_ssim[k], a[k], b[k]}};
+    }, [](const Raw3 &r) {
+        const float d = r.v[1] - r.v[2];
+        return Terms3{{(double)r.v[0], (double)fabsf(d), (double)d * d}};
+    }, rows);
 }
 
-// Metrics pass 4: the rows in order, then PSNR / SSIM / L1 (msplat_cpu.cpp:1713-1720).
-__global__ void metrics_final_kernel(int h, int w, const double *rows, double *out) {
-    double ssim = 0.0, l1 = 0.0, sq = 0.0;
-    for (int y = 0; y < h; y++) {
-        ssim += rows[3 * (size_t)y];
-        l1 += rows[3 * (size_t)y + 1];
-        sq += rows[3 * (size_t)y + 2];
-    }
+// Metrics pass 3: the rows in order, then PSNR / SSIM / L1 (msplat_cpu.cpp:1713-1720).
+__global__ void __launch_bounds__(32) metrics_final_kernel(int h, int w, const double *rows, double *out) {
+    __shared__ double buf[3 * ORD_PITCH];
+    const double s = warp_ordered_sums3(h, [&](int y) {
+        return Terms3{{rows[3 * (size_t)y], rows[3 * (size_t)y + 1], rows[3 * (size_t)y + 2]}};
+    }, [](const Terms3 &t) { return t; }, buf);
+    const double l1 = __shfl_sync(0xffffffffu, s, 1), sq = __shfl_sync(0xffffffffu, s, 2);
+    if (threadIdx.x != 0) return;
     const double cnt = (double)h * w * 3, mse = sq / cnt;
     out[0] = mse > 0 ? 10.0 * log10(1.0 / mse) : INFINITY;
-    out[1] = ssim / cnt;
+    out[1] = s / cnt;
     out[2] = l1 / cnt;
 }
 
@@ -206,11 +191,10 @@ void launch_undistort(const float *src, int sw, int sh, const float *intr, const
 
 void launch_image_metrics(const float *a, const float *b, int h, int w, const MetricsScratch &s, double *out,
                           cudaStream_t st) {
-    const dim3 grid((w + 127) / 128, h);
-    metrics_h_kernel<<<grid, 128, 0, st>>>(a, b, h, w, s.hbuf);
-    metrics_v_kernel<<<grid, 128, 0, st>>>(a, b, h, w, s.hbuf, s.t_ssim, s.t_l1, s.t_sq);
-    metrics_rows_kernel<<<(h + 127) / 128, 128, 0, st>>>(h, w, s.t_ssim, s.t_l1, s.t_sq, s.rows);
-    metrics_final_kernel<<<1, 1, 0, st>>>(h, w, s.rows, out);
+    const int64_t tiles = (int64_t)((w + MT - 1) / MT) * ((h + MT - 1) / MT);
+    metrics_ssim_kernel<<<(unsigned)(3 * tiles), METRICS_THREADS, 0, st>>>(a, b, h, w, s.t_ssim);
+    metrics_rows_kernel<<<(h + ORD_WARPS - 1) / ORD_WARPS, 32 * ORD_WARPS, 0, st>>>(a, b, h, w, s.t_ssim, s.rows);
+    metrics_final_kernel<<<1, 32, 0, st>>>(h, w, s.rows, out);
 }
 
 void launch_pack_rgba8(const float *img, uint32_t n, uint8_t *out, cudaStream_t st) {

@@ -283,10 +283,8 @@ void launch_opacity_reset(float *o, float *m1, float *m2, int n, float reset_log
 
 // Image pipeline, metrics and display (image.cu).
 struct MetricsScratch {
-    float *hbuf;            // h * w * 15
-    float *t_ssim, *t_l1;   // h * w * 3
-    double *t_sq;           // h * w * 3
-    double *rows;           // h * 3
+    float *t_ssim;  // h * w * 3
+    double *rows;   // h * 3
 };
 void launch_resize_area(const void *src, int u8in, int sw, int sh, float *dst, int dw, int dh, cudaStream_t st);
 void launch_undistort(const float *src, int sw, int sh, const float *intr, const float *dist, int rx, int ry,

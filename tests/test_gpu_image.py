@@ -60,6 +60,17 @@ def test_image_metrics(oracle, hw):
     assert np.array_equal(got, oracle.image_metrics(a, b))
 
 
+@pytest.mark.parametrize("hw", [(32, 42), (31, 43), (33, 128), (129, 32), (65, 171)])
+def test_image_metrics_tile_and_chunk_edges(oracle, hw):
+    """Sizes around the 32x32 tiles and the 128-term chunks of the ordered sums (a row of
+    128 pixels is three whole chunks): the oracle's values bit for bit."""
+    rng = np.random.default_rng(hw[0] + hw[1])
+    a = _img(rng, *hw)
+    b = np.clip(a + rng.normal(0, 0.1, a.shape), 0, 1).astype(np.float32)
+    got = np.array(Context().image_metrics(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()))
+    assert np.array_equal(got, oracle.image_metrics(a, b))
+
+
 def test_image_metrics_identical_images_give_infinite_psnr(oracle):
     a = _img(np.random.default_rng(2), 20, 30)
     t = torch.from_numpy(a).cuda()
