@@ -144,6 +144,28 @@ def test_train_step_with_prior(oracle, modes):
     set_prior(oracle, None)
 
 
+@pytest.mark.parametrize("sky_w,sky_h", [(5, 3), (4, 2), (9, 7), (130, 33)])
+def test_sky_gradient_texture_sizes(oracle, sky_w, sky_h):
+    """Textures whose texel counts are no multiple of a block's eight, from a few texels
+    with thousands of contributions each to texels with a handful, against the oracle
+    with the tolerances of the other sky tests."""
+    g, cam = _scene(), _camera()
+    set_prior(oracle, None)
+    gt = oracle.render(scenes.random_gaussians(3000, 51, sh_degree=2), cam, BACKGROUND)
+    pr = make_prior(cam.width, cam.height, 8, ("aux", "sky"), sky_w=sky_w, sky_h=sky_h)
+    po = copy_prior(pr)
+    set_prior(oracle, po)
+    go = g.copy()
+    oracle.train_step(go, cam, BACKGROUND, gt, new_adam_state(go, C1_LRS, 1),
+                      {k: np.zeros(g.n, np.float32) for k in ("vis", "gn", "ms")})
+    ctx, ps, p = Context(), to_gpu(pr), GaussianParams.from_numpy(g)
+    ctx.set_prior(ps)
+    ctx.train_step(p, AdamState.zeros_like(p, C1_LRS), cam, BACKGROUND, torch.from_numpy(gt).cuda(), None)
+    assert rel_l2(ps.sky_grad.cpu().numpy(), po["sky_grad"]) <= GRAD_RTOL_L2
+    assert max_abs(ps.sky_tex.cpu().numpy(), po["sky_tex"]) <= 1e-5
+    set_prior(oracle, None)
+
+
 def test_prior_steps_track_the_oracle(oracle):
     """Five steps with every extra on, each started from the oracle's state, so the
     comparison stays per step; the prior arrays are carried by each side."""
