@@ -1,17 +1,17 @@
 // Fused per-Gaussian backward + Adam + densification statistics.
 //
-// One thread per Gaussian replaces four reference passes:
-//  1. reduce_isect_grads (core/cpu/msplat_cpu.cpp:1034-1064): the Gaussian's
-//     intersection slots, found through the inverse sort permutation, are summed in
-//     sorted (= tile) order;
+// A block of Gaussians replaces four reference passes:
+//  1. reduce_isect_grads (core/cpu/msplat_cpu.cpp:1034-1064): each visible Gaussian's
+//     intersection slots, found through the inverse sort permutation, are summed;
 //  2. project_and_sh_backward_adam (:1068-1139): projection, EWA and covariance VJPs
 //     (:197-291) for visible Gaussians, SH gradients fused into Adam for DC and rest;
 //  3. adam_dense (:1142-1147) over ALL N for means, scales, quats and opacity
 //     (invisible Gaussians see a zero gradient, their moments decay);
 //  4. the densification statistics (:1312-1324).
-// The SH-rest Adam is warp-cooperative: each lane computes its Gaussian's basis and
-// colour gradient, then the warp walks the 32 x (B-1) x 3 rest block of its 32
-// Gaussians in memory order, so those loads and stores coalesce.
+// The block first lists its visible Gaussians (a street view sees a tenth to a third of
+// them, scattered over the indices), so that the slot sums and the VJPs run on full
+// warps; the gradients pass through shared memory to the Adam steps, which walk each
+// parameter array as one flat range, coalesced, a thread's loads issued together.
 // Compiled with -fmad=false; expressions keep the reference's operation order.
 #include "common.cuh"
 #include "kernels.h"
@@ -113,63 +113,172 @@ __device__ __forceinline__ void cov3d_vjp(V3 sc, float gs, Q4 q, const float *gc
 }
 
 
-// Sums of the 9 raster-backward values over each visible Gaussian's intersection
-// slots, in sorted (tile) order. Most Gaussians cover a few tiles: each lane sums its
-// own Gaussian's slots one after another, so the lanes' independent loads overlap.
-// A Gaussian covering more than SLOT_LANE_MAX tiles (near the camera: hundreds) is
-// summed by the whole warp afterwards: lane l takes its intersections l, l+32, ... and
-// a fixed butterfly combines the lanes. Both orders are fixed, so the sums do not
-// depend on scheduling. g0 = index of the warp's first Gaussian in offsets / n_tiles;
-// s9 is zero for invisible Gaussians. With slots_depth (aux mode) the depth slots are
-// summed the same way into *sd.
-constexpr int SLOT_LANE_MAX = 64;
+constexpr int MAX_REST = 15;  // SH bases beyond DC that the backward updates (degree <= 3)
 
-__device__ __forceinline__ void warp_slot_sums(bool vis, int64_t g0, const int64_t *offsets, const int32_t *n_tiles,
-                                               const int32_t *inv, const float *slots, float s9[9],
-                                               const float *slots_depth = nullptr, float *sd = nullptr) {
-    const int lane = threadIdx.x & 31;
+// A block's visible Gaussians, and the sums of their intersection slots.
+template <int NB>
+struct VisibleList {
+    int count;
+    int warp_count[NB / 32];
+    uint16_t idx[NB];   // local indices, ascending
+    float s9[NB * 9];   // by local index: xy(2) conic(3) rgb(3) opacity
+    float depth[NB];    // aux mode: dL/d(view depth)
+    int64_t first[NB];  // by local index: first emission index and tiles
+    int tiles[NB];
+    // listed ones whose slots several lanes, or the whole block, add
+    int n_mid, n_large;
+    uint16_t mid[NB], large[NB];
+    float part[NB / 32][10];
+    __device__ __forceinline__ void store(int i, const float p[9], float pd) {
 #pragma unroll
-    for (int c = 0; c < 9; c++) s9[c] = 0.f;
-    if (sd) *sd = 0.f;
-    long long my_e0 = 0;
-    int my_cnt = 0;
-    if (vis) {
-        my_e0 = offsets[g0 + lane];
-        my_cnt = n_tiles[g0 + lane];
+        for (int c = 0; c < 9; c++) s9[i * 9 + c] = p[c];
+        depth[i] = pd;
     }
-    if (vis && my_cnt <= SLOT_LANE_MAX) {
-        for (int j = 0; j < my_cnt; j++) {
-            const int32_t k = inv[my_e0 + j];
-            const float *sl = slots + (size_t)k * 9;
+};
+
+// Lists the threads with vis set. Every thread of the block must call it; on return the
+// list is complete (block-wide).
+template <int NB>
+__device__ __forceinline__ void list_visible(bool vis, VisibleList<NB> &L) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned m = __ballot_sync(0xffffffffu, vis);
+    if (lane == 0) L.warp_count[warp] = __popc(m);
+    __syncthreads();
+    int before = 0, all = 0;
 #pragma unroll
-            for (int c = 0; c < 9; c++) s9[c] += sl[c];
-            if (slots_depth) *sd += slots_depth[k];
-        }
+    for (int w = 0; w < NB / 32; w++) {
+        const int c = L.warp_count[w];
+        if (w < warp) before += c;
+        all += c;
     }
-    const unsigned big = __ballot_sync(0xffffffffu, vis && my_cnt > SLOT_LANE_MAX);
-    for (unsigned bits = big; bits; bits &= bits - 1u) {  // warp-uniform
-        const int gl = __ffs(bits) - 1;
-        const long long e0 = __shfl_sync(0xffffffffu, my_e0, gl);
-        const int cnt = __shfl_sync(0xffffffffu, my_cnt, gl);
-        float p[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, pd = 0.f;
-        for (int j = lane; j < cnt; j += 32) {
-            const int32_t k = inv[e0 + j];
-            const float *sl = slots + (size_t)k * 9;
+    if (vis) L.idx[before + __popc(m & ((1u << lane) - 1u))] = (uint16_t)threadIdx.x;
+    if (threadIdx.x == 0) {
+        L.count = all;
+        L.n_mid = L.n_large = 0;
+    }
+    __syncthreads();
+}
+
+// Lists the visible ones of a block's instances g0 .. g0 + rows - 1 with their slots'
+// emission indices.
+template <int NB>
+__device__ __forceinline__ bool list_instances(VisibleList<NB> &L, int64_t g0, int rows, const int32_t *radii,
+                                               const int64_t *offsets, const int32_t *n_tiles) {
+    const int t = threadIdx.x;
+    const bool in = t < rows, vis = in && radii[g0 + t] > 0;
+    const int64_t first = in ? offsets[g0 + t] : 0;  // not behind the radius: one latency for all three
+    const int tiles = in ? n_tiles[g0 + t] : 0;
+    L.first[t] = first;
+    L.tiles[t] = tiles;
+    list_visible<NB>(vis, L);
+    return vis;
+}
+
+// Sums of the 9 (with slots_depth: 10) raster-backward values over each listed
+// Gaussian's intersection slots. A Gaussian of up to SLOT_LANE_MAX tiles is one lane's,
+// of up to SLOT_GROUP_MAX SLOT_LANES neighbouring lanes' (lane l adds slots l,
+// l + SLOT_LANES, ..., the lanes' sums are added as a fixed tree), of up to
+// SLOT_WARP_MAX a warp's, and one of more (near the camera) the block's. The orders are
+// fixed, so the sums do not depend on scheduling. Every thread of the block must call
+// it; the sums are complete after the next block barrier.
+//
+// Bound by the latency of two dependent loads a slot (its sorted position, then the slot
+// in L2), about a microsecond; a step fetches two slots a lane. One lane walking its
+// Gaussian's slots alone (34 on average in an early street view) and one warp walking
+// the 2000 of a Gaussian in front of the camera were most of the kernel's time.
+constexpr int SLOT_LANES = 8, SLOT_LANE_MAX = 8, SLOT_GROUP_MAX = 64, SLOT_WARP_MAX = 256;
+
+// A lane's share: slots l, l + step, ... of the cnt from emission index e0.
+__device__ __forceinline__ void add_slots(int l, int step, int64_t e0, int cnt, const int32_t *inv,
+                                          const float *slots, const float *slots_depth, float p[9], float &pd) {
 #pragma unroll
-            for (int c = 0; c < 9; c++) p[c] += sl[c];
-            if (slots_depth) pd += slots_depth[k];
-        }
+    for (int c = 0; c < 9; c++) p[c] = 0.f;
+    pd = 0.f;
+    int j = l;
+    for (; j + step < cnt; j += 2 * step) {
+        const int32_t k0 = inv[e0 + j], k1 = inv[e0 + j + step];
+        const float *s0 = slots + (size_t)k0 * 9, *s1 = slots + (size_t)k1 * 9;
+        float a[9], b[9];
 #pragma unroll
         for (int c = 0; c < 9; c++) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) p[c] += __shfl_xor_sync(0xffffffffu, p[c], o);
-            if (lane == gl) s9[c] = p[c];
+            a[c] = s0[c];
+            b[c] = s1[c];
         }
-        if (slots_depth) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) pd += __shfl_xor_sync(0xffffffffu, pd, o);
-            if (lane == gl) *sd = pd;
+        for (int c = 0; c < 9; c++) p[c] = (p[c] + a[c]) + b[c];
+        if (slots_depth) pd = (pd + slots_depth[k0]) + slots_depth[k1];
+    }
+    if (j < cnt) {
+        const int32_t k = inv[e0 + j];
+        const float *s = slots + (size_t)k * 9;
+#pragma unroll
+        for (int c = 0; c < 9; c++) p[c] += s[c];
+        if (slots_depth) pd += slots_depth[k];
+    }
+}
+
+// The sums of `lanes` neighbouring lanes, on each of them. Every lane of the warp calls it.
+__device__ __forceinline__ void add_lanes(int lanes, bool with_depth, float p[9], float &pd) {
+    for (int o = lanes / 2; o > 0; o >>= 1) {
+#pragma unroll
+        for (int c = 0; c < 9; c++) p[c] += __shfl_xor_sync(0xffffffffu, p[c], o);
+        if (with_depth) pd += __shfl_xor_sync(0xffffffffu, pd, o);
+    }
+}
+
+template <int NB>
+__device__ __forceinline__ void sum_slots(VisibleList<NB> &L, const int32_t *inv, const float *slots,
+                                          const float *slots_depth) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, l = lane & (SLOT_LANES - 1);
+    const bool wd = slots_depth != nullptr;
+    float p[9], pd;
+    if (t < L.count) {
+        const int i = L.idx[t], cnt = L.tiles[i];
+        if (cnt <= SLOT_LANE_MAX) {
+            add_slots(0, 1, L.first[i], cnt, inv, slots, slots_depth, p, pd);
+            L.store(i, p, pd);
+        } else if (cnt <= SLOT_WARP_MAX) {  // the order of either list changes no sum
+            L.mid[atomicAdd(&L.n_mid, 1)] = (uint16_t)i;
+        } else {
+            L.large[atomicAdd(&L.n_large, 1)] = (uint16_t)i;
         }
+    }
+    __syncthreads();
+    for (int b = 0; b < L.n_mid; b += NB / SLOT_LANES) {  // block-uniform
+        const int li = b + t / SLOT_LANES;
+        const int i = li < L.n_mid ? L.mid[li] : -1, all = i >= 0 ? L.tiles[i] : 0;
+        const int cnt = all <= SLOT_GROUP_MAX ? all : 0;
+        add_slots(l, SLOT_LANES, i >= 0 ? L.first[i] : 0, cnt, inv, slots, slots_depth, p, pd);
+        add_lanes(SLOT_LANES, wd, p, pd);
+        if (l == 0 && cnt > 0) L.store(i, p, pd);
+        unsigned m = __ballot_sync(0xffffffffu, l == 0 && all > SLOT_GROUP_MAX);
+        while (m) {  // warp-uniform: this warp's larger ones, one after another
+            const int bi = __shfl_sync(0xffffffffu, i, __ffs(m) - 1);
+            m &= m - 1;
+            add_slots(lane, 32, L.first[bi], L.tiles[bi], inv, slots, slots_depth, p, pd);
+            add_lanes(32, wd, p, pd);
+            if (lane == 0) L.store(bi, p, pd);
+        }
+    }
+    for (int q = 0; q < L.n_large; q++) {  // block-uniform
+        const int i = L.large[q];
+        add_slots(t, NB, L.first[i], L.tiles[i], inv, slots, slots_depth, p, pd);
+        add_lanes(32, wd, p, pd);
+        if (lane == 0) {
+#pragma unroll
+            for (int c = 0; c < 9; c++) L.part[warp][c] = p[c];
+            L.part[warp][9] = pd;
+        }
+        __syncthreads();
+        if (t == 0) {
+            for (int w = 1; w < NB / 32; w++) {
+#pragma unroll
+                for (int c = 0; c < 9; c++) p[c] += L.part[w][c];
+                pd += L.part[w][9];
+            }
+            L.store(i, p, pd);
+        }
+        __syncthreads();
     }
 }
 
@@ -233,350 +342,355 @@ __device__ __forceinline__ void sh_rest_basis(V3 d, float *bs) {
     bs[14] = SH_C3_6 * x * (xx - 3.f * yy);
 }
 
-// Adam over the SH-rest rows of a warp's Gaussians (rows of `stride` floats starting at
-// p, m1, m2), walked as one flat range of rows x stride floats: every access of the
-// warp covers 32 consecutive floats, and each lane loads its U elements before it
-// updates any, so the loads of a row block overlap instead of following one row at a
-// time. grad(r, e) is the gradient of float e of row r; rows with vis[r] == 0 and
-// floats e >= used keep their values. Each element gets the same adam_step as in the
-// row-by-row walk.
-template <int U, typename Grad>
-__device__ __forceinline__ void warp_rest_adam(float *__restrict__ p, float *__restrict__ m1,
-                                               float *__restrict__ m2, int rows, int stride, int used,
-                                               const int *vis, Grad grad, float ss, float b1, float b2, float bc2,
-                                               float eps) {
-    if (stride <= 0 || rows <= 0) return;
-    const int lane = threadIdx.x & 31;
-    const int total = rows * stride;
-    int r = 0, e = lane;  // row and float of this lane's next element
-    while (e >= stride) {
-        e -= stride;
-        r++;
-    }
-    for (int j0 = 0; j0 < total; j0 += 32 * U) {
-        float pv[U], v1[U], v2[U];
-        int rr[U], ee[U];
-        bool up[U];
+// Adam over one array of a block's Gaussians, `count` consecutive floats of it with
+// their gradients in shared memory: every access of a warp covers 32 consecutive floats.
+// load() only reads, so that a thread can have two arrays' loads on their way at once.
+// use(j): whether element j is updated.
+template <int NB, int U>
+struct AdamFlat {
+    float pv[U], v1[U], v2[U];
+    template <typename Use>
+    __device__ __forceinline__ void load(const float *p, const float *m1, const float *m2, int count, Use use) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int j = j0 + u * 32 + lane;
-            rr[u] = r;
-            ee[u] = e;
-            up[u] = j < total && e < used && vis[r] != 0;  // vis[r] read only for j < total
-            if (up[u]) {
+            const int j = u * NB + (int)threadIdx.x;
+            if (j < count && use(j)) {
                 pv[u] = p[j];
                 v1[u] = m1[j];
                 v2[u] = m2[j];
             }
-            e += 32;
-            while (e >= stride) {
-                e -= stride;
-                r++;
-            }
         }
+    }
+    template <typename Use>
+    __device__ __forceinline__ void update(float *p, float *m1, float *m2, const float *g, int count, float ss,
+                                           float b1, float b2, float bc2, float eps, Use use) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            if (up[u]) {
-                const int j = j0 + u * 32 + lane;
-                adam_step(pv[u], v1[u], v2[u], grad(rr[u], ee[u]), ss, b1, b2, bc2, eps);
-                p[j] = pv[u];
-                m1[j] = v1[u];
-                m2[j] = v2[u];
-            }
+            const int j = u * NB + (int)threadIdx.x;
+            if (!(j < count && use(j))) continue;
+            adam_step(pv[u], v1[u], v2[u], g[j], ss, b1, b2, bc2, eps);
+            p[j] = pv[u];
+            m1[j] = v1[u];
+            m2[j] = v2[u];
+        }
+    }
+};
+
+// The dense groups and DC of a block's Gaussians (all but the SH rest).
+template <int NB>
+__device__ __forceinline__ void adam_groups(float *const p[6], float *const m1[6], float *const m2[6], int64_t g0,
+                                            int rows, const float *s_mean, const float *s_scale, const float *s_quat,
+                                            const float *s_op, const float *s_dc, const uint8_t *s_vis,
+                                            const float *ss, const float *bc2, float b1, float b2, float eps) {
+    auto all = [](int) { return true; };
+    auto seen = [&](int j) { return s_vis[j / 3] != 0; };
+    const size_t o3 = 3 * (size_t)g0, o4 = 4 * (size_t)g0;
+    const bool op = m1[5] != nullptr;
+    AdamFlat<NB, 3> mean, scale, dc;
+    AdamFlat<NB, 4> quat;
+    AdamFlat<NB, 1> opac;
+    mean.load(p[0] + o3, m1[0] + o3, m2[0] + o3, 3 * rows, all);
+    scale.load(p[1] + o3, m1[1] + o3, m2[1] + o3, 3 * rows, all);
+    mean.update(p[0] + o3, m1[0] + o3, m2[0] + o3, s_mean, 3 * rows, ss[0], b1, b2, bc2[0], eps, all);
+    quat.load(p[2] + o4, m1[2] + o4, m2[2] + o4, 4 * rows, all);
+    scale.update(p[1] + o3, m1[1] + o3, m2[1] + o3, s_scale, 3 * rows, ss[1], b1, b2, bc2[1], eps, all);
+    dc.load(p[3] + o3, m1[3] + o3, m2[3] + o3, 3 * rows, seen);
+    quat.update(p[2] + o4, m1[2] + o4, m2[2] + o4, s_quat, 4 * rows, ss[2], b1, b2, bc2[2], eps, all);
+    if (op) opac.load(p[5] + g0, m1[5] + g0, m2[5] + g0, rows, all);
+    dc.update(p[3] + o3, m1[3] + o3, m2[3] + o3, s_dc, 3 * rows, ss[3], b1, b2, bc2[3], eps, seen);
+    if (op) opac.update(p[5] + g0, m1[5] + g0, m2[5] + g0, s_op, rows, ss[5], b1, b2, bc2[5], eps, all);
+}
+
+// Adam over the SH-rest rows (`stride` floats, of which the first `used` have gradients)
+// of `rows` Gaussians: row(r) is the r-th one's local index, grad(i, base, c, e) the
+// gradient of local Gaussian i's float e = 3 base + c. A warp takes as many whole rows at
+// a time as fit three floats a lane (two of 45 floats, four of 24, ten of 9), as one flat
+// range, all loads issued before any update.
+template <int NB, typename Row, typename Grad>
+__device__ __forceinline__ void adam_rest(float *__restrict__ p, float *__restrict__ m1, float *__restrict__ m2,
+                                          int rows, int stride, int used, Row row, Grad grad, float ss, float b1,
+                                          float b2, float bc2, float eps) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int E = 3;
+    const int per = 32 * E / used;
+    int r[E], e[E];  // the lane's floats: row within the step, float within the row
+#pragma unroll
+    for (int q = 0; q < E; q++) {
+        const int k = q * 32 + lane;
+        r[q] = k / used;
+        e[q] = k - r[q] * used;
+    }
+    for (int r0 = warp * per; r0 < rows; r0 += NB / 32 * per) {
+        float pv[E], v1[E], v2[E];
+        int at[E];
+#pragma unroll
+        for (int q = 0; q < E; q++) {
+            at[q] = r[q] < per && r0 + r[q] < rows ? row(r0 + r[q]) : -1;
+            if (at[q] < 0) continue;
+            const size_t j = (size_t)at[q] * stride + e[q];
+            pv[q] = p[j];
+            v1[q] = m1[j];
+            v2[q] = m2[j];
+        }
+#pragma unroll
+        for (int q = 0; q < E; q++) {
+            if (at[q] < 0) continue;
+            const size_t j = (size_t)at[q] * stride + e[q];
+            const int base = e[q] / 3;
+            adam_step(pv[q], v1[q], v2[q], grad(at[q], base, e[q] - 3 * base, e[q]), ss, b1, b2, bc2, eps);
+            p[j] = pv[q];
+            m1[j] = v1[q];
+            m2[j] = v2[q];
         }
     }
 }
 
-// Writes a warp's SH-rest gradient rows (gradient-only mode) as one flat range:
-// grad(r, e) where e < used and row r is visible (every row when vis is null), else 0.
-template <typename Grad>
-__device__ __forceinline__ void warp_rest_grad(float *__restrict__ out, int rows, int stride, int used,
-                                               const int *vis, Grad grad) {
-    if (stride <= 0 || rows <= 0) return;
-    const int lane = threadIdx.x & 31;
-    const int total = rows * stride;
-    int r = 0, e = lane;
-    while (e >= stride) {
-        e -= stride;
-        r++;
-    }
-    for (int j = lane; j < total; j += 32) {
-        out[j] = (e < used && (vis == nullptr || vis[r] != 0)) ? grad(r, e) : 0.f;
-        e += 32;
-        while (e >= stride) {
-            e -= stride;
-            r++;
+// Writes every SH-rest gradient row of a block (gradient-only mode): grad(i, base, c, e)
+// where e < used, else 0.
+template <int NB, typename Grad>
+__device__ __forceinline__ void write_rest(float *__restrict__ out, int rows, int stride, int used, Grad grad) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = warp; i < rows; i += NB / 32)
+        for (int e = lane; e < stride; e += 32) {
+            const int base = e / 3;
+            out[(size_t)i * stride + e] = e < used ? grad(i, base, e - 3 * base, e) : 0.f;
         }
-    }
 }
 
-constexpr int REST_UNROLL = 4;
+// The bases beyond DC that get gradients at an SH degree in use.
+__device__ __forceinline__ int active_bases(uint32_t dtu) { return dtu < 1 ? 0 : dtu < 2 ? 3 : dtu < 3 ? 8 : 15; }
 
 }  // namespace
 
-constexpr int BWD_THREADS = 256;
-constexpr int MAX_REST = 15;  // SH bases beyond DC that the backward updates (degree <= 3)
+// Gaussians (and threads) a block. 64 was no faster for a 10 k scene (29.7 against 29.2
+// us).
+constexpr int NB = 128;
 
-__global__ void __launch_bounds__(BWD_THREADS, 4) backward_adam_kernel(BackwardArgs a) {
-    __shared__ float s_basis[BWD_THREADS][MAX_REST + 1];
-    __shared__ float s_vrgb[BWD_THREADS][3];
-    __shared__ int s_vis[BWD_THREADS];
-    const int i = blockIdx.x * BWD_THREADS + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    const bool valid = i < a.n;
-    const bool vis = valid && a.radii[i] > 0;
-    const float b1 = a.beta1, b2 = a.beta2, eps = a.eps;
+// Bound by the latency of its chain of phases (radii; slot positions; slots; parameters;
+// three rounds of Adam loads) and, where most Gaussians are visible and SH degree 3 is in
+// use, by issue (Adam's exact square root and divisions). Against one thread a Gaussian
+// with its slots, VJPs and Adam in one lane: a 1 M-Gaussian street step at 1600 x 1060
+// 545 -> 297 us, an early 100 k street view 100 -> 69 us, 200 k gradients with everything
+// visible 65 -> 67 us.
+__global__ void __launch_bounds__(NB, 1024 / NB) backward_adam_kernel(BackwardArgs a) {
+    __shared__ VisibleList<NB> L;
+    __shared__ float s_mean[NB * 3], s_scale[NB * 3], s_quat[NB * 4], s_op[NB], s_dc[NB * 3];
+    __shared__ float s_basis[NB][MAX_REST + 2];
+    __shared__ uint8_t s_vis[NB];
+    const int t = threadIdx.x;
+    const int64_t g0 = (int64_t)blockIdx.x * NB;
+    const int rows = (int)min((int64_t)NB, (int64_t)a.n - g0);
+    const int active = active_bases(a.cam.degrees_to_use);
 
-    // 1. per-Gaussian sums of the intersection slots
-    float s9[9], sd = 0.f;
-    warp_slot_sums(vis, (int64_t)blockIdx.x * BWD_THREADS + (threadIdx.x - lane), a.offsets, a.n_tiles, a.inv,
-                   a.slots, s9, a.slots_depth, a.slots_depth ? &sd : nullptr);
-    if (valid) {  // s9 is zero for invisible Gaussians
+    // 1. the visible Gaussians and their slot sums
+    const bool vis = list_instances<NB>(L, g0, rows, a.radii, a.offsets, a.n_tiles);
+    if (!vis) {
+#pragma unroll
+        for (int c = 0; c < 9; c++) L.s9[t * 9 + c] = 0.f;
+        L.depth[t] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; c++) s_mean[t * 3 + c] = s_scale[t * 3 + c] = s_dc[t * 3 + c] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; c++) s_quat[t * 4 + c] = 0.f;
+        s_op[t] = 0.f;
+    }
+    s_vis[t] = vis;
+    sum_slots<NB>(L, a.inv, a.slots, a.slots_depth);
+    __syncthreads();
+
+    // 2. projection VJPs and densification statistics, a listed Gaussian per thread
+    if (t < L.count) {
+        const int li = L.idx[t], i = (int)g0 + li;
+        float s9[9], gm[3], gsv[3], gq[4];
+#pragma unroll
+        for (int c = 0; c < 9; c++) s9[c] = L.s9[li * 9 + c];
+        V3 dir;
+        projection_vjp(a.cam, a.means, a.scales, a.quats, a.glob_scale, a.splats + i, i, s9, gm, gsv, gq, dir,
+                       a.slots_depth ? L.depth[li] : 0.f);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            s_mean[li * 3 + c] = gm[c];
+            s_scale[li * 3 + c] = gsv[c];
+            s_dc[li * 3 + c] = SH_C0 * s9[5 + c];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) s_quat[li * 4 + c] = gq[c];
+        s_op[li] = s9[8];
+        if (active > 0) sh_rest_basis(dir, s_basis[li]);
+        if (a.vis_counts) {
+            a.vis_counts[i] += 1.0f;
+            a.xys_grad_norm[i] += sqrtf(s9[0] * s9[0] + s9[1] * s9[1]);
+            a.max_2d_size[i] = fmaxf(a.max_2d_size[i], (float)a.radii[i] * a.inv_max_dim);
+        }
+    }
+    __syncthreads();
+
+    // 3. gradient outputs (zero for invisible Gaussians)
+    if (t < rows) {
+        const size_t i = (size_t)g0 + t;
+        const float *s9 = L.s9 + t * 9;
         if (a.v_xy) {
             a.v_xy[2 * i] = s9[0];
             a.v_xy[2 * i + 1] = s9[1];
         }
-        if (a.v_conic) {
-            a.v_conic[3 * i] = s9[2];
-            a.v_conic[3 * i + 1] = s9[3];
-            a.v_conic[3 * i + 2] = s9[4];
-        }
-        if (a.v_rgb) {
-            a.v_rgb[3 * i] = s9[5];
-            a.v_rgb[3 * i + 1] = s9[6];
-            a.v_rgb[3 * i + 2] = s9[7];
-        }
+        if (a.v_conic)
+            for (int c = 0; c < 3; c++) a.v_conic[3 * i + c] = s9[2 + c];
+        if (a.v_rgb)
+            for (int c = 0; c < 3; c++) a.v_rgb[3 * i + c] = s9[5 + c];
         if (a.v_opacity) a.v_opacity[i] = s9[8];
-        if (a.v_depth) a.v_depth[i] = sd;
-    }
-
-    // 2. projection VJPs
-    float gm[3] = {0.f, 0.f, 0.f}, gsv[3] = {0.f, 0.f, 0.f}, gq[4] = {0.f, 0.f, 0.f, 0.f};
-    V3 dir{0.f, 0.f, 1.f};
-    if (vis)
-        projection_vjp(a.cam, a.means, a.scales, a.quats, a.glob_scale, a.splats + i, i, s9, gm, gsv, gq, dir, sd);
-    if (valid && a.v_mean3d) {
-        for (int c = 0; c < 3; c++) {
-            a.v_mean3d[3 * i + c] = gm[c];
-            a.v_scale[3 * i + c] = gsv[c];
-        }
-        for (int c = 0; c < 4; c++) a.v_quat[4 * i + c] = gq[c];
-    }
-
-    // 3. dense Adam: means, scales, quats, opacity (all N)
-    if (valid && a.do_adam) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const size_t k = 3 * (size_t)i + c;
-            adam_step(a.p[0][k], a.m1[0][k], a.m2[0][k], gm[c], a.ss[0], b1, b2, a.bc2[0], eps);
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const size_t k = 3 * (size_t)i + c;
-            adam_step(a.p[1][k], a.m1[1][k], a.m2[1][k], gsv[c], a.ss[1], b1, b2, a.bc2[1], eps);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const size_t k = 4 * (size_t)i + c;
-            adam_step(a.p[2][k], a.m1[2][k], a.m2[2][k], gq[c], a.ss[2], b1, b2, a.bc2[2], eps);
-        }
-        if (a.m1[5]) adam_step(a.p[5][i], a.m1[5][i], a.m2[5][i], s9[8], a.ss[5], b1, b2, a.bc2[5], eps);
-        // needle cap after the scale update (scale_ratio_cap, core/cpu/msplat_cpu.cpp:1295-1309)
-        if (a.log_max_scale_ratio > 0.f) {
-            float *sc = a.p[1] + 3 * (size_t)i;
-            const float x = sc[0], y = sc[1], z = sc[2];
-            const float mx = fmaxf(x, fmaxf(y, z)), mn = fminf(x, fminf(y, z));
-            const float cap = (x + y + z - mx - mn) + a.log_max_scale_ratio;
-            if (mx > cap) {
-                if (x == mx) sc[0] = cap;
-                else if (y == mx) sc[1] = cap;
-                else sc[2] = cap;
-            }
-        }
-        // DC for visible Gaussians
-        if (vis) {
-#pragma unroll
+        if (a.v_depth) a.v_depth[i] = L.depth[t];
+        if (a.v_mean3d) {
             for (int c = 0; c < 3; c++) {
-                const size_t k = 3 * (size_t)i + c;
-                adam_step(a.p[3][k], a.m1[3][k], a.m2[3][k], SH_C0 * s9[5 + c], a.ss[3], b1, b2, a.bc2[3], eps);
+                a.v_mean3d[3 * i + c] = s_mean[t * 3 + c];
+                a.v_scale[3 * i + c] = s_scale[t * 3 + c];
+            }
+            for (int c = 0; c < 4; c++) a.v_quat[4 * i + c] = s_quat[t * 4 + c];
+        }
+        if (a.g_dc)
+            for (int c = 0; c < 3; c++) a.g_dc[3 * i + c] = s_dc[t * 3 + c];
+    }
+
+    // 4. Adam: means, scales, quats, opacity of all N; DC and the SH rest of the visible
+    const float b1 = a.beta1, b2 = a.beta2, eps = a.eps;
+    if (a.do_adam) {
+        adam_groups<NB>(a.p, a.m1, a.m2, g0, rows, s_mean, s_scale, s_quat, s_op, s_dc, s_vis, a.ss, a.bc2, b1, b2,
+                        eps);
+        // needle cap after the scale update (scale_ratio_cap, core/cpu/msplat_cpu.cpp:1295-1309)
+        if (a.log_max_scale_ratio > 0.f) {  // grid-uniform
+            __syncthreads();  // a Gaussian's three scales were updated by three threads
+            if (t < rows) {
+                float *sc = a.p[1] + 3 * ((size_t)g0 + t);
+                const float x = sc[0], y = sc[1], z = sc[2];
+                const float mx = fmaxf(x, fmaxf(y, z)), mn = fminf(x, fminf(y, z));
+                const float cap = (x + y + z - mx - mn) + a.log_max_scale_ratio;
+                if (mx > cap) {
+                    if (x == mx) sc[0] = cap;
+                    else if (y == mx) sc[1] = cap;
+                    else sc[2] = cap;
+                }
             }
         }
     }
 
-    // 4. densification statistics
-    if (vis && a.vis_counts) {
-        a.vis_counts[i] += 1.0f;
-        const float gx = s9[0], gy = s9[1];
-        a.xys_grad_norm[i] += sqrtf(gx * gx + gy * gy);
-        a.max_2d_size[i] = fmaxf(a.max_2d_size[i], (float)a.radii[i] * a.inv_max_dim);
-    }
-
-    // gradient-only mode (autograd): the SH colour gradients as arrays
-    if (valid && a.g_dc) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) a.g_dc[3 * (size_t)i + c] = vis ? SH_C0 * s9[5 + c] : 0.f;
-    }
-
-    // 5. SH rest Adam (or its gradient), warp-cooperative over the warp's 32 Gaussians
-    if ((!a.do_adam && !a.g_rest) || a.rest_stride <= 0) return;
-    const uint32_t dtu = a.cam.degrees_to_use;
-    const int active = dtu < 1 ? 0 : dtu < 2 ? 3 : dtu < 3 ? 8 : 15;  // bases updated
-    if (active == 0 && !a.g_rest) return;
-    {
-        sh_rest_basis(dir, s_basis[threadIdx.x]);
-        s_vrgb[threadIdx.x][0] = s9[5];
-        s_vrgb[threadIdx.x][1] = s9[6];
-        s_vrgb[threadIdx.x][2] = s9[7];
-        s_vis[threadIdx.x] = vis ? 1 : 0;
-    }
-    __syncwarp();
-    const int wbase_t = threadIdx.x - lane;                          // first thread of this warp
-    const int64_t g0 = (int64_t)blockIdx.x * BWD_THREADS + wbase_t;  // its Gaussian
-    const int stride = a.rest_stride;
-    const int used = 3 * active;  // floats of each row that get a gradient
-    const int rows = (int)min((int64_t)32, (int64_t)a.n - g0);
+    // 5. SH rest: its gradient rows, or Adam
+    const int stride = a.rest_stride, used = 3 * active;
+    if (stride <= 0) return;
+    auto grad = [&](int i, int base, int c, int) { return s_basis[i][base] * L.s9[i * 9 + 5 + c]; };
     const size_t off = (size_t)g0 * stride;
-    auto grad = [&](int r, int e) {
-        const int base = e / 3;
-        return s_basis[wbase_t + r][base] * s_vrgb[wbase_t + r][e - 3 * base];
-    };
-    if (a.g_rest) {  // gradient-only mode: every row, zero where invisible or inactive
-        warp_rest_grad(a.g_rest + off, rows, stride, used, s_vis + wbase_t, grad);
+    if (a.g_rest) {
+        write_rest<NB>(a.g_rest + off, rows, stride, used,
+                       [&](int i, int base, int c, int e) { return s_vis[i] ? grad(i, base, c, e) : 0.f; });
         return;
     }
-    warp_rest_adam<REST_UNROLL>(a.p[4] + off, a.m1[4] + off, a.m2[4] + off, rows, stride, used, s_vis + wbase_t, grad,
-                                a.ss[4], b1, b2, a.bc2[4], eps);
+    if (!a.do_adam || active == 0) return;
+    adam_rest<NB>(a.p[4] + off, a.m1[4] + off, a.m2[4] + off, L.count, stride, used,
+                  [&](int r) { return (int)L.idx[r]; }, grad, a.ss[4], b1, b2, a.bc2[4], eps);
 }
 
 void launch_backward_adam(const BackwardArgs &a, cudaStream_t st) {
     if (a.n <= 0) return;
-    backward_adam_kernel<<<(a.n + BWD_THREADS - 1) / BWD_THREADS, BWD_THREADS, 0, st>>>(a);
+    backward_adam_kernel<<<(a.n + NB - 1) / NB, NB, 0, st>>>(a);
 }
 
-// The multi-view form: one thread per Gaussian walks the batch's views in order,
-// sums each view's slots (instance v * n + i), runs that view's projection VJPs and
-// accumulates the gradients, then applies one Adam step. The densification
-// statistics advance once per view that sees the Gaussian, as consecutive
+// The multi-view form: a block walks the batch's views in order, lists the Gaussians each
+// view sees, sums their slots (instance v * n + i), runs that view's projection VJPs and
+// accumulates the gradients in shared memory, then applies one Adam step. The
+// densification statistics advance once per view that sees the Gaussian, as consecutive
 // single-view steps would advance them. A one-view batch reproduces
-// backward_adam_kernel's update.
-__global__ void __launch_bounds__(BWD_THREADS) backward_adam_batch_kernel(BackwardBatchArgs a) {
-    __shared__ float s_grest[BWD_THREADS][3 * MAX_REST];
-    __shared__ int s_vis[BWD_THREADS];
+// backward_adam_kernel's update. Eight street views of 100 k Gaussians: 916 -> 652 us
+// against one thread a Gaussian.
+__global__ void __launch_bounds__(NB, 768 / NB) backward_adam_batch_kernel(BackwardBatchArgs a) {
+    __shared__ VisibleList<NB> L;
+    __shared__ float s_mean[NB * 3], s_scale[NB * 3], s_quat[NB * 4], s_op[NB], s_dc[NB * 3];
+    __shared__ uint8_t s_vis[NB];
+    extern __shared__ float s_rest[];  // [NB][3 * MAX_REST], when an SH degree above 0 is in use
     if (a.skip && *a.skip) return;  // block-uniform: the step overflowed its capacity
-    const int i = blockIdx.x * BWD_THREADS + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    const bool valid = i < a.n;
-    const float b1 = a.beta1, b2 = a.beta2, eps = a.eps;
-    const uint32_t dtu = a.degrees_to_use;
-    const int active = dtu < 1 ? 0 : dtu < 2 ? 3 : dtu < 3 ? 8 : 15;  // SH bases beyond DC with gradients
-    const int used = 3 * active;
-    float *grest = s_grest[threadIdx.x];
-    for (int j = 0; j < 3 * MAX_REST; j++) grest[j] = 0.f;
-    float gm[3] = {0.f, 0.f, 0.f}, gsv[3] = {0.f, 0.f, 0.f}, gq[4] = {0.f, 0.f, 0.f, 0.f};
-    float gop = 0.f, gdc[3] = {0.f, 0.f, 0.f};
-    float st_vis = 0.f, st_gn = 0.f, st_ms = 0.f;
-    if (valid && a.vis_counts) {
-        st_vis = a.vis_counts[i];
-        st_gn = a.xys_grad_norm[i];
-        st_ms = a.max_2d_size[i];
-    }
-    bool any = false;
-    for (int v = 0; v < a.n_views; v++) {
-        const int64_t g = (int64_t)v * a.n + i;
-        const bool vis = valid && a.radii[g] > 0;
-        float s9[9];
-        warp_slot_sums(vis, (int64_t)v * a.n + (int64_t)blockIdx.x * BWD_THREADS + (threadIdx.x - lane), a.offsets,
-                       a.n_tiles, a.inv, a.slots, s9);
-        if (!vis) continue;
-        any = true;
-        const CamParams &cam = a.proj[v].cam;
-        float vm[3] = {0.f, 0.f, 0.f}, vs[3] = {0.f, 0.f, 0.f}, vq[4] = {0.f, 0.f, 0.f, 0.f};
-        V3 dir;
-        projection_vjp(cam, a.means, a.scales, a.quats, a.glob_scale, a.splats + g, i, s9, vm, vs, vq, dir);
+    const int t = threadIdx.x;
+    const int64_t g0 = (int64_t)blockIdx.x * NB;
+    const int rows = (int)min((int64_t)NB, (int64_t)a.n - g0);
+    const int active = active_bases(a.degrees_to_use), used = 3 * active;
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            gm[c] += vm[c];
-            gsv[c] += vs[c];
-            gdc[c] += SH_C0 * s9[5 + c];
-        }
+    for (int c = 0; c < 3; c++) s_mean[t * 3 + c] = s_scale[t * 3 + c] = s_dc[t * 3 + c] = 0.f;
 #pragma unroll
-        for (int c = 0; c < 4; c++) gq[c] += vq[c];
-        gop += s9[8];
-        if (active > 0) {
-            float bs[MAX_REST];
-            sh_rest_basis(dir, bs);
+    for (int c = 0; c < 4; c++) s_quat[t * 4 + c] = 0.f;
+    s_op[t] = 0.f;
+    s_vis[t] = 0;
+    if (active > 0)
+        for (int j = 0; j < 3 * MAX_REST; j++) s_rest[t * 3 * MAX_REST + j] = 0.f;
+    for (int v = 0; v < a.n_views; v++) {  // block-uniform
+        const int64_t gv = (int64_t)v * a.n + g0;
+        list_instances<NB>(L, gv, rows, a.radii, a.offsets, a.n_tiles);
+        sum_slots<NB>(L, a.inv, a.slots, nullptr);
+        __syncthreads();
+        if (t < L.count) {
+            const int li = L.idx[t], i = (int)g0 + li;
+            const int64_t g = gv + li;
+            float s9[9], vm[3], vs[3], vq[4];
 #pragma unroll
-            for (int k = 0; k < MAX_REST; k++) {
-                if (k >= active) break;
-#pragma unroll
-                for (int c = 0; c < 3; c++) grest[3 * k + c] += bs[k] * s9[5 + c];
-            }
-        }
-        st_vis += 1.0f;
-        st_gn += sqrtf(s9[0] * s9[0] + s9[1] * s9[1]);
-        st_ms = fmaxf(st_ms, (float)a.radii[g] * a.inv_max_dim[v]);
-    }
-    s_vis[threadIdx.x] = any ? 1 : 0;
-    if (valid && a.vis_counts && any) {
-        a.vis_counts[i] = st_vis;
-        a.xys_grad_norm[i] = st_gn;
-        a.max_2d_size[i] = st_ms;
-    }
-    if (valid && a.g[0]) {  // summed gradients (zero for Gaussians no view sees)
-        for (int c = 0; c < 3; c++) {
-            a.g[0][3 * (size_t)i + c] = gm[c];
-            a.g[1][3 * (size_t)i + c] = gsv[c];
-            a.g[3][3 * (size_t)i + c] = gdc[c];
-        }
-        for (int c = 0; c < 4; c++) a.g[2][4 * (size_t)i + c] = gq[c];
-        a.g[5][i] = gop;
-    }
-    const float *ss = a.adam_scalars, *bc2 = a.adam_scalars + 6;
-    if (valid && a.do_adam) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const size_t k = 3 * (size_t)i + c;
-            adam_step(a.p[0][k], a.m1[0][k], a.m2[0][k], gm[c], ss[0], b1, b2, bc2[0], eps);
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const size_t k = 3 * (size_t)i + c;
-            adam_step(a.p[1][k], a.m1[1][k], a.m2[1][k], gsv[c], ss[1], b1, b2, bc2[1], eps);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const size_t k = 4 * (size_t)i + c;
-            adam_step(a.p[2][k], a.m1[2][k], a.m2[2][k], gq[c], ss[2], b1, b2, bc2[2], eps);
-        }
-        if (a.m1[5]) adam_step(a.p[5][i], a.m1[5][i], a.m2[5][i], gop, ss[5], b1, b2, bc2[5], eps);
-        if (any) {
+            for (int c = 0; c < 9; c++) s9[c] = L.s9[li * 9 + c];
+            V3 dir;
+            projection_vjp(a.proj[v].cam, a.means, a.scales, a.quats, a.glob_scale, a.splats + g, i, s9, vm, vs, vq,
+                           dir);
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                const size_t k = 3 * (size_t)i + c;
-                adam_step(a.p[3][k], a.m1[3][k], a.m2[3][k], gdc[c], ss[3], b1, b2, bc2[3], eps);
+                s_mean[li * 3 + c] += vm[c];
+                s_scale[li * 3 + c] += vs[c];
+                s_dc[li * 3 + c] += SH_C0 * s9[5 + c];
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) s_quat[li * 4 + c] += vq[c];
+            s_op[li] += s9[8];
+            s_vis[li] = 1;
+            if (active > 0) {
+                float bs[MAX_REST];
+                sh_rest_basis(dir, bs);
+                float *r = s_rest + li * 3 * MAX_REST;
+#pragma unroll
+                for (int k = 0; k < MAX_REST; k++) {
+                    if (k >= active) break;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) r[3 * k + c] += bs[k] * s9[5 + c];
+                }
+            }
+            if (a.vis_counts) {
+                a.vis_counts[i] += 1.0f;
+                a.xys_grad_norm[i] += sqrtf(s9[0] * s9[0] + s9[1] * s9[1]);
+                a.max_2d_size[i] = fmaxf(a.max_2d_size[i], (float)a.radii[g] * a.inv_max_dim[v]);
             }
         }
+        __syncthreads();  // the list and the statistics are another thread's in the next view
     }
-    // SH rest: Adam (or the gradient) warp-cooperatively over the warp's 32 Gaussians
-    if ((!a.do_adam && !a.g[4]) || a.rest_stride <= 0) return;
-    __syncwarp();
-    const int wbase_t = threadIdx.x - lane;
-    const int64_t g0 = (int64_t)blockIdx.x * BWD_THREADS + wbase_t;
+    if (t < rows && a.g[0]) {  // summed gradients (zero for Gaussians no view sees)
+        const size_t i = (size_t)g0 + t;
+        for (int c = 0; c < 3; c++) {
+            a.g[0][3 * i + c] = s_mean[t * 3 + c];
+            a.g[1][3 * i + c] = s_scale[t * 3 + c];
+            a.g[3][3 * i + c] = s_dc[t * 3 + c];
+        }
+        for (int c = 0; c < 4; c++) a.g[2][4 * i + c] = s_quat[t * 4 + c];
+        a.g[5][i] = s_op[t];
+    }
+    const float *ss = a.adam_scalars, *bc2 = a.adam_scalars + 6;
+    const float b1 = a.beta1, b2 = a.beta2, eps = a.eps;
+    if (a.do_adam) {
+        adam_groups<NB>(a.p, a.m1, a.m2, g0, rows, s_mean, s_scale, s_quat, s_op, s_dc, s_vis, ss, bc2, b1, b2, eps);
+    }
+    // SH rest: the summed gradient rows (zero where no view saw the Gaussian), and Adam
     const int stride = a.rest_stride;
-    const int rows = (int)min((int64_t)32, (int64_t)a.n - g0);
+    if (stride <= 0) return;
+    auto grad = [&](int i, int, int, int e) { return s_rest[i * 3 * MAX_REST + e]; };
     const size_t off = (size_t)g0 * stride;
-    auto grad = [&](int r, int e) { return s_grest[wbase_t + r][e]; };
-    if (a.g[4]) {  // every row: the summed gradient where used (zero where no view saw it)
-        warp_rest_grad(a.g[4] + off, rows, stride, used, nullptr, grad);
-    }
+    if (a.g[4]) write_rest<NB>(a.g[4] + off, rows, stride, used, grad);
     if (!a.do_adam || active == 0) return;
-    warp_rest_adam<REST_UNROLL>(a.p[4] + off, a.m1[4] + off, a.m2[4] + off, rows, stride, used, s_vis + wbase_t, grad,
-                                ss[4], b1, b2, bc2[4], eps);
+    list_visible<NB>(s_vis[t] != 0, L);
+    adam_rest<NB>(a.p[4] + off, a.m1[4] + off, a.m2[4] + off, L.count, stride, used,
+                  [&](int r) { return (int)L.idx[r]; }, grad, ss[4], b1, b2, bc2[4], eps);
 }
 
 void launch_backward_adam_batch(const BackwardBatchArgs &a, cudaStream_t st) {
     if (a.n <= 0) return;
-    backward_adam_batch_kernel<<<(a.n + BWD_THREADS - 1) / BWD_THREADS, BWD_THREADS, 0, st>>>(a);
+    const size_t smem = a.degrees_to_use > 0 ? NB * 3 * MAX_REST * sizeof(float) : 0;
+    backward_adam_batch_kernel<<<(a.n + NB - 1) / NB, NB, smem, st>>>(a);
 }
 
 }  // namespace msplat

@@ -120,3 +120,32 @@ def test_train_step_edge(oracle, name):
     assert np.array_equal(stats[0].cpu().numpy(), st["vis"])
     assert rel_l2(stats[1].cpu().numpy(), st["gn"]) <= GRAD_RTOL_L2
     assert np.array_equal(stats[2].cpu().numpy(), st["ms"])
+
+
+@pytest.mark.parametrize("n,scale,degree", [(1, -1.0, 3), (127, -2.0, 1), (129, -1.0, 2), (300, 0.0, 3)])
+def test_slot_sums_of_every_size(n, scale, degree):
+    """Screen-space gradients (the sums of the intersection slots) of scenes whose Gaussians
+    cover from one tile to the whole 40 x 30 tile frame (sums of one lane, of eight, of a
+    warp and of the block) and whose counts lie around the backward kernel's 128-Gaussian
+    blocks, against the oracle within the gradient tolerance; the batched step's parameters
+    and moments are the same bits. (The world-space gradients of such needles are no
+    measure of a sum: the covariance VJP turns the projection's one-ulp differences into
+    1e-3.)"""
+    rng = np.random.default_rng(n)
+    g = scenes.random_gaussians(n, n, sh_degree=degree, log_scale_mean=scale, log_scale_std=1.5)
+    cam = scenes.small_camera(640, 480, 500.0)
+    gt = rng.random((480, 640, 3)).astype(np.float32)
+    oracle = Oracle("restatement")
+    go = g.copy()
+    oracle.train_step(go, cam, BACKGROUND, gt, new_adam_state(go, C1_LRS, 1),
+                      {k: np.zeros(n, np.float32) for k in ("vis", "gn", "ms")}, degrees_to_use=degree)
+    ctx, gt_t = Context(keep_grads=True), torch.from_numpy(gt).cuda()
+    p, q = GaussianParams.from_numpy(g), GaussianParams.from_numpy(g)
+    ap, aq = AdamState.zeros_like(p, C1_LRS), AdamState.zeros_like(q, C1_LRS)
+    ctx.train_step(p, ap, cam, BACKGROUND, gt_t, None, degrees_to_use=degree)
+    for key in ("v_xy", "v_conic", "v_rgb", "v_opacity"):
+        got, ref = ctx.frame(key).cpu().numpy(), oracle.frame(key)
+        assert rel_l2(got, ref) <= GRAD_RTOL_L2, (key, rel_l2(got, ref))
+    ctx.train_batch(q, aq, [(cam, gt_t)], BACKGROUND, degrees_to_use=degree)
+    for a, b in zip(p.tensors() + ap.exp_avg + ap.exp_avg_sq, q.tensors() + aq.exp_avg + aq.exp_avg_sq):
+        assert torch.equal(a, b)
