@@ -125,14 +125,19 @@ struct VisibleList {
     float depth[NB];    // aux mode: dL/d(view depth)
     int64_t first[NB];  // by local index: first emission index and tiles
     int tiles[NB];
-    // listed ones whose slots several lanes, or the whole block, add
-    int n_mid, n_large;
-    uint16_t mid[NB], large[NB];
-    float part[NB / 32][10];
+    // listed ones whose slots four lanes, a warp, or the whole block add
+    int n_mid, n_wide, n_large;
+    uint16_t mid[NB], wide[NB], large[NB];
     __device__ __forceinline__ void store(int i, const float p[9], float pd) {
 #pragma unroll
         for (int c = 0; c < 9; c++) s9[i * 9 + c] = p[c];
         depth[i] = pd;
+    }
+    __device__ __forceinline__ void store_share(int i, int part, const float p[3]) {  // add_share's
+        s9[i * 9 + part] = p[0];
+        s9[i * 9 + part + 4] = p[1];
+        if (part == 0) s9[i * 9 + 8] = p[2];
+        if (part == 1) depth[i] = p[2];
     }
 };
 
@@ -154,7 +159,7 @@ __device__ __forceinline__ void list_visible(bool vis, VisibleList<NB> &L) {
     if (vis) L.idx[before + __popc(m & ((1u << lane) - 1u))] = (uint16_t)threadIdx.x;
     if (threadIdx.x == 0) {
         L.count = all;
-        L.n_mid = L.n_large = 0;
+        L.n_mid = L.n_wide = L.n_large = 0;
     }
     __syncthreads();
 }
@@ -175,28 +180,32 @@ __device__ __forceinline__ bool list_instances(VisibleList<NB> &L, int64_t g0, i
 }
 
 // Sums of the 9 (with slots_depth: 10) raster-backward values over each listed
-// Gaussian's intersection slots. A Gaussian of up to SLOT_LANE_MAX tiles is one lane's,
-// of up to SLOT_GROUP_MAX SLOT_LANES neighbouring lanes' (lane l adds slots l,
-// l + SLOT_LANES, ..., the lanes' sums are added as a fixed tree), of up to
-// SLOT_WARP_MAX a warp's, and one of more (near the camera) the block's. The orders are
-// fixed, so the sums do not depend on scheduling. Every thread of the block must call
-// it; the sums are complete after the next block barrier.
+// Gaussian's intersection slots. Of up to SLOT_SERIAL tiles, every value is added slot
+// after slot; of more (near the camera: hundreds), lane l of a warp adds slots l,
+// l + 32, ... and a fixed butterfly the lanes. The orders are fixed, so the sums do not
+// depend on scheduling. Every thread of the block must call it; the sums are complete
+// after the next block barrier.
 //
 // Bound by the latency of two dependent loads a slot (its sorted position, then the slot
-// in L2), about a microsecond; a step fetches two slots a lane. One lane walking its
-// Gaussian's slots alone (34 on average in an early street view) and one warp walking
-// the 2000 of a Gaussian in front of the camera were most of the kernel's time.
-constexpr int SLOT_LANES = 8, SLOT_LANE_MAX = 8, SLOT_GROUP_MAX = 64, SLOT_WARP_MAX = 256;
+// in L2), about a microsecond. A Gaussian of up to SLOT_LANE_MAX tiles is one lane's; of
+// up to SLOT_SERIAL, four neighbouring lanes', which share out its values (two or three
+// each) and fetch SLOT_AHEAD slots before they add any; of up to SLOT_WARP_MAX, a warp's,
+// and of more the block's, whose warps share out the values. One lane walking its
+// Gaussian's slots alone (34 on average in an early street view) and one warp walking the
+// 2000 of a Gaussian in front of the camera were most of the kernel's time.
+constexpr int SLOT_LANE_MAX = 8, SLOT_SERIAL = 64, SLOT_WARP_MAX = 256, SLOT_AHEAD = 8;
 
-// A lane's share: slots l, l + step, ... of the cnt from emission index e0.
-__device__ __forceinline__ void add_slots(int l, int step, int64_t e0, int cnt, const int32_t *inv,
-                                          const float *slots, const float *slots_depth, float p[9], float &pd) {
+// All values of the slots first, first + step, ... of cnt, two slots fetched at a time.
+__device__ __forceinline__ void add_slots(int first, int step, const int32_t *pos, int cnt, const float *slots,
+                                          const float *slots_depth, float p[9], float &pd) {
 #pragma unroll
     for (int c = 0; c < 9; c++) p[c] = 0.f;
     pd = 0.f;
-    int j = l;
+    int32_t k0 = first < cnt ? pos[first] : 0, k1 = first + step < cnt ? pos[first + step] : 0;
+    int j = first;
     for (; j + step < cnt; j += 2 * step) {
-        const int32_t k0 = inv[e0 + j], k1 = inv[e0 + j + step];
+        const int32_t n0 = j + 2 * step < cnt ? pos[j + 2 * step] : 0;  // the next two's places, with these two
+        const int32_t n1 = j + 3 * step < cnt ? pos[j + 3 * step] : 0;
         const float *s0 = slots + (size_t)k0 * 9, *s1 = slots + (size_t)k1 * 9;
         float a[9], b[9];
 #pragma unroll
@@ -207,78 +216,96 @@ __device__ __forceinline__ void add_slots(int l, int step, int64_t e0, int cnt, 
 #pragma unroll
         for (int c = 0; c < 9; c++) p[c] = (p[c] + a[c]) + b[c];
         if (slots_depth) pd = (pd + slots_depth[k0]) + slots_depth[k1];
+        k0 = n0;
+        k1 = n1;
     }
     if (j < cnt) {
-        const int32_t k = inv[e0 + j];
-        const float *s = slots + (size_t)k * 9;
+        const float *s = slots + (size_t)k0 * 9;
 #pragma unroll
         for (int c = 0; c < 9; c++) p[c] += s[c];
-        if (slots_depth) pd += slots_depth[k];
+        if (slots_depth) pd += slots_depth[k0];
     }
 }
 
-// The sums of `lanes` neighbouring lanes, on each of them. Every lane of the warp calls it.
-__device__ __forceinline__ void add_lanes(int lanes, bool with_depth, float p[9], float &pd) {
-    for (int o = lanes / 2; o > 0; o >>= 1) {
+// One share of a Gaussian's sums over its slots first, first + step, ... of cnt: values
+// part and part + 4, and for part 0 value 8, for part 1 the depth.
+__device__ __forceinline__ void add_share(int part, int first, int step, const int32_t *pos, int cnt,
+                                          const float *slots, const float *slots_depth, float p[3]) {
+    p[0] = p[1] = p[2] = 0.f;
+    int32_t k[SLOT_AHEAD];
 #pragma unroll
-        for (int c = 0; c < 9; c++) p[c] += __shfl_xor_sync(0xffffffffu, p[c], o);
-        if (with_depth) pd += __shfl_xor_sync(0xffffffffu, pd, o);
+    for (int u = 0; u < SLOT_AHEAD; u++) k[u] = first + u * step < cnt ? pos[first + u * step] : 0;
+    for (int j = first; j < cnt; j += step * SLOT_AHEAD) {
+        int32_t next[SLOT_AHEAD];  // the places of the slots after these, with these
+        float v[3][SLOT_AHEAD];
+        const int jn = j + step * SLOT_AHEAD;
+#pragma unroll
+        for (int u = 0; u < SLOT_AHEAD; u++) next[u] = jn + u * step < cnt ? pos[jn + u * step] : 0;
+#pragma unroll
+        for (int u = 0; u < SLOT_AHEAD; u++) {
+            const float *s = slots + (size_t)k[u] * 9 + part;
+            const bool in = j + u * step < cnt;
+            v[0][u] = in ? s[0] : 0.f;
+            v[1][u] = in ? s[4] : 0.f;
+            v[2][u] = 0.f;
+            if (in && part == 0) v[2][u] = s[8];
+            if (in && part == 1 && slots_depth) v[2][u] = slots_depth[k[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < SLOT_AHEAD; u++)
+            if (j + u * step < cnt) {
+                p[0] += v[0][u];
+                p[1] += v[1][u];
+                p[2] += v[2][u];
+            }
+#pragma unroll
+        for (int u = 0; u < SLOT_AHEAD; u++) k[u] = next[u];
     }
 }
 
 template <int NB>
 __device__ __forceinline__ void sum_slots(VisibleList<NB> &L, const int32_t *inv, const float *slots,
                                           const float *slots_depth) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, l = lane & (SLOT_LANES - 1);
-    const bool wd = slots_depth != nullptr;
+    static_assert(NB == 128, "four warps share the values of a large Gaussian");
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     float p[9], pd;
     if (t < L.count) {
         const int i = L.idx[t], cnt = L.tiles[i];
         if (cnt <= SLOT_LANE_MAX) {
-            add_slots(0, 1, L.first[i], cnt, inv, slots, slots_depth, p, pd);
+            add_slots(0, 1, inv + L.first[i], cnt, slots, slots_depth, p, pd);
             L.store(i, p, pd);
-        } else if (cnt <= SLOT_WARP_MAX) {  // the order of either list changes no sum
-            L.mid[atomicAdd(&L.n_mid, 1)] = (uint16_t)i;
-        } else {
-            L.large[atomicAdd(&L.n_large, 1)] = (uint16_t)i;
+        } else {  // the order of a list changes no sum
+            int *n = cnt <= SLOT_SERIAL ? &L.n_mid : cnt <= SLOT_WARP_MAX ? &L.n_wide : &L.n_large;
+            uint16_t *list = cnt <= SLOT_SERIAL ? L.mid : cnt <= SLOT_WARP_MAX ? L.wide : L.large;
+            list[atomicAdd(n, 1)] = (uint16_t)i;
         }
     }
     __syncthreads();
-    for (int b = 0; b < L.n_mid; b += NB / SLOT_LANES) {  // block-uniform
-        const int li = b + t / SLOT_LANES;
-        const int i = li < L.n_mid ? L.mid[li] : -1, all = i >= 0 ? L.tiles[i] : 0;
-        const int cnt = all <= SLOT_GROUP_MAX ? all : 0;
-        add_slots(l, SLOT_LANES, i >= 0 ? L.first[i] : 0, cnt, inv, slots, slots_depth, p, pd);
-        add_lanes(SLOT_LANES, wd, p, pd);
-        if (l == 0 && cnt > 0) L.store(i, p, pd);
-        unsigned m = __ballot_sync(0xffffffffu, l == 0 && all > SLOT_GROUP_MAX);
-        while (m) {  // warp-uniform: this warp's larger ones, one after another
-            const int bi = __shfl_sync(0xffffffffu, i, __ffs(m) - 1);
-            m &= m - 1;
-            add_slots(lane, 32, L.first[bi], L.tiles[bi], inv, slots, slots_depth, p, pd);
-            add_lanes(32, wd, p, pd);
-            if (lane == 0) L.store(bi, p, pd);
+    for (int li = t / 4; li < L.n_mid; li += NB / 4) {
+        const int i = L.mid[li], part = t & 3;
+        add_share(part, 0, 1, inv + L.first[i], L.tiles[i], slots, slots_depth, p);
+        L.store_share(i, part, p);
+    }
+    __syncwarp();
+    for (int li = warp; li < L.n_wide; li += NB / 32) {  // warp-uniform
+        const int i = L.wide[li];
+        add_slots(lane, 32, inv + L.first[i], L.tiles[i], slots, slots_depth, p, pd);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int c = 0; c < 9; c++) p[c] += __shfl_xor_sync(0xffffffffu, p[c], o);
+            if (slots_depth) pd += __shfl_xor_sync(0xffffffffu, pd, o);
         }
+        if (lane == 0) L.store(i, p, pd);
     }
     for (int q = 0; q < L.n_large; q++) {  // block-uniform
         const int i = L.large[q];
-        add_slots(t, NB, L.first[i], L.tiles[i], inv, slots, slots_depth, p, pd);
-        add_lanes(32, wd, p, pd);
-        if (lane == 0) {
+        add_share(warp, lane, 32, inv + L.first[i], L.tiles[i], slots, slots_depth, p);
 #pragma unroll
-            for (int c = 0; c < 9; c++) L.part[warp][c] = p[c];
-            L.part[warp][9] = pd;
-        }
-        __syncthreads();
-        if (t == 0) {
-            for (int w = 1; w < NB / 32; w++) {
+        for (int c = 0; c < 3; c++)
 #pragma unroll
-                for (int c = 0; c < 9; c++) p[c] += L.part[w][c];
-                pd += L.part[w][9];
-            }
-            L.store(i, p, pd);
-        }
-        __syncthreads();
+            for (int o = 16; o > 0; o >>= 1) p[c] += __shfl_xor_sync(0xffffffffu, p[c], o);
+        if (lane == 0) L.store_share(i, warp, p);
     }
 }
 
@@ -404,14 +431,14 @@ __device__ __forceinline__ void adam_groups(float *const p[6], float *const m1[6
 // Adam over the SH-rest rows (`stride` floats, of which the first `used` have gradients)
 // of `rows` Gaussians: row(r) is the r-th one's local index, grad(i, base, c, e) the
 // gradient of local Gaussian i's float e = 3 base + c. A warp takes as many whole rows at
-// a time as fit three floats a lane (two of 45 floats, four of 24, ten of 9), as one flat
+// a time as fit six floats a lane (four of 45 floats, eight of 24, 21 of 9), as one flat
 // range, all loads issued before any update.
 template <int NB, typename Row, typename Grad>
 __device__ __forceinline__ void adam_rest(float *__restrict__ p, float *__restrict__ m1, float *__restrict__ m2,
                                           int rows, int stride, int used, Row row, Grad grad, float ss, float b1,
                                           float b2, float bc2, float eps) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int E = 3;
+    constexpr int E = 6;
     const int per = 32 * E / used;
     int r[E], e[E];  // the lane's floats: row within the step, float within the row
 #pragma unroll
@@ -469,9 +496,9 @@ constexpr int NB = 128;
 // Bound by the latency of its chain of phases (radii; slot positions; slots; parameters;
 // three rounds of Adam loads) and, where most Gaussians are visible and SH degree 3 is in
 // use, by issue (Adam's exact square root and divisions). Against one thread a Gaussian
-// with its slots, VJPs and Adam in one lane: a 1 M-Gaussian street step at 1600 x 1060
-// 545 -> 297 us, an early 100 k street view 100 -> 69 us, 200 k gradients with everything
-// visible 65 -> 67 us.
+// with its slots, VJPs and Adam in one lane (whose order of additions the slot sums
+// keep): a 1 M-Gaussian street step at 1600 x 1060 545 -> 345 us, an early 100 k street
+// view 100 -> 76 us, 200 k gradients with everything visible 65 -> 69 us.
 __global__ void __launch_bounds__(NB, 1024 / NB) backward_adam_kernel(BackwardArgs a) {
     __shared__ VisibleList<NB> L;
     __shared__ float s_mean[NB * 3], s_scale[NB * 3], s_quat[NB * 4], s_op[NB], s_dc[NB * 3];
@@ -597,7 +624,7 @@ void launch_backward_adam(const BackwardArgs &a, cudaStream_t st) {
 // accumulates the gradients in shared memory, then applies one Adam step. The
 // densification statistics advance once per view that sees the Gaussian, as consecutive
 // single-view steps would advance them. A one-view batch reproduces
-// backward_adam_kernel's update. Eight street views of 100 k Gaussians: 916 -> 652 us
+// backward_adam_kernel's update. Eight street views of 100 k Gaussians: 916 -> 654 us
 // against one thread a Gaussian.
 __global__ void __launch_bounds__(NB, 768 / NB) backward_adam_batch_kernel(BackwardBatchArgs a) {
     __shared__ VisibleList<NB> L;
