@@ -43,71 +43,70 @@ __device__ __forceinline__ float exp_ref(float x) { return (float)exp((double)x)
 
 // The rasterizers' exponential, exp(x) rounded once to float for x = -sigma in
 // [-5.55, 0]: Tang's table-driven method (P. T. P. Tang, ACM TOMS 15(2), 1989) in
-// double precision. x = (64 m + j) ln2 / 64 + r with |r| <= ln2 / 128, so
-// exp(x) = 2^m 2^(j/64) exp(r); exp(r) is its Taylor polynomial of degree 5 (truncation
-// below 3.5e-17 on the interval) and 2^(j/64) comes from a 64-entry table that the
-// block fills once (exp_table_init). The double result is within a few ulps of exp(x),
-// so the float it rounds to equals exp_ref's unless exp(x) lies within about 1e-15 of
-// a float rounding boundary. Valid for x in [-700, 0].
-constexpr double EXP_INV_LN2_64 = 92.33248261689366;    // 64 / ln 2
-constexpr double EXP_LN2_64_HI = 0x1.62e42fefa2000p-7;  // ln 2 / 64 to 40 bits: k * HI is exact
-constexpr double EXP_LN2_64_LO = 0x1.9ef35793c7673p-47; // ln 2 / 64 - HI
-constexpr int EXP_TABLE = 64;
+// double precision. x = (128 m + j) ln2 / 128 + r with |r| <= ln2 / 256, so
+// exp(x) = 2^m 2^(j/128) exp(r); exp(r) is a polynomial of degree 4 (1 + r s(r), s the
+// cubic through (exp(r) - 1) / r at the Chebyshev nodes of the interval: off by at most
+// 1.6e-16), and 2^m 2^(j/128) comes from a table over the range that the block fills
+// once (exp_span_init_a, a barrier, exp_span_init_b). The reduction is one fused step:
+// k times the rounding of ln2 / 128 stays below 4.5e-16 for |k| <= 1026. The double
+// result is within about 1e-15 of exp(x), so the float it rounds to equals exp_ref's
+// unless exp(x) lies that close to a float rounding boundary. (A 64-entry table needs a
+// degree 5 and two reduction steps for the same: two operations more of fifteen.)
+constexpr double EXP_INV_LN2_T = 0x1.71547652b82fep+7;    // 128 / ln 2
+constexpr double EXP_LN2_T = 0x1.62e42fefa39efp-8;     // ln 2 / 128
+constexpr double EXP_LN2_T_HI = 0x1.62e42fefa2000p-8;  // its upper 40 bits: k * HI is exact
+constexpr double EXP_LN2_T_LO = 0x1.9ef35793c7673p-48;  // ln 2 / 128 - HI
+constexpr int EXP_TABLE = 128, EXP_BITS = 7;
+constexpr int EXP_SPAN = 1040;  // covers k down to -1039 (x >= -5.62)
 
-// Every thread of the block calls it; the table is ready after the next barrier.
-__device__ __forceinline__ void exp_table_init(double *t) {
+// exp(r) - 1 over r, |r| <= ln2 / 256
+__device__ __forceinline__ double exp_poly(double r) {
+    double p = fma(r, 0x1.55555acd08c2ep-5, 0x1.55555d88e27efp-3);
+    p = fma(p, r, 0x1.fffffffffff58p-2);
+    p = fma(p, r, 0x1.ffffffffffe08p-1);
+    return fma(p, r, 1.0);
+}
+
+// k = round(x 128 / ln 2): adding 1.5 * 2^52 leaves the rounded integer in the low word
+// of the sum (exact for |k| < 2^31)
+__device__ __forceinline__ int exp_index(double x, double &k) {
+    const double shifted = fma(x, EXP_INV_LN2_T, 0x1.8p52);
+    k = shifted - 0x1.8p52;
+    return __double2loint(shifted);
+}
+
+// v 2^m, exactly, for v in [1, 2) and m in [-1020, 0]: the exponent field moved
+__device__ __forceinline__ double exp_scale(double v, int m) {
+    return __hiloint2double(__double2hiint(v) + m * (1 << 20), __double2loint(v));
+}
+
+// Every thread of the block calls each; the span is ready after the barrier that follows
+// init_b. t: EXP_TABLE doubles of scratch, read by init_b.
+__device__ __forceinline__ void exp_span_init_a(double *t) {
     for (int j = threadIdx.x; j < EXP_TABLE; j += blockDim.x) t[j] = exp2((double)j * (1.0 / EXP_TABLE));
 }
-
-__device__ __forceinline__ float exp_tab(float xf, const double *t) {
-    const double x = (double)xf;
-    // k = round(x 64 / ln 2): adding 1.5 * 2^52 leaves the rounded integer in the low
-    // word of the sum (exact for |k| < 2^31)
-    const double shifted = fma(x, EXP_INV_LN2_64, 0x1.8p52);
-    const int ki = __double2loint(shifted);
-    const double k = shifted - 0x1.8p52;
-    double r = fma(-k, EXP_LN2_64_HI, x);
-    r = fma(-k, EXP_LN2_64_LO, r);
-    double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
-    p = fma(p, r, 1.0 / 6.0);
-    p = fma(p, r, 0.5);
-    p = fma(p, r, 1.0);
-    p = fma(p, r, 1.0);
-    const double v = t[ki & (EXP_TABLE - 1)] * p;
-    const int m = ki >> 6;  // floor(ki / 64): the power of two, added to the exponent field
-    return (float)__hiloint2double(__double2hiint(v) + m * (1 << 20), __double2loint(v));
-}
-
-// The same exponential with the power of two folded into the table, for x in
-// [-5.55, 0] (-sigma over the rasterizers' range): entry i = 2^m 2^(j/64) for
-// ki = -i = 64 m + j, the old table's entry scaled exactly, so v = entry * p is the
-// old t[j] * p scaled by 2^m -- the same double, rounded to the same float -- with the
-// exponent-field arithmetic gone. Indices past the span are clamped (not reached for
-// x >= -5.55). The block fills the table in two steps with one barrier between
-// (exp_span_init_a, __syncthreads, exp_span_init_b).
-constexpr int EXP_SPAN = 520;  // covers ki = round(x 64 / ln 2) down to -519 (x >= -5.62)
-
-__device__ __forceinline__ void exp_span_init_a(double *t64) { exp_table_init(t64); }
-__device__ __forceinline__ void exp_span_init_b(double *span, const double *t64) {
-    for (int i = threadIdx.x; i < EXP_SPAN; i += blockDim.x) {
-        const int ki = -i;
-        span[i] = scalbn(t64[ki & (EXP_TABLE - 1)], ki >> 6);
-    }
+__device__ __forceinline__ void exp_span_init_b(double *span, const double *t) {
+    for (int i = threadIdx.x; i < EXP_SPAN; i += blockDim.x) span[i] = exp_scale(t[-i & (EXP_TABLE - 1)], -i >> EXP_BITS);
 }
 
 __device__ __forceinline__ float exp_span(float xf, const double *span) {
     const double x = (double)xf;
-    const double shifted = fma(x, EXP_INV_LN2_64, 0x1.8p52);
-    const int ki = __double2loint(shifted);
-    const double k = shifted - 0x1.8p52;
-    double r = fma(-k, EXP_LN2_64_HI, x);
-    r = fma(-k, EXP_LN2_64_LO, r);
-    double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
-    p = fma(p, r, 1.0 / 6.0);
-    p = fma(p, r, 0.5);
-    p = fma(p, r, 1.0);
-    p = fma(p, r, 1.0);
-    return (float)(span[min(-ki, EXP_SPAN - 1)] * p);
+    double k;
+    const int ki = exp_index(x, k);
+    const double r = fma(-k, EXP_LN2_T, x);
+    return (float)(span[min((unsigned)-ki, (unsigned)EXP_SPAN - 1u)] * exp_poly(r));
+}
+
+// The same double without a table, for the few pairs a pass evaluates so (the backward's
+// near the cut-offs, the pair counter): the span's entry computed on the spot. FAR: for x
+// down to -700, with the reduction in two steps.
+template <bool FAR = false>
+__device__ __noinline__ float exp_once(float xf) {
+    const double x = (double)xf;
+    double k;
+    const int ki = exp_index(x, k);
+    const double r = FAR ? fma(-k, EXP_LN2_T_LO, fma(-k, EXP_LN2_T_HI, x)) : fma(-k, EXP_LN2_T, x);
+    return (float)(exp_scale(exp2((double)(ki & (EXP_TABLE - 1)) * (1.0 / EXP_TABLE)), ki >> EXP_BITS) * exp_poly(r));
 }
 
 // Two float32 values in one 64-bit register pair, for sm_100's packed FP32

@@ -71,6 +71,7 @@ void launch_clamp_count(const int64_t *total, int64_t cap, int *d_n, int *overfl
 struct RasterArgs {
     int W, H, tiles_x, tiles_y;
     const int32_t *tile_start, *tile_end, *isect_gid;
+    int64_t n_isect;  // single-view frames: all entries, where the host knows them
     const Splat *splats;
     float bg[3];
     float *out_img, *final_T;

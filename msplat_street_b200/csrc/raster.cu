@@ -108,6 +108,62 @@ __device__ __forceinline__ int sub_tile_thread(int t, int q) {
     return ((4 * (q >> 1) + (q & 1) + 2 * (t >> 5)) << 5) + (t & 31);
 }
 
+// The sigma above which a pixel skips a splat of opacity o: the smaller of the float below
+// 5.55 (sigma >= 5.55 is sigma > that float) and the sigma above which
+// alpha = o exp(-sigma) < 1/255 for certain, ln(255 o) plus a margin far above the
+// roundings of logf, of the exponential and of the product -- so one compare takes both
+// decisions the exact tests would take.
+__device__ __forceinline__ float sigma_cut(float o) { return fminf(logf(255.f * o) + 1e-3f, SIGMA_SKIP); }
+
+// A forward block's shared memory: one round of FB staged splats, and the exponential's
+// table.
+//
+// LINES: with each splat's terms of sigma per column and per row of the tile (32 pairs)
+// instead of its centre and conic, so that a visit costs three operations and two loads
+// for sigma instead of eleven and one. The forward is bound by instruction issue, and a
+// splat that reaches a tile is visited by most of its eight warps: 228 -> 185 warp
+// instructions an intersection with the exponential's shorter form, an early street view
+// 271 -> 257 us, eight mixed ones 3224 -> 3060. Whole-tile blocks of up to 128 staged
+// splats take it (42 KB a block, four blocks per SM); smaller blocks have fewer warps to
+// share the terms, and their occupancy would pay for the space. Two kinds of frames do
+// without as well (fwd_lines): those of fewer tiles than the GPU has places for, where a
+// block's own latency counts, which the terms' extra step lengthens (256 tiles: 40
+// against 43 us); and those of long lists, whose small splats reach few of a tile's warps
+// before its pixels are done (1600 entries a tile at 800 x 600: the frame 3 us slower
+// with the terms; 575 a tile: the 14 us faster of above).
+template <int FB, bool LINES>
+struct FwdGeom {
+    float4 axis[2][FB];   // (x, a / 2, b), (y, c / 2, 1)
+    float2 line[FB][32];  // columns (a/2 dx dx, b dx), then rows (c/2 dy dy, dy)
+};
+template <int FB>
+struct FwdGeom<FB, false> {
+    float4 geom[FB];  // x, y, a / 2, b
+    float cz[FB];     // c / 2
+};
+template <int FB, int NT>
+constexpr bool can_lines = NT == FWD_THREADS && FB <= 128;
+constexpr int LINES_MIN_TILES = 4 * 148, LINES_MAX_LIST = 1024;
+inline bool fwd_lines(int tiles, int64_t isects) {
+    return tiles >= LINES_MIN_TILES && isects <= (int64_t)LINES_MAX_LIST * tiles;
+}
+template <int FB, bool LINES>
+struct FwdStage : FwdGeom<FB, LINES> {
+    float4 colour[FB];  // colours as staged_colour leaves them, depth
+    float2 cut[FB];     // opacity, sigma_cut
+    double espan[EXP_SPAN];
+    uint8_t mask[FB];   // warp_block_mask
+    unsigned alive;     // the warps with unfinished pixels (LINES)
+    // the exponential's table; ready after the next block barrier
+    __device__ __forceinline__ void init() {
+        static_assert(sizeof(colour) >= EXP_TABLE * sizeof(double), "scratch for the table's first octave");
+        double *t = reinterpret_cast<double *>(colour);
+        exp_span_init_a(t);
+        __syncthreads();
+        exp_span_init_b(espan, t);
+    }
+};
+
 // One 16x16 tile: `tile` indexes tile_start / tile_end (a global tile id in a batch),
 // (tx, ty) is its position in its view. Every thread of the block must call it.
 // NT, q: the block runs sub-block q of the tile with NT threads (sub_tile_thread), each
@@ -118,12 +174,12 @@ __device__ __forceinline__ int sub_tile_thread(int t, int q) {
 // (rasterize_forward_aux, core/cpu/msplat_cpu.cpp:574-626 with f.aux).
 // CHUNK: composite only piece `chunk` of the list (ck->chunk_len long) from T = 1 and
 // write the piece's transmittance, colour and last contributor to item `item`.
-template <int FB, bool AUX = false, bool CHUNK = false, bool TS = false, int NT = FWD_THREADS>
-__device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, int tx, int ty, float4 *s0,
-                                                float4 *s1, float4 *s2, uint8_t *sm, const double *espan,
+template <int FB, bool AUX, bool CHUNK, bool TS, int NT, bool LINES>
+__device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, int tx, int ty, FwdStage<FB, LINES> &s,
                                                 const ChunkArgs *ck = nullptr, int item = 0, int chunk = 0,
                                                 int q = 0) {
     static_assert(!CHUNK || NT == FWD_THREADS, "depth pieces are composited by whole-tile blocks");
+    static_assert(!LINES || can_lines<FB, NT>, "a warp stages FB / 8 splats, a lane each");
     const int g = sub_tile_thread<NT>(threadIdx.x, q);  // this thread's place in the tile
     int lx, ly;
     tile_pixel(g, lx, ly);
@@ -142,39 +198,82 @@ __device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, i
     const size_t npix = (size_t)a.W * a.H;
     const size_t pid = inside ? (size_t)py * a.W + px : 0;
     int stored = 0;  // contributions seen (stored-transmittance mode)
+    // LINES: a warp whose pixels are all done leaves s.alive, and splats get their terms
+    // for the others only (a stale s.alive costs the terms of a splat nobody visits).
+    bool left = false;
+    if (LINES && threadIdx.x == 0) s.alive = 0xffu;
     for (int b0 = start; b0 < end; b0 += FB) {
+        if (LINES && b0 > start && !left && __all_sync(0xffffffffu, done)) {  // warp-uniform
+            if (lane == 0) atomicAnd(&s.alive, ~(1u << w));
+            left = true;
+        }
         if (__syncthreads_count(done) == NT) break;
-        for (int si = threadIdx.x; si < FB; si += NT) {
-            const int k = b0 + si;
-            if (k >= end) break;
-            const float4 *rec = reinterpret_cast<const float4 *>(a.splats + a.isect_gid[k]);
-            const float4 A = rec[0], B = rec[1], C = rec[2];
-            // the conic's diagonal halved: 0.5 (a dx dx + c dy dy) == (a/2) dx dx +
-            // (c/2) dy dy bit for bit (scaling by 2^-1 commutes with each rounding)
-            s0[si] = make_float4(A.x, A.y, 0.5f * A.z, A.w);
-            s1[si] = make_float4(0.5f * B.x, B.y, staged_colour(B.z), staged_colour(B.w));
-            // z: the sigma above which the pixel skips the splat -- the smaller of the
-            // float below 5.55 (sigma >= 5.55 is sigma > that float) and the sigma above
-            // which alpha = o exp(-sigma) < 1/255 for certain, ln(255 o) plus a margin
-            // far above the roundings of logf, of the exponential and of the product --
-            // so one compare takes both decisions the exact tests would take
-            s2[si] = make_float4(staged_colour(C.x), C.y, fminf(logf(255.f * B.y) + 1e-3f, SIGMA_SKIP), C.w);
-            sm[si] = (uint8_t)warp_block_mask(A, C, tx, ty);
+        if constexpr (LINES) {
+            // a warp stages FB / 8 splats: their records, then each one's 16 column and
+            // 16 row terms of sigma, a lane each
+            constexpr int PER = FB / (NT / 32);
+            const int wl = threadIdx.x >> 5, si = wl * PER + lane, k = b0 + si;
+            bool live = false;
+            if (lane < PER && k < end) {
+                const float4 *rec = reinterpret_cast<const float4 *>(a.splats + a.isect_gid[k]);
+                const float4 A = rec[0], B = rec[1], C = rec[2];
+                s.axis[0][si] = make_float4(A.x, 0.5f * A.z, A.w, 0.f);
+                s.axis[1][si] = make_float4(A.y, 0.5f * B.x, 1.f, 0.f);
+                s.cut[si] = make_float2(B.y, sigma_cut(B.y));
+                s.colour[si] = make_float4(staged_colour(B.z), staged_colour(B.w), staged_colour(C.x), C.y);
+                const uint32_t m = warp_block_mask(A, C, tx, ty) & s.alive;
+                s.mask[si] = (uint8_t)m;
+                live = m != 0u;
+            }
+            unsigned todo = __ballot_sync(0xffffffffu, live);
+            __syncwarp();
+            const int axis = lane >> 4;
+            const float origin = (float)((axis ? ty : tx) * TILE + (lane & 15));
+            while (todo) {  // warp-uniform
+                const int j = wl * PER + __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const float4 p = s.axis[axis][j];
+                const float d = p.x - origin;
+                s.line[j][lane] = make_float2(p.y * d * d, p.z * d);
+            }
+        } else {
+            for (int si = threadIdx.x; si < FB; si += NT) {
+                const int k = b0 + si;
+                if (k >= end) break;
+                const float4 *rec = reinterpret_cast<const float4 *>(a.splats + a.isect_gid[k]);
+                const float4 A = rec[0], B = rec[1], C = rec[2];
+                // the conic's diagonal halved: 0.5 (a dx dx + c dy dy) == (a/2) dx dx +
+                // (c/2) dy dy bit for bit (scaling by 2^-1 commutes with each rounding)
+                s.geom[si] = make_float4(A.x, A.y, 0.5f * A.z, A.w);
+                s.cz[si] = 0.5f * B.x;
+                s.cut[si] = make_float2(B.y, sigma_cut(B.y));
+                s.colour[si] = make_float4(staged_colour(B.z), staged_colour(B.w), staged_colour(C.x), C.y);
+                s.mask[si] = (uint8_t)warp_block_mask(A, C, tx, ty);
+            }
         }
         __syncthreads();
         const int cnt = min(FB, end - b0);
         // this warp's splats in list order: 32 mask bits per ballot, then one per hit
         for (int base = 0; base < cnt; base += 32) {
             const int jl = base + lane;
-            unsigned bits = __ballot_sync(0xffffffffu, jl < cnt && ((sm[jl] >> w) & 1u));
+            unsigned bits = __ballot_sync(0xffffffffu, jl < cnt && ((s.mask[jl] >> w) & 1u));
             while (bits && !done) {
                 const int j = base + __ffs(bits) - 1;
                 bits &= bits - 1u;
-                const float4 A = s0[j], B = s1[j], C = s2[j];
-                const float dx = A.x - fpx, dy = A.y - fpy;
-                const float sigma = (A.z * dx * dx + B.x * dy * dy) + A.w * dx * dy;  // A.z, B.x halved
-                if (sigma < 0.f || sigma > C.z) continue;
-                const float alpha = fminf(0.999f, B.y * exp_span(-sigma, espan));
+                // sigma = (a/2 dx dx + c/2 dy dy) + b dx dy in the reference's roundings; a
+                // column's pixels share a/2 dx dx and b dx, a row's c/2 dy dy and dy
+                float sigma;
+                if constexpr (LINES) {
+                    const float2 cx = s.line[j][lx], cy = s.line[j][TILE + ly];
+                    sigma = (cx.x + cy.x) + cx.y * cy.y;
+                } else {
+                    const float4 A = s.geom[j];
+                    const float dx = A.x - fpx, dy = A.y - fpy;
+                    sigma = (A.z * dx * dx + s.cz[j] * dy * dy) + A.w * dx * dy;
+                }
+                const float2 cut = s.cut[j];
+                if (sigma < 0.f || sigma > cut.y) continue;
+                const float alpha = fminf(0.999f, cut.x * exp_span(-sigma, s.espan));
                 if (alpha < 1.f / 255.f) continue;
                 const float nT = T * (1.f - alpha);
                 if (nT <= 1e-4f) {
@@ -187,10 +286,11 @@ __device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, i
                     stored++;
                 }
                 const float vis = alpha * T;
-                cr = B.z * vis + cr;  // staged colours: max(raw + 0.5, 0)
-                cg = B.w * vis + cg;
-                cb = C.x * vis + cb;
-                if (AUX) depth += C.y * vis;
+                const float4 C = s.colour[j];
+                cr = C.x * vis + cr;  // staged colours: max(raw + 0.5, 0)
+                cg = C.y * vis + cg;
+                cb = C.z * vis + cb;
+                if (AUX) depth += C.w * vis;
                 T = nT;
                 last = b0 + j;
             }
@@ -235,18 +335,15 @@ __device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, i
 
 // One block per sub-block of a tile (NT threads: the whole 16 x 16 tile, a 16 x 8
 // half or an 8 x 8 quarter; blocks SUB * t .. SUB * t + SUB - 1 share tile t's list).
-template <int FB, bool AUX = false, bool TS = false, int NT = FWD_THREADS>
+template <int FB, bool AUX, bool TS, int NT, bool LINES>
 __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_kernel(RasterArgs a) {
     constexpr int SUB = FWD_THREADS / NT;
-    __shared__ float4 s0[FB], s1[FB], s2[FB];
-    __shared__ uint8_t sm[FB];
-    __shared__ double et64[EXP_TABLE], espan[EXP_SPAN];
-    exp_span_init_a(et64);
-    __syncthreads();
-    exp_span_init_b(espan, et64);  // ready after the tile's first barrier
+    extern __shared__ __align__(16) unsigned char fwd_smem[];
+    FwdStage<FB, LINES> &s = *reinterpret_cast<FwdStage<FB, LINES> *>(fwd_smem);
+    s.init();  // ready after the tile's first barrier
     const int tile = blockIdx.x / SUB;
-    raster_fwd_tile<FB, AUX, false, TS, NT>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s0, s1, s2, sm, espan,
-                                            nullptr, 0, 0, blockIdx.x % SUB);
+    raster_fwd_tile<FB, AUX, false, TS, NT, LINES>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s, nullptr, 0, 0,
+                                                   blockIdx.x % SUB);
 }
 
 // Persistent forward over the tiles of a batch of views (each with its own scene,
@@ -259,14 +356,12 @@ __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_kernel(Ra
 template <int FB, int NT>
 __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_batch_kernel(const BatchDesc d, int *counter) {
     constexpr int SUB = FWD_THREADS / NT;
-    __shared__ float4 s0[FB], s1[FB], s2[FB];
-    __shared__ uint8_t sm[FB];
+    constexpr bool LINES = can_lines<FB, NT>;
+    extern __shared__ __align__(16) unsigned char fwd_smem[];
+    FwdStage<FB, LINES> &s = *reinterpret_cast<FwdStage<FB, LINES> *>(fwd_smem);
     __shared__ int s_item, s_lt;
     __shared__ RasterArgs s_args;  // the tile's view, read from shared memory (keeps registers down)
-    __shared__ double et64[EXP_TABLE], espan[EXP_SPAN];
-    exp_span_init_a(et64);
-    __syncthreads();
-    exp_span_init_b(espan, et64);  // ready after the loop's first barrier
+    s.init();  // ready after the loop's first barrier
     const int total_items = d.tile_off[d.n_views] * SUB;  // read on the device: the launch is graph-capturable
     for (;;) {
         __syncthreads();  // the previous item's shared state is no longer read
@@ -283,8 +378,8 @@ __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_batch_ker
         __syncthreads();
         const int it = s_item, lt = s_lt;
         if (it >= total_items) break;
-        raster_fwd_tile<FB, false, false, false, NT>(s_args, it / SUB, lt % s_args.tiles_x, lt / s_args.tiles_x, s0,
-                                                     s1, s2, sm, espan, nullptr, 0, 0, it % SUB);
+        raster_fwd_tile<FB, false, false, false, NT, LINES>(s_args, it / SUB, lt % s_args.tiles_x,
+                                                            lt / s_args.tiles_x, s, nullptr, 0, 0, it % SUB);
     }
 }
 
@@ -300,11 +395,14 @@ int resident_grid(K kernel, size_t smem, int threads = TILE_PIX) {
 
 template <int FB, int NT>
 void fwd_batch_launch(const BatchDesc &d, int tiles_hint, int *d_counter, cudaStream_t st) {
-    // once per variant and shape, thread-safe
-    static const int grid = resident_grid(raster_fwd_batch_kernel<FB, NT>, 0, NT);
+    constexpr size_t smem = sizeof(FwdStage<FB, can_lines<FB, NT>>);
+    static const int grid = [] {  // once per variant and shape, thread-safe
+        cudaFuncSetAttribute(raster_fwd_batch_kernel<FB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return resident_grid(raster_fwd_batch_kernel<FB, NT>, smem, NT);
+    }();
     const int items = tiles_hint * (FWD_THREADS / NT);
     const int g = tiles_hint > 0 ? std::min(grid, items) : grid;
-    raster_fwd_batch_kernel<FB, NT><<<g, NT, 0, st>>>(d, d_counter);
+    raster_fwd_batch_kernel<FB, NT><<<g, NT, smem, st>>>(d, d_counter);
 }
 
 template <int NT>
@@ -403,8 +501,8 @@ __device__ __forceinline__ void bwd_warp_sums(const float *mypb, float *red, uin
 // colour cotangent, so one running scalar replaces the three-channel buffer.
 template <int BB, int SB, bool AUX = false, bool CHUNK = false, bool TS = false>
 __device__ __forceinline__ void raster_bwd_tile(const RasterBwdArgs &a, int tile, int tx, int ty, float4 *smem4,
-                                                int &kmax, const double *etab, const ChunkArgs *ck = nullptr,
-                                                int item = 0, int chunk = 0) {
+                                                int &kmax, const ChunkArgs *ck = nullptr, int item = 0,
+                                                int chunk = 0) {
     constexpr int NG = AUX ? 10 : 9;
     constexpr int SUB = SB, SUB_OUT = SB * NG;
     static_assert(BB <= BWD_THREADS, "one staging thread per splat");
@@ -534,7 +632,7 @@ __device__ __forceinline__ void raster_bwd_tile(const RasterBwdArgs &a, int tile
                         const float va_fast = B.y * __expf(-sigma);
                         float alpha = fminf(0.999f, va_fast);
                         if (fabsf(va_fast - 1.f / 255.f) <= 1e-5f * (1.f / 255.f) || fabsf(va_fast - 0.999f) <= 1e-5f)
-                            alpha = fminf(0.999f, B.y * exp_tab(-sigma, etab));
+                            alpha = fminf(0.999f, B.y * exp_once(-sigma));
                         if (alpha >= 1.f / 255.f) {
                             hit[i] = true;
                             al[i] = alpha;
@@ -666,10 +764,8 @@ template <int BB, int SB, bool AUX = false, bool TS = false>
 __global__ void __launch_bounds__(BWD_THREADS, BB <= 64 ? 6 : 5) raster_bwd_kernel(RasterBwdArgs a) {
     extern __shared__ __align__(16) float4 smem4[];
     __shared__ int kmax;
-    __shared__ double etab[EXP_TABLE];
-    exp_table_init(etab);  // ready after the tile's first barrier
     const int tile = blockIdx.x;
-    raster_bwd_tile<BB, SB, AUX, false, TS>(a, tile, tile % a.tiles_x, tile / a.tiles_x, smem4, kmax, etab);
+    raster_bwd_tile<BB, SB, AUX, false, TS>(a, tile, tile % a.tiles_x, tile / a.tiles_x, smem4, kmax);
 }
 
 // Persistent backward over the tiles of a batch of views, pulling global tile ids
@@ -681,8 +777,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 5) raster_bwd_batch_kernel(const 
     extern __shared__ __align__(16) float4 smem4[];
     __shared__ int kmax, s_tile, s_lt;
     __shared__ RasterBwdArgs s_args;  // the tile's view, read from shared memory (keeps registers down)
-    __shared__ double etab[EXP_TABLE];
-    exp_table_init(etab);  // ready after the loop's first barrier
     const int total_tiles = tile_off[n_views];
     for (;;) {
         if (threadIdx.x == 0) {
@@ -697,14 +791,21 @@ __global__ void __launch_bounds__(BWD_THREADS, 5) raster_bwd_batch_kernel(const 
         __syncthreads();
         const int t = s_tile, lt = s_lt;
         if (t >= total_tiles) break;
-        raster_bwd_tile<BB, SB>(s_args, t, lt % s_args.tiles_x, lt / s_args.tiles_x, smem4, kmax, etab);
+        raster_bwd_tile<BB, SB>(s_args, t, lt % s_args.tiles_x, lt / s_args.tiles_x, smem4, kmax);
         __syncthreads();  // the tile's shared state is free before thread 0 claims the next tile
     }
 }
 
-template <int FB, bool AUX, bool TS, int NT>
+template <int FB, bool AUX, bool TS, int NT, bool LINES = false>
 void fwd_launch(const RasterArgs &a, int T, cudaStream_t st) {
-    raster_fwd_kernel<FB, AUX, TS, NT><<<T * (FWD_THREADS / NT), NT, 0, st>>>(a);
+    constexpr size_t smem = sizeof(FwdStage<FB, LINES>);
+    static const bool attr = [] {  // once per instance, thread-safe
+        cudaFuncSetAttribute(raster_fwd_kernel<FB, AUX, TS, NT, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
+        return true;
+    }();
+    (void)attr;
+    raster_fwd_kernel<FB, AUX, TS, NT, LINES><<<T * (FWD_THREADS / NT), NT, smem, st>>>(a);
 }
 
 template <int FB, bool AUX, bool TS>
@@ -712,7 +813,10 @@ void fwd_launch_shape(const RasterArgs &a, int T, cudaStream_t st, int shape) {
     switch (shape_index(shape)) {
         case 1: fwd_launch<FB, AUX, TS, FWD_THREADS / 2>(a, T, st); break;
         case 2: fwd_launch<FB, AUX, TS, FWD_THREADS / 4>(a, T, st); break;
-        default: fwd_launch<FB, AUX, TS, FWD_THREADS>(a, T, st); break;
+        default:
+            if (fwd_lines(T, a.n_isect)) fwd_launch<FB, AUX, TS, FWD_THREADS, can_lines<FB, FWD_THREADS>>(a, T, st);
+            else fwd_launch<FB, AUX, TS, FWD_THREADS>(a, T, st);
+            break;
     }
 }
 
@@ -817,9 +921,6 @@ void launch_raster_bwd_batch(const RasterBwdArgs *d_views, const int *d_tile_off
 // list's end; rasterize_backward (:959-1031) walks from min(final_idx, end - 1) down
 // to the start. out[0] += forward pairs, out[1] += backward pairs.
 __global__ void __launch_bounds__(TILE_PIX) pair_count_kernel(RasterArgs a, unsigned long long *out) {
-    __shared__ double etab[EXP_TABLE];
-    exp_table_init(etab);
-    __syncthreads();
     const int tile = blockIdx.x, tx = tile % a.tiles_x, ty = tile / a.tiles_x;
     int lx, ly;
     tile_pixel(threadIdx.x, lx, ly);
@@ -837,7 +938,7 @@ __global__ void __launch_bounds__(TILE_PIX) pair_count_kernel(RasterArgs a, unsi
             const float dx = A.x - (float)px, dy = A.y - (float)py;
             const float sigma = 0.5f * (A.z * dx * dx + B.x * dy * dy) + A.w * dx * dy;
             if (sigma < 0.f || sigma >= 5.55f) continue;
-            if (fminf(0.999f, B.y * exp_tab(-sigma, etab)) < 1.f / 255.f) continue;
+            if (fminf(0.999f, B.y * exp_once(-sigma)) < 1.f / 255.f) continue;
             stop = k + 1;
             break;
         }
@@ -854,20 +955,24 @@ __global__ void __launch_bounds__(TILE_PIX) pair_count_kernel(RasterArgs a, unsi
     }
 }
 
-// The rasterizers' exponential over n inputs (test hook for exp_span / exp_tab
-// against exp_ref).
+// The rasterizers' exponential over n inputs (test hook).
 __global__ void exp_tab_kernel(const float *x, int64_t n, float *out) {
-    __shared__ double etab[EXP_TABLE], espan[EXP_SPAN];
-    exp_span_init_a(etab);
+    __shared__ double first[EXP_TABLE], espan[EXP_SPAN];
+    exp_span_init_a(first);
     __syncthreads();
-    exp_span_init_b(espan, etab);
+    exp_span_init_b(espan, first);
     __syncthreads();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        // over the rasterizers' range [-5.55, 0] the forward's span-table form, NaN
-        // wherever it differs from the 64-entry form the backward uses (the two are the
-        // same function by construction); below it the 64-entry form
-        const float xi = x[i], v = exp_tab(xi, etab);
-        out[i] = xi < -5.55f ? v : (exp_span(xi, espan) == v ? v : __int_as_float(0x7fc00000));
+        // over the rasterizers' range [-5.55, 0] the forward's table form, NaN wherever it
+        // differs from the form the backward uses (the same function by construction);
+        // below it the latter with the two-step reduction
+        const float xi = x[i];
+        if (xi < -5.55f) {
+            out[i] = exp_once<true>(xi);
+        } else {
+            const float v = exp_once(xi);
+            out[i] = exp_span(xi, espan) == v ? v : __int_as_float(0x7fc00000);
+        }
     }
 }
 
@@ -917,17 +1022,15 @@ __device__ __forceinline__ int chunk_tile(const int32_t *first, int T, int i) {
 
 template <int FB>
 __global__ void __launch_bounds__(FWD_THREADS, 4) raster_fwd_chunk_kernel(RasterArgs a, ChunkArgs c) {
-    __shared__ float4 s0[FB], s1[FB], s2[FB];
-    __shared__ uint8_t sm[FB];
+    extern __shared__ __align__(16) unsigned char fwd_smem[];
+    constexpr bool LINES = can_lines<FB, FWD_THREADS>;
+    FwdStage<FB, LINES> &s = *reinterpret_cast<FwdStage<FB, LINES> *>(fwd_smem);
     const int T = a.tiles_x * a.tiles_y, item = blockIdx.x;
     if (item >= c.first[T]) return;  // block-uniform
     const int tile = chunk_tile(c.first, T, item);
-    __shared__ double et64[EXP_TABLE], espan[EXP_SPAN];
-    exp_span_init_a(et64);
-    __syncthreads();
-    exp_span_init_b(espan, et64);  // ready after the tile's first barrier
-    raster_fwd_tile<FB, false, true>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s0, s1, s2, sm, espan, &c, item,
-                                     item - c.first[tile]);
+    s.init();  // ready after the tile's first barrier
+    raster_fwd_tile<FB, false, true, false, FWD_THREADS, LINES>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s, &c,
+                                                                item, item - c.first[tile]);
 }
 
 // rasterize_forward_merge_kernel (.metal:2741-2808): per pixel, the tile's pieces front
@@ -968,7 +1071,13 @@ __global__ void __launch_bounds__(TILE_PIX) chunk_merge_kernel(RasterArgs a, Chu
 
 template <int FB>
 void fwd_chunk_launch(const RasterArgs &a, const ChunkArgs &c, int64_t items, cudaStream_t st) {
-    raster_fwd_chunk_kernel<FB><<<(unsigned)items, FWD_THREADS, 0, st>>>(a, c);
+    constexpr size_t smem = sizeof(FwdStage<FB, can_lines<FB, FWD_THREADS>>);
+    static const bool attr = [] {
+        cudaFuncSetAttribute(raster_fwd_chunk_kernel<FB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return true;
+    }();
+    (void)attr;
+    raster_fwd_chunk_kernel<FB><<<(unsigned)items, FWD_THREADS, smem, st>>>(a, c);
 }
 
 void launch_raster_fwd_chunked(const RasterArgs &a, const ChunkArgs &c, int64_t item_cap, cudaStream_t st,
@@ -1020,9 +1129,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 5) raster_bwd_chunk_kernel(Raster
     const int T = a.tiles_x * a.tiles_y, item = blockIdx.x;
     if (item >= c.first[T]) return;  // block-uniform
     const int tile = chunk_tile(c.first, T, item);
-    __shared__ double etab[EXP_TABLE];
-    exp_table_init(etab);  // ready after the tile's first barrier
-    raster_bwd_tile<BB, SB, false, true>(a, tile, tile % a.tiles_x, tile / a.tiles_x, smem4, kmax, etab, &c,
+    raster_bwd_tile<BB, SB, false, true>(a, tile, tile % a.tiles_x, tile / a.tiles_x, smem4, kmax, &c,
                                          item, item - c.first[tile]);
 }
 
