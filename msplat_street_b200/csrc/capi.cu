@@ -92,7 +92,7 @@ SkyArgs sky_args(const msplat_cuda_prior &p, const CamParams &cam) {
 
 // Projection, binning and forward rasterization: the shared forward of render and
 // train (core/cpu/msplat_cpu.cpp:629-657). One host synchronisation reads the
-// intersection count, which sizes the sort. With a prior whose aux flag is set, the
+// intersection count, which sizes the lists. With a prior whose aux flag is set, the
 // aux rasterizer also writes the expected-depth numerator and the per-pixel
 // background, sampled from the learned sky when one is set.
 // The depth-chunked planes of the current frame (ctx->n_isect intersections over T
@@ -163,6 +163,21 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
         bg_img = bi;
     }
 
+    BinArgs ba{};
+    ba.n = n;
+    ba.tiles_x = cam.tiles_x;
+    ba.tiles_y = cam.tiles_y;
+    ba.chunks = bin_chunks(n, bin_chunk_len(n, T));
+    ba.tile_cap = T;
+    bin_plan(ba);
+    DepthScratch ds;
+    if (int r = ensure_bin_scratch(ctx, n, (int64_t)ba.chunks * T, ds, ba)) return r;
+    ba.splats = splats;
+    ba.aabb = aabb;
+    ba.n_tiles = n_tiles;
+    ba.tile_start = tile_start;
+    ba.tile_end = tile_end;
+
     ProjectArgs pa;
     pa.n = n;
     pa.means = means;
@@ -178,25 +193,25 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     pa.radii = radii;
     pa.aabb = aabb;
     pa.n_tiles = n_tiles;
-    DepthScratch ds;
-    if (int r = ensure_depth_scratch(ctx, n, ds)) return r;
+    pa.depth_keys = ds.keys[0];
+    pa.depth_vals = ds.vals[0];
     ctx->timer.reset_marks();
     ctx->timer.mark(0, st);
     launch_project(pa, st);
-    launch_depth_offsets(n, splats, n_tiles, ds, offsets, d_total, scan_part, st);
+    launch_depth_order(ba, ds, scan_part, d_total, st);
     CUDA_TRY(cudaMemcpyAsync(ctx->h_total, d_total, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     if (!ctx->total_ev) CUDA_TRY(cudaEventCreateWithFlags(&ctx->total_ev, cudaEventDisableTiming));
     CUDA_TRY(cudaEventRecord(ctx->total_ev, st));
-    // The key emission needs the count only for its buffers' size: it is queued before
-    // the host waits for the count, into the buffers as they are (entries past their
-    // capacity dropped), so the device runs it while the host reads the count and
-    // queues the rest; when the buffers were too small it runs again below.
     ctx->timer.mark(1, st);
-    const int64_t cap0 = (int64_t)std::min({ctx->keys[0].bytes, ctx->vals[0].bytes, ctx->emit_gid.bytes}) / 4;
-    if (cap0 > 0 && n > 0)
-        launch_emit_keys(n, splats, aabb, n_tiles, offsets, cam.tiles_x, cam.tiles_y,
-                         reinterpret_cast<uint32_t *>(ctx->keys[0].ptr), reinterpret_cast<uint32_t *>(ctx->vals[0].ptr),
-                         reinterpret_cast<int32_t *>(ctx->emit_gid.ptr), st, cap0);
+    launch_bin_count(ba, offsets, st);
+    // The lists are written before the host waits for the count, into the buffers as they
+    // are (entries past their capacity dropped), so the device runs on while the host
+    // reads the count and queues the rest; when the buffers were too small they are
+    // written again below.
+    const int64_t cap0 = (int64_t)std::min(ctx->isect_gid.bytes, ctx->inv.bytes) / 4;
+    if (cap0 > 0)
+        launch_bin_emit(ba, reinterpret_cast<int32_t *>(ctx->isect_gid.ptr), reinterpret_cast<int32_t *>(ctx->inv.ptr),
+                        cap0, st);
     CUDA_TRY(cudaEventSynchronize(ctx->total_ev));
     const int64_t n_isect = *ctx->h_total;
     if (n_isect > (int64_t)INT32_MAX)
@@ -205,24 +220,9 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ctx->n_isect = n_isect;
     const bool emitted = cap0 > 0 && n_isect <= cap0;
     if (!emitted) CUDA_TRY(cudaStreamSynchronize(st));  // the early emission is done before buffers move
-    ENSURE(ctx->keys[0], n_isect, uint32_t, k0);
-    ENSURE(ctx->keys[1], n_isect, uint32_t, k1);
-    ENSURE(ctx->vals[0], n_isect, uint32_t, v0);
-    ENSURE(ctx->vals[1], n_isect, uint32_t, v1);
-    ENSURE(ctx->emit_gid, n_isect, int32_t, emit_gid);
     ENSURE(ctx->isect_gid, n_isect, int32_t, isect_gid);
     ENSURE(ctx->inv, n_isect, int32_t, inv);
-    ENSURE(ctx->radix_scratch, radix_scratch_bytes((int)n_isect), unsigned char, rscratch);
-
-    if (!emitted)
-        launch_emit_keys(n, splats, aabb, n_tiles, offsets, cam.tiles_x, cam.tiles_y, k0, v0, emit_gid, st);
-    uint32_t *kk[2] = {k0, k1};
-    uint32_t *vv[2] = {v0, v1};
-    const int cur = radix_sort_pairs32(kk, vv, (int)n_isect, ceil_log2(std::max(T, 1)), rscratch, st);
-    ctx->sorted = cur;
-    ctx->gid_in_vals = false;
-    launch_tile_ranges(kk[cur], (int)n_isect, T, tile_start, tile_end, st);
-    launch_isect_map(vv[cur], (int)n_isect, emit_gid, isect_gid, inv, st);
+    if (!emitted) launch_bin_emit(ba, isect_gid, inv, n_isect, st);
 
     RasterArgs ra{};
     ra.W = (int)cam.width;
@@ -306,14 +306,30 @@ int forward_batch(msplat_cuda_ctx *ctx, int nv, const msplat_cuda_view *views) {
                     (long long)nt);
     const int n = (int)ni, T = (int)nt;
 
-    // staging layout: ProjectArgs[nv] | RasterArgs[nv] | inst_off, tile_off [nv+1] | tiles_x, tiles_y [nv]
+    // staging layout: ProjectArgs[nv] | RasterArgs[nv] | count_off [nv] | inst_off, tile_off, chunk_off [nv+1] |
+    // tiles_x, tiles_y [nv]
     const size_t o_proj = 0;
     const size_t o_ras = align_up(o_proj + nv * sizeof(ProjectArgs), 256);
-    const size_t o_inst = align_up(o_ras + nv * sizeof(RasterArgs), 256);
+    const size_t o_cnt = align_up(o_ras + nv * sizeof(RasterArgs), 256);
+    const size_t o_inst = o_cnt + nv * sizeof(int64_t);
     const size_t o_toff = o_inst + (nv + 1) * sizeof(int);
-    const size_t o_tx = o_toff + (nv + 1) * sizeof(int);
+    const size_t o_chk = o_toff + (nv + 1) * sizeof(int);
+    const size_t o_tx = o_chk + (nv + 1) * sizeof(int);
     const size_t o_ty = o_tx + nv * sizeof(int);
     const size_t bytes = o_ty + nv * sizeof(int);
+    BinArgs ba{};
+    ba.n = n;
+    int64_t most_tiles = 0, counts_len = 0;
+    for (int v = 0; v < nv; v++)
+        most_tiles = std::max(most_tiles, (int64_t)((views[v].img_width + TILE - 1) / TILE) *
+                                              ((views[v].img_height + TILE - 1) / TILE));
+    const int chunk_len = bin_chunk_len(n, most_tiles);
+    for (int v = 0; v < nv; v++) {
+        const msplat_cuda_view &w = views[v];
+        const int c = bin_chunks(w.num_points, chunk_len);
+        ba.chunks += c;
+        counts_len += (int64_t)c * ((w.img_width + TILE - 1) / TILE) * ((w.img_height + TILE - 1) / TILE);
+    }
     if (ctx->bdesc_pending) {  // the previous batch's raster upload still reads the staging
         CUDA_TRY(cudaEventSynchronize(ctx->bdesc_ev));
         ctx->bdesc_pending = false;
@@ -332,21 +348,22 @@ int forward_batch(msplat_cuda_ctx *ctx, int nv, const msplat_cuda_view *views) {
     ENSURE(ctx->radii, n, int32_t, radii);
     ENSURE(ctx->aabb, 2 * (size_t)n, float, aabb);
     ENSURE(ctx->n_tiles, n, int32_t, n_tiles);
-    ENSURE(ctx->offsets, n, int64_t, offsets);
     ENSURE(ctx->scan_part, scan_blocks(std::max(n, 1)) + 1, int64_t, scan_part);
     ENSURE(ctx->total, 1, int64_t, d_total);
     ENSURE(ctx->tile_start, T, int32_t, tile_start);
     ENSURE(ctx->tile_end, T, int32_t, tile_end);
     if (!ctx->h_total) CUDA_TRY(cudaMallocHost(&ctx->h_total, sizeof(int64_t)));
     DepthScratch ds;
-    if (int r = ensure_depth_scratch(ctx, n, ds)) return r;
+    if (int r = ensure_bin_scratch(ctx, n, counts_len, ds, ba)) return r;
 
     unsigned char *h = ctx->h_bdesc;
     ProjectArgs *hp = reinterpret_cast<ProjectArgs *>(h + o_proj);
     RasterArgs *hr = reinterpret_cast<RasterArgs *>(h + o_ras);
     int *h_inst = reinterpret_cast<int *>(h + o_inst), *h_toff = reinterpret_cast<int *>(h + o_toff);
     int *h_tx = reinterpret_cast<int *>(h + o_tx), *h_ty = reinterpret_cast<int *>(h + o_ty);
-    int io = 0, to = 0;
+    int *h_chk = reinterpret_cast<int *>(h + o_chk);
+    int64_t *h_cnt = reinterpret_cast<int64_t *>(h + o_cnt), cnt_off = 0;
+    int io = 0, to = 0, chk = 0;
     for (int v = 0; v < nv; v++) {
         const msplat_cuda_view &w = views[v];
         const int tx = (int)((w.img_width + TILE - 1) / TILE), ty = (int)((w.img_height + TILE - 1) / TILE);
@@ -366,21 +383,31 @@ int forward_batch(msplat_cuda_ctx *ctx, int nv, const msplat_cuda_view *views) {
         pa.radii = radii;
         pa.aabb = aabb;
         pa.n_tiles = n_tiles;
-        h_inst[v] = io;
+        pa.depth_keys = ds.keys[0];
+        pa.depth_vals = ds.vals[0];
+            h_inst[v] = io;
         h_toff[v] = to;
         h_tx[v] = tx;
         h_ty[v] = ty;
+        h_chk[v] = chk;
+        h_cnt[v] = cnt_off;
+        const int c = bin_chunks(w.num_points, chunk_len);
         io += w.num_points;
         to += tx * ty;
+        chk += c;
+        cnt_off += (int64_t)c * tx * ty;
     }
     h_inst[nv] = io;
     h_toff[nv] = to;
+    h_chk[nv] = chk;
     BatchDesc d;
     d.n_views = nv;
     d.inst_off = reinterpret_cast<const int *>(d_desc + o_inst);
     d.tile_off = reinterpret_cast<const int *>(d_desc + o_toff);
     d.tiles_x = reinterpret_cast<const int *>(d_desc + o_tx);
     d.tiles_y = reinterpret_cast<const int *>(d_desc + o_ty);
+    d.chunk_off = reinterpret_cast<const int *>(d_desc + o_chk);
+    d.count_off = reinterpret_cast<const int64_t *>(d_desc + o_cnt);
     d.proj = reinterpret_cast<const ProjectArgs *>(d_desc + o_proj);
     d.raster = reinterpret_cast<const RasterArgs *>(d_desc + o_ras);
 
@@ -389,33 +416,36 @@ int forward_batch(msplat_cuda_ctx *ctx, int nv, const msplat_cuda_view *views) {
     ctx->timer.reset_marks();
     ctx->timer.mark(0, st);
     CUDA_TRY(cudaMemcpyAsync(d_desc, h, o_ras, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(d_desc + o_inst, h + o_inst, bytes - o_inst, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(d_desc + o_cnt, h + o_cnt, bytes - o_cnt, cudaMemcpyHostToDevice, st));
+    ba.d = d;
+    ba.tile_cap = T;
+    ba.splats = splats;
+    ba.aabb = aabb;
+    ba.n_tiles = n_tiles;
+    ba.tile_start = tile_start;
+    ba.tile_end = tile_end;
+    bin_plan(ba);
     launch_project_batch(d, n, st);
-    launch_depth_offsets(n, splats, n_tiles, ds, offsets, d_total, scan_part, st);
+    launch_depth_order(ba, ds, scan_part, d_total, st);
     CUDA_TRY(cudaMemcpyAsync(ctx->h_total, d_total, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    // as in the single-view frame: the lists go to the buffer as it is while the host
+    // waits for the count
+    if (!ctx->total_ev) CUDA_TRY(cudaEventCreateWithFlags(&ctx->total_ev, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventRecord(ctx->total_ev, st));
+    ctx->timer.mark(1, st);
+    launch_bin_count(ba, nullptr, st);
+    const int64_t cap0 = (int64_t)ctx->isect_gid.bytes / 4;
+    if (cap0 > 0) launch_bin_emit(ba, reinterpret_cast<int32_t *>(ctx->isect_gid.ptr), nullptr, cap0, st);
+    CUDA_TRY(cudaEventSynchronize(ctx->total_ev));
     const int64_t n_isect = *ctx->h_total;
     if (n_isect > (int64_t)INT32_MAX)
         return fail(MSPLAT_CUDA_EOVERFLOW, "more than 2^31 tile intersections in the batch (%lld)",
                     (long long)n_isect);
     ctx->n_isect = n_isect;
-    ENSURE(ctx->keys[0], n_isect, uint32_t, k0);
-    ENSURE(ctx->keys[1], n_isect, uint32_t, k1);
-    ENSURE(ctx->vals[0], n_isect, uint32_t, v0);
-    ENSURE(ctx->vals[1], n_isect, uint32_t, v1);
-    ENSURE(ctx->radix_scratch, radix_scratch_bytes((int)n_isect), unsigned char, rscratch);
-
-    ctx->timer.mark(1, st);
-    // render only: the sort carries Gaussian ids, so its sorted values are the
-    // per-intersection ids (no emission-index map, no inverse map)
-    launch_emit_keys_batch(n, splats, aabb, n_tiles, offsets, &ds, d, k0, v0, nullptr, st);
-    uint32_t *kk[2] = {k0, k1};
-    uint32_t *vv[2] = {v0, v1};
-    const int cur = radix_sort_pairs32(kk, vv, (int)n_isect, ceil_log2(std::max(T, 1)), rscratch, st);
-    ctx->sorted = cur;
-    ctx->gid_in_vals = true;
-    const int32_t *isect_gid = reinterpret_cast<const int32_t *>(vv[cur]);
-    launch_tile_ranges(kk[cur], (int)n_isect, T, tile_start, tile_end, st);
+    const bool emitted = cap0 > 0 && n_isect <= cap0;
+    if (!emitted) CUDA_TRY(cudaStreamSynchronize(st));
+    ENSURE(ctx->isect_gid, n_isect, int32_t, isect_gid);
+    if (!emitted) launch_bin_emit(ba, isect_gid, nullptr, n_isect, st);
 
     for (int v = 0; v < nv; v++) {
         const msplat_cuda_view &w = views[v];
@@ -1271,7 +1301,6 @@ int msplat_cuda_frame_pair_counts(msplat_cuda_ctx *ctx, int64_t *out) {
     if (!ctx || !out) return fail(MSPLAT_CUDA_EINVAL, "null argument");
     out[0] = out[1] = 0;
     if (ctx->tiles_x <= 0 || ctx->tiles_y <= 0 || !ctx->tile_start.ptr || !ctx->final_idx.ptr) return MSPLAT_CUDA_OK;
-    if (ctx->gid_in_vals) return fail(MSPLAT_CUDA_EINVAL, "the last frame was a batched render");
     ENSURE(ctx->pairs, 2, unsigned long long, d);
     launch_pair_counts(pair_count_args(ctx), d, ctx->stream);
     unsigned long long h[2] = {0, 0};
@@ -1285,7 +1314,6 @@ int msplat_cuda_frame_pair_counts(msplat_cuda_ctx *ctx, int64_t *out) {
 int msplat_cuda_frame_pair_counts_device(msplat_cuda_ctx *ctx, uint64_t *d_sum) {
     if (!ctx || !d_sum) return fail(MSPLAT_CUDA_EINVAL, "null argument");
     if (ctx->tiles_x <= 0 || ctx->tiles_y <= 0 || !ctx->tile_start.ptr || !ctx->final_idx.ptr) return MSPLAT_CUDA_OK;
-    if (ctx->gid_in_vals) return fail(MSPLAT_CUDA_EINVAL, "the last frame was a batched render");
     launch_pair_counts(pair_count_args(ctx), reinterpret_cast<unsigned long long *>(d_sum), ctx->stream, true);
     CUDA_TRY(cudaGetLastError());
     return MSPLAT_CUDA_OK;
@@ -1313,14 +1341,15 @@ int64_t msplat_cuda_ctx_device_bytes(msplat_cuda_ctx *ctx) {
     const Buf *all[] = {&ctx->splats, &ctx->radii, &ctx->aabb, &ctx->n_tiles, &ctx->offsets, &ctx->scan_part,
                         &ctx->total, &ctx->v_xy, &ctx->v_conic, &ctx->v_rgb, &ctx->v_opacity, &ctx->v_mean3d,
                         &ctx->v_scale, &ctx->v_quat, &ctx->keys[0], &ctx->keys[1], &ctx->vals[0], &ctx->vals[1],
-                        &ctx->emit_gid, &ctx->isect_gid, &ctx->inv, &ctx->slots, &ctx->radix_scratch,
+                        &ctx->isect_gid, &ctx->inv, &ctx->slots, &ctx->radix_scratch,
                         &ctx->tile_start, &ctx->tile_end, &ctx->out_img, &ctx->final_T, &ctx->final_idx,
                         &ctx->v_rendered, &ctx->loss_part, &ctx->loss, &ctx->d_flags, &ctx->d_counts,
                         &ctx->d_scratch, &ctx->k_bounds, &ctx->k_sorted, &ctx->k_box, &ctx->k_md, &ctx->tstore,
                         &ctx->tcount, &ctx->bdesc, &ctx->bcounter, &ctx->tb.desc, &ctx->tb.pix_img,
                         &ctx->tb.pix_T, &ctx->tb.pix_idx, &ctx->tb.pix_v, &ctx->tb.partials, &ctx->tb.losses,
                         &ctx->tb.counters, &ctx->dkeys[0], &ctx->dkeys[1], &ctx->dvals[0], &ctx->dvals[1],
-                        &ctx->dcounts, &ctx->doff, &ctx->img[0], &ctx->img[1], &ctx->img[2]};
+                        &ctx->rects, &ctx->rect_tiles,
+                        &ctx->off_sorted, &ctx->bin_bounds, &ctx->bin_counts, &ctx->img[0], &ctx->img[1], &ctx->img[2]};
     int64_t total = 0;
     for (const Buf *b : all) total += (int64_t)b->bytes;
     for (const Buf &b : ctx->pri) total += (int64_t)b.bytes;
@@ -1381,12 +1410,6 @@ int msplat_cuda_frame(msplat_cuda_ctx *ctx, const char *name, const void **dev_p
         {"chunk_first", &ctx->ch[CH_FIRST], ctx->chunk_frame ? T + 1 : 0},
         {"knn_evals", &ctx->k_evals, 2},  // one uint64: the last kNN call's point distances
     };
-    if (ctx->gid_in_vals && !std::strcmp(name, "isect_gid")) {  // a batched render's ids: the sorted values
-        if (!ctx->vals[ctx->sorted].ptr) return fail(MSPLAT_CUDA_EINVAL, "frame buffer 'isect_gid' has not been produced");
-        *dev_ptr = ctx->vals[ctx->sorted].ptr;
-        *count = ctx->n_isect;
-        return MSPLAT_CUDA_OK;
-    }
     for (const Entry &e : table)
         if (!std::strcmp(e.name, name)) {
             if (!e.buf->ptr) return fail(MSPLAT_CUDA_EINVAL, "frame buffer '%s' has not been produced", name);

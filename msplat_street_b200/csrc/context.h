@@ -183,13 +183,13 @@ struct msplat_cuda_ctx {
     // frame description
     int n = 0, W = 0, H = 0, tiles_x = 0, tiles_y = 0;
     int64_t n_isect = 0;
-    int sorted = 0;  // which key/value buffer pair holds the sorted result
-    bool gid_in_vals = false;  // the sorted values are Gaussian ids (batched render) rather than emission indices
     // per Gaussian
     Buf splats, radii, aabb, n_tiles, offsets, scan_part, total;
     Buf v_xy, v_conic, v_rgb, v_opacity, v_mean3d, v_scale, v_quat;
     // per intersection
-    Buf keys[2], vals[2], emit_gid, isect_gid, inv, slots, radix_scratch;
+    Buf isect_gid, inv, slots;
+    // key / value buffers of the sort and kNN primitives, and the radix sorts' scratch
+    Buf keys[2], vals[2], radix_scratch;
     // per tile / pixel
     Buf tile_start, tile_end, out_img, final_T, final_idx, v_rendered, loss_part, loss;
     // densification and primitive scratch
@@ -205,8 +205,10 @@ struct msplat_cuda_ctx {
     bool chunk_frame = false;
     int64_t chunk_cap = 0;
     Buf ch[CH_COUNT];
-    // depth order of the Gaussians (or batch instances) before key emission
-    Buf dkeys[2], dvals[2], dcounts, doff;
+    // depth order of the Gaussians (or batch instances), their tile rectangles, tile
+    // counts and first emission indices in that order, and the chunks' positions and
+    // per-tile counts (BinArgs)
+    Buf dkeys[2], dvals[2], rects, rect_tiles, off_sorted, bin_bounds, bin_counts;
     // image pipeline scratch: metrics (SSIM terms, row sums) and RGBA8 packing
     Buf img[3];
     // prior-guided extras: the prior in force, whether the last frame ran in aux
@@ -231,11 +233,11 @@ struct msplat_cuda_ctx {
     }
     void release() {
         Buf *all[] = {&splats, &radii, &aabb, &n_tiles, &offsets, &scan_part, &total, &v_xy, &v_conic, &v_rgb,
-                      &v_opacity, &v_mean3d, &v_scale, &v_quat, &keys[0], &keys[1], &vals[0], &vals[1], &emit_gid,
+                      &v_opacity, &v_mean3d, &v_scale, &v_quat, &keys[0], &keys[1], &vals[0], &vals[1],
                       &isect_gid, &inv, &slots, &radix_scratch, &tile_start, &tile_end, &out_img, &final_T,
                       &final_idx, &v_rendered, &loss_part, &loss, &d_flags, &d_counts, &d_scratch, &k_bounds,
                       &k_sorted, &k_box, &k_md, &k_evals, &tstore, &tcount, &pairs, &bdesc, &bcounter, &dkeys[0], &dkeys[1],
-                      &dvals[0], &dvals[1], &dcounts, &doff, &img[0], &img[1], &img[2]};
+                      &dvals[0], &dvals[1], &rects, &rect_tiles, &off_sorted, &bin_bounds, &bin_counts, &img[0], &img[1], &img[2]};
         for (Buf *b : all) {
             if (b->ptr) cudaFree(b->ptr);
             b->ptr = nullptr;
@@ -310,22 +312,30 @@ int check_camera(int num_points, unsigned H, unsigned W, int tx, int ty, unsigne
 CamParams make_cam(const float *viewmat, const float *projmat, float fx, float fy, float cx, float cy, unsigned H,
                    unsigned W, int tx, int ty, float clip, unsigned degree, unsigned dtu, const float *cam_pos);
 
-// Depth-order scratch for n Gaussians (or batch instances) from the context's buffers.
-inline int ensure_depth_scratch(msplat_cuda_ctx *ctx, int64_t n, DepthScratch &s) {
+// Binning buffers for n Gaussians (or batch instances) whose a.chunks chunks hold
+// counts_len per-tile counts in all. Fills the depth-sort scratch and a's scratch
+// pointers (the projection takes its key outputs from s).
+inline int ensure_bin_scratch(msplat_cuda_ctx *ctx, int64_t n, int64_t counts_len, DepthScratch &s, BinArgs &a) {
     ENSURE(ctx->dkeys[0], n, uint32_t, k0);
     ENSURE(ctx->dkeys[1], n, uint32_t, k1);
     ENSURE(ctx->dvals[0], n, uint32_t, v0);
     ENSURE(ctx->dvals[1], n, uint32_t, v1);
-    ENSURE(ctx->dcounts, n, int32_t, counts);
-    ENSURE(ctx->doff, n, int64_t, off);
+    ENSURE(ctx->rects, n, int4, rects);
+    ENSURE(ctx->rect_tiles, n, int32_t, rect_tiles);
+    ENSURE(ctx->off_sorted, n, int64_t, off_sorted);
+    ENSURE(ctx->bin_bounds, a.chunks, int2, bounds);
+    ENSURE(ctx->bin_counts, counts_len, int32_t, counts);
     ENSURE(ctx->radix_scratch, radix_scratch_bytes((int)std::max<int64_t>(n, 1)), unsigned char, rs);
     s.keys[0] = k0;
     s.keys[1] = k1;
     s.vals[0] = v0;
     s.vals[1] = v1;
-    s.counts = counts;
-    s.off_sorted = off;
     s.radix_scratch = rs;
+    a.rects = rects;
+    a.rect_tiles = rect_tiles;
+    a.offsets_sorted = off_sorted;
+    a.bounds = bounds;
+    a.counts = counts;
     return 0;
 }
 

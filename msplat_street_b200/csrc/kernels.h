@@ -33,6 +33,9 @@ struct ProjectArgs {
     int32_t *radii;
     float *aabb;
     int32_t *n_tiles;
+    // depth-order keys and values: the depth's bits (which for the positive depths of
+    // visible Gaussians order like the numbers), 0xffffffff for the others; the index
+    uint32_t *depth_keys, *depth_vals;
 };
 void launch_project(const ProjectArgs &a, cudaStream_t st);
 
@@ -40,34 +43,12 @@ int scan_blocks(int n);
 template <typename TO>
 void scan_exclusive(const int32_t *in, TO *out, int n, TO *d_total, TO *partials, cudaStream_t st);
 
-// Depth order of n Gaussians (stable) and their emission offsets in that order:
-// offsets[g] = tiles of every Gaussian before g by (depth, index); *d_total = all.
-struct DepthScratch {
-    uint32_t *keys[2], *vals[2];  // n each
-    int32_t *counts;              // n
-    int64_t *off_sorted;          // n
-    void *radix_scratch;          // radix_scratch_bytes(n)
-};
-void launch_depth_offsets(int n, const Splat *splats, const int32_t *n_tiles, DepthScratch &s, int64_t *offsets,
-                          int64_t *d_total, int64_t *scan_part, cudaStream_t st);
-// Emission: key = tile id (global tile id in a batch), value = emission index, or
-// the Gaussian id when emit_gid is null (render only: no backward needs the map).
-// cap: entries at or past it are not written (the buffers' capacity)
-void launch_emit_keys(int n, const Splat *splats, const float *aabb, const int32_t *n_tiles, const int64_t *offsets,
-                      int tiles_x, int tiles_y, uint32_t *keys, uint32_t *vals, int32_t *emit_gid, cudaStream_t st,
-                      int64_t cap = INT64_MAX);
 size_t radix_scratch_bytes(int n);
 // d_n / d_T (optional): device-side counts capping the host-side capacities n / T
 int radix_sort_pairs(uint64_t *k[2], uint32_t *v[2], int n, int key_bits, void *scratch, cudaStream_t st,
                      const int *d_n = nullptr);
 int radix_sort_pairs32(uint32_t *k[2], uint32_t *v[2], int n, int key_bits, void *scratch, cudaStream_t st,
                        const int *d_n = nullptr);
-void launch_tile_ranges(const uint32_t *keys, int n, int T, int32_t *tile_start, int32_t *tile_end, cudaStream_t st,
-                        const int *d_n = nullptr, const int *d_T = nullptr);
-void launch_isect_map(const uint32_t *sorted_e, int n, const int32_t *emit_gid, int32_t *isect_gid, int32_t *inv,
-                      cudaStream_t st, const int *d_n = nullptr);
-void launch_clamp_count(const int64_t *total, int64_t cap, int *d_n, int *overflow, cudaStream_t st);
-
 struct RasterArgs {
     int W, H, tiles_x, tiles_y;
     const int32_t *tile_start, *tile_end, *isect_gid;
@@ -152,6 +133,8 @@ struct BatchDesc {
     const int *inst_off;       // [n_views + 1] first instance of each view
     const int *tile_off;       // [n_views + 1] first global tile of each view
     const int *tiles_x, *tiles_y;
+    const int *chunk_off;      // [n_views + 1] first chunk of each view (BinArgs)
+    const int64_t *count_off;  // [n_views] first per-tile count of each view (BinArgs)
     const ProjectArgs *proj;   // per view; outputs point at the batch-wide arrays
     const RasterArgs *raster;  // per view; tile ranges and lists are batch-wide
 };
@@ -169,11 +152,40 @@ __device__ __forceinline__ int find_view(const int *off, int n_views, int g) {
 }
 
 void launch_project_batch(const BatchDesc &d, int total, cudaStream_t st);
-// ds (may be null): threads take Gaussians in ds's depth order (after
-// launch_depth_offsets) instead of by index; the entries are the same.
-void launch_emit_keys_batch(int n, const Splat *splats, const float *aabb, const int32_t *n_tiles,
-                            const int64_t *offsets, const DepthScratch *ds, const BatchDesc &d, uint32_t *keys,
-                            uint32_t *vals, int32_t *emit_gid, cudaStream_t st, int64_t cap = INT64_MAX);
+
+// Tile binning (bin.cu): every tile's list of Gaussians in (depth, index) order.
+struct DepthScratch {
+    uint32_t *keys[2], *vals[2];  // n each
+    void *radix_scratch;          // radix_scratch_bytes(n)
+};
+struct BinArgs {
+    int n;                 // Gaussians, or a batch's instances
+    int tiles_x, tiles_y;  // single view
+    BatchDesc d;           // batch; n_views = 0 for a single view
+    int chunks;            // chunks of the depth order, at most (in a batch: of all views)
+    int grid_y, win_rows;  // blocks per chunk and the tile rows of their windows (bin_plan)
+    int tile_cap;          // tiles (in a batch: at least as many as the views have)
+    const Splat *splats;
+    const float *aabb;
+    const int32_t *n_tiles;
+    const uint32_t *order;    // launch_depth_order
+    const int64_t *total;     // all intersections
+    int4 *rects;              // per position of the order: its tiles [x, z) x [y, w)
+    int32_t *rect_tiles;      // and their number
+    int64_t *offsets_sorted;  // and its first emission index
+    int2 *bounds;             // per chunk: its positions
+    int32_t *counts;          // per chunk, the tiles of its view
+    int32_t *tile_start, *tile_end;
+};
+int bin_chunk_len(int64_t n, int64_t tiles);
+int bin_chunks(int n, int len);
+void bin_plan(BinArgs &a);
+void launch_depth_order(BinArgs &a, DepthScratch &s, int64_t *scan_part, int64_t *total, cudaStream_t st);
+void launch_bin_count(const BinArgs &a, int64_t *offsets, cudaStream_t st);
+// inv may be null (render only); entries at or past cap (the buffers' capacity) are dropped
+void launch_bin_emit(const BinArgs &a, int32_t *gids, int32_t *inv, int64_t cap, cudaStream_t st);
+void launch_bin_clamp(const BinArgs &a, int64_t cap, int *d_n, int *overflow, cudaStream_t st);
+
 void launch_raster_fwd_batch(const BatchDesc &d, int tiles_hint, int *d_counter, cudaStream_t st, int variant = 0,
                              int shape = 0);
 

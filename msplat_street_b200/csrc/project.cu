@@ -11,6 +11,12 @@ namespace msplat {
 
 constexpr int PROJ_THREADS = 128;
 
+// Key and value of the depth order at output slot o.
+__device__ __forceinline__ void depth_key(const ProjectArgs &a, int o, bool kept, float depth) {
+    a.depth_keys[o] = kept ? __float_as_uint(depth) : 0xffffffffu;
+    a.depth_vals[o] = (uint32_t)o;
+}
+
 // With SH degree 3 in use the warp stages its SH-rest rows while the geometry runs
 // (issue_rest_rows); no lane leaves before the wait that every lane of the warp takes.
 __global__ void __launch_bounds__(PROJ_THREADS) project_kernel(ProjectArgs a) {
@@ -23,6 +29,7 @@ __global__ void __launch_bounds__(PROJ_THREADS) project_kernel(ProjectArgs a) {
         staged = issue_rest_rows(a.features_rest + (size_t)PROJ_REST3 * (valid ? i : 0), valid, buf);
     ProjState st;
     const bool kept = valid && project_geom(a, i, i, st);
+    if (valid) depth_key(a, i, kept, st.depth);
     if (staged) rest_rows_wait();
     if (kept) project_finish(a, i, i, st, staged ? buf + PROJ_REST3 * (threadIdx.x & 31) : nullptr);
 }
@@ -47,6 +54,7 @@ __global__ void __launch_bounds__(PROJ_THREADS) project_batch_kernel(const Batch
         issue_rest_rows(deg3 ? d.proj[v].features_rest + (size_t)PROJ_REST3 * i : nullptr, deg3, buf);
     ProjState st;
     const bool kept = valid && project_geom(d.proj[v], i, g, st);
+    if (valid) depth_key(d.proj[v], g, kept, st.depth);
     if (staged) rest_rows_wait();
     if (kept) project_finish(d.proj[v], i, g, st, staged ? buf + PROJ_REST3 * (threadIdx.x & 31) : nullptr);
 }

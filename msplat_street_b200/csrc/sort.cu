@@ -1,20 +1,8 @@
-// Tile-intersection binning: exclusive scan, depth order, key emission, stable LSD
-// radix sort and tile ranges.
-//
-// The reference builds per-tile lists ordered by (depth bits, Gaussian index)
-// (bin_and_sort, core/cpu/msplat_cpu.cpp:505-567). Here the visible Gaussians are
-// sorted by depth bits once (stable, so ties keep index order); every (Gaussian, tile)
-// pair is then emitted in that order at offsets from an exclusive scan of
-// tiles-per-Gaussian, keyed by its tile id alone. A STABLE radix sort over the
-// ceil(log2 tiles) tile bits then yields, within each tile, ascending depth with ties
-// in Gaussian order -- exactly the reference's order -- without a per-tile sort or any
-// cap on a tile's list. The sort carries the emission index as its value; the map
-// kernel turns it into the Gaussian id per sorted slot and the inverse permutation
-// that the backward pass uses to reduce per-Gaussian gradients deterministically.
+// Exclusive scan and stable radix sort.
 //
 // The radix sort is reduce-then-scan per 8-bit digit: a histogram kernel, a device
 // scan of the digit-major counts, and a scatter kernel that ranks keys stably inside
-// each 2048-key block with warp match/popc. No block waits on another block.
+// each 2048-key block with warp ballots and popc. No block waits on another block.
 #include <algorithm>
 #include <atomic>
 
@@ -152,188 +140,6 @@ void scan_exclusive(const int32_t *in, TO *out, int n, TO *d_total, TO *partials
 }
 template void scan_exclusive<int32_t>(const int32_t *, int32_t *, int, int32_t *, int32_t *, cudaStream_t);
 template void scan_exclusive<int64_t>(const int32_t *, int64_t *, int, int64_t *, int64_t *, cudaStream_t);
-
-// ---------------------------------------------------------------------------------
-// Depth order and key emission.
-//
-// The reference orders each tile's list by (depth bits, Gaussian index). Here the
-// Gaussians are first sorted by depth bits, stably (ties keep index order), and each
-// one's intersections are emitted at offsets from a scan of tile counts taken in that
-// order; a stable sort of the emitted entries by tile id alone then leaves every tile's
-// entries in (depth, index) order. The per-intersection sort needs only ceil(log2
-// tiles) key bits (2 passes up to 65,536 tiles) instead of 32 more depth bits.
-
-// Depth keys: the float bits of the depth, which for the positive depths of visible
-// Gaussians order like the numbers; Gaussians with no tiles go last.
-__global__ void depth_keys_kernel(int n, const Splat *splats, const int32_t *n_tiles, uint32_t *keys, uint32_t *vals) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    keys[i] = n_tiles[i] > 0 ? __float_as_uint(splats[i].depth) : 0xffffffffu;
-    vals[i] = (uint32_t)i;
-}
-
-__global__ void gather_counts_kernel(int n, const uint32_t *order, const int32_t *n_tiles, int32_t *cnt) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n) cnt[r] = n_tiles[order[r]];
-}
-
-__global__ void scatter_offsets_kernel(int n, const uint32_t *order, const int64_t *off_sorted, int64_t *offsets) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n) offsets[order[r]] = off_sorted[r];
-}
-
-void launch_depth_offsets(int n, const Splat *splats, const int32_t *n_tiles, DepthScratch &s, int64_t *offsets,
-                          int64_t *d_total, int64_t *scan_part, cudaStream_t st) {
-    if (n <= 0) {
-        cudaMemsetAsync(d_total, 0, sizeof(int64_t), st);
-        return;
-    }
-    const int nb = (n + 255) / 256;
-    depth_keys_kernel<<<nb, 256, 0, st>>>(n, splats, n_tiles, s.keys[0], s.vals[0]);
-    const int cur = radix_sort_pairs32(s.keys, s.vals, n, 32, s.radix_scratch, st);
-    if (cur != 0)  // four 8-bit passes end in buffer 0; emission reads the order there
-        cudaMemcpyAsync(s.vals[0], s.vals[1], (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-    gather_counts_kernel<<<nb, 256, 0, st>>>(n, s.vals[cur], n_tiles, s.counts);
-    scan_exclusive<int64_t>(s.counts, s.off_sorted, n, d_total, scan_part, st);
-    scatter_offsets_kernel<<<nb, 256, 0, st>>>(n, s.vals[cur], s.off_sorted, offsets);
-}
-
-__device__ __forceinline__ void rect_of(const Splat &s, float ax, float ay, int tx, int ty, int &x0, int &y0, int &x1,
-                                        int &y1) {
-    float ccx = s.x / (float)TILE, ccy = s.y / (float)TILE;
-    float rrx = ax / (float)TILE, rry = ay / (float)TILE;
-    x0 = min(max(0, (int)(ccx - rrx)), tx);
-    x1 = min(max(0, (int)(ccx + rrx + 1)), tx);
-    y0 = min(max(0, (int)(ccy - rry)), ty);
-    y1 = min(max(0, (int)(ccy + rry + 1)), ty);
-}
-
-// Emission of each Gaussian's intersections: the tiles of its rectangle [x0, x1) x
-// [y0, y1) in row-major order at emission indices e0, e0 + 1, ..., key = base + tile
-// id, value = emission index (or, with emit_gid null -- render-only frames with no
-// backward -- the Gaussian id itself, so the sorted values are the per-intersection
-// ids with no gather). cap: buffer capacity (entries at or past it are dropped).
-// Rectangles of up to SMALL_RECT tiles are written by their own thread; larger ones by
-// the whole warp, lane l writing entries l, l + 32, ..., so their stores coalesce.
-//
-// Two thread-to-Gaussian maps, the same entries either way. BY_DEPTH: thread j takes
-// the Gaussian at position j of the depth order; the emission offsets follow that
-// order, so neighbouring threads write neighbouring ranges and stores fill whole
-// sectors between them -- the better map when most Gaussians cover a few tiles each
-// (renders of large scenes). By index: thread i takes Gaussian i; near-camera
-// Gaussians with hundreds of tiles, which sit side by side in the depth order, then
-// spread over many warps instead of falling to a few warps one after another -- the
-// better map for training views, where such Gaussians carry much of the work.
-constexpr int SMALL_RECT = 8;
-
-__device__ __forceinline__ void emit_one(int64_t e, uint32_t key, int gid, uint32_t *keys, uint32_t *vals,
-                                         int32_t *emit_gid) {
-    keys[e] = key;
-    if (emit_gid) {
-        vals[e] = (uint32_t)e;
-        emit_gid[e] = gid;
-    } else {
-        vals[e] = (uint32_t)gid;
-    }
-}
-
-// Every lane of the warp must call it.
-__device__ __forceinline__ void emit_rect(bool ok, int x0, int y0, int x1, int y1, int tiles_x, uint32_t base,
-                                          int64_t e0, int gid, int64_t cap, uint32_t *keys, uint32_t *vals,
-                                          int32_t *emit_gid) {
-    const int w = x1 - x0, cnt = ok ? w * (y1 - y0) : 0;
-    if (cnt > 0 && cnt <= SMALL_RECT) {
-        int64_t e = e0;
-        for (int y = y0; y < y1; y++)
-            for (int x = x0; x < x1 && e < cap; x++, e++)
-                emit_one(e, base + (uint32_t)(y * tiles_x + x), gid, keys, vals, emit_gid);
-    }
-    unsigned big = __ballot_sync(0xffffffffu, cnt > SMALL_RECT);
-    const int lane = threadIdx.x & 31;
-    while (big) {  // warp-uniform
-        const int src = __ffs(big) - 1;
-        big &= big - 1;
-        const int sw = __shfl_sync(0xffffffffu, w, src), sc = __shfl_sync(0xffffffffu, cnt, src);
-        const int sx0 = __shfl_sync(0xffffffffu, x0, src), sy0 = __shfl_sync(0xffffffffu, y0, src);
-        const int stx = __shfl_sync(0xffffffffu, tiles_x, src), sg = __shfl_sync(0xffffffffu, gid, src);
-        const uint32_t sb = __shfl_sync(0xffffffffu, base, src);
-        const int64_t se = __shfl_sync(0xffffffffu, (long long)e0, src);
-        for (int j = lane; j < sc; j += 32) {
-            const int64_t e = se + j;
-            if (e >= cap) break;
-            emit_one(e, sb + (uint32_t)((sy0 + j / sw) * stx + sx0 + j % sw), sg, keys, vals, emit_gid);
-        }
-    }
-}
-
-struct EmitSrc {
-    const int32_t *n_tiles;      // per Gaussian (index map)
-    const int64_t *offsets;      // per Gaussian (index map)
-    const uint32_t *order;       // depth order (BY_DEPTH)
-    const int32_t *cnt_sorted;   // tile counts in depth order (BY_DEPTH)
-    const int64_t *off_sorted;   // emission offsets in depth order (BY_DEPTH)
-};
-
-// BATCH: instance g (a Gaussian of one view) keys its tiles with the view's first
-// global tile added, so one stable sort orders every view's tiles at once and each
-// tile's list is the one the single-view sort gives.
-template <bool BATCH, bool BY_DEPTH>
-__global__ void emit_keys_kernel(int n, const Splat *splats, const float *aabb, const EmitSrc src, int tiles_x,
-                                 int tiles_y, const BatchDesc d, uint32_t *keys, uint32_t *vals, int32_t *emit_gid,
-                                 int64_t cap) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool ok = j < n && (BY_DEPTH ? src.cnt_sorted[j] : src.n_tiles[j]) > 0;
-    int x0 = 0, y0 = 0, x1 = 0, y1 = 0, g = 0, tx = tiles_x;
-    uint32_t base = 0;
-    int64_t e0 = 0;
-    if (ok) {
-        g = BY_DEPTH ? (int)src.order[j] : j;
-        int ty = tiles_y;
-        if (BATCH) {
-            const int v = find_view(d.inst_off, d.n_views, g);
-            tx = d.tiles_x[v];
-            ty = d.tiles_y[v];
-            base = (uint32_t)d.tile_off[v];
-        }
-        rect_of(splats[g], aabb[2 * g], aabb[2 * g + 1], tx, ty, x0, y0, x1, y1);
-        e0 = BY_DEPTH ? src.off_sorted[j] : src.offsets[g];
-    }
-    emit_rect(ok, x0, y0, x1, y1, tx, base, e0, g, cap, keys, vals, emit_gid);
-}
-
-namespace {
-EmitSrc emit_src(const int32_t *n_tiles, const int64_t *offsets, const DepthScratch *ds) {
-    EmitSrc s{n_tiles, offsets, nullptr, nullptr, nullptr};
-    if (ds) {
-        s.order = ds->vals[0];
-        s.cnt_sorted = ds->counts;
-        s.off_sorted = ds->off_sorted;
-    }
-    return s;
-}
-}  // namespace
-
-void launch_emit_keys(int n, const Splat *splats, const float *aabb, const int32_t *n_tiles, const int64_t *offsets,
-                      int tiles_x, int tiles_y, uint32_t *keys, uint32_t *vals, int32_t *emit_gid, cudaStream_t st,
-                      int64_t cap) {
-    if (n <= 0 || cap <= 0) return;
-    emit_keys_kernel<false, false><<<(n + 127) / 128, 128, 0, st>>>(
-        n, splats, aabb, emit_src(n_tiles, offsets, nullptr), tiles_x, tiles_y, BatchDesc{}, keys, vals, emit_gid,
-        cap);
-}
-
-void launch_emit_keys_batch(int n, const Splat *splats, const float *aabb, const int32_t *n_tiles,
-                            const int64_t *offsets, const DepthScratch *ds, const BatchDesc &d, uint32_t *keys,
-                            uint32_t *vals, int32_t *emit_gid, cudaStream_t st, int64_t cap) {
-    if (n <= 0) return;
-    const EmitSrc src = emit_src(n_tiles, offsets, ds);
-    if (ds)
-        emit_keys_kernel<true, true><<<(n + 127) / 128, 128, 0, st>>>(n, splats, aabb, src, 0, 0, d, keys, vals,
-                                                                      emit_gid, cap);
-    else
-        emit_keys_kernel<true, false><<<(n + 127) / 128, 128, 0, st>>>(n, splats, aabb, src, 0, 0, d, keys, vals,
-                                                                       emit_gid, cap);
-}
 
 // ---------------------------------------------------------------------------------
 // Stable LSD radix sort of (key, u32 value) pairs by key bits [0, key_bits), for
@@ -588,64 +394,6 @@ int radix_sort_pairs(uint64_t *k[2], uint32_t *v[2], int n, int key_bits, void *
 int radix_sort_pairs32(uint32_t *k[2], uint32_t *v[2], int n, int key_bits, void *scratch, cudaStream_t st,
                        const int *d_n) {
     return radix_sort_dispatch<uint32_t>(k, v, n, std::min(key_bits, 32), scratch, st, d_n);
-}
-
-// ---------------------------------------------------------------------------------
-// Tile ranges by binary search over the sorted tile ids (empty tiles get start ==
-// end == the running count, as the reference's prefix sums give), and the per-slot
-// Gaussian id / inverse map.
-
-__global__ void tile_ranges_kernel(const uint32_t *keys, int n, int T, int32_t *tile_start, int32_t *tile_end,
-                                   const int *d_n, const int *d_T) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d_n) n = min(n, *d_n);
-    if (d_T) T = min(T, *d_T);
-    if (t > T) return;
-    int lo = 0, hi = n;  // first position whose tile id >= t
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if ((int)keys[mid] < t) lo = mid + 1;
-        else hi = mid;
-    }
-    if (t < T) tile_start[t] = lo;
-    if (t > 0) tile_end[t - 1] = lo;
-}
-
-// inv (may be null, render-only frames): emission index -> sorted position, for the
-// backward's per-Gaussian reduction
-__global__ void isect_map_kernel(const uint32_t *sorted_e, int n, const int32_t *emit_gid, int32_t *isect_gid,
-                                 int32_t *inv, const int *d_n) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d_n) n = min(n, *d_n);
-    if (k >= n) return;
-    const uint32_t e = sorted_e[k];
-    isect_gid[k] = emit_gid[e];
-    if (inv) inv[e] = k;
-}
-
-void launch_tile_ranges(const uint32_t *keys, int n, int T, int32_t *tile_start, int32_t *tile_end, cudaStream_t st,
-                        const int *d_n, const int *d_T) {
-    tile_ranges_kernel<<<(T + 1 + 255) / 256, 256, 0, st>>>(keys, n, T, tile_start, tile_end, d_n, d_T);
-}
-
-void launch_isect_map(const uint32_t *sorted_e, int n, const int32_t *emit_gid, int32_t *isect_gid, int32_t *inv,
-                      cudaStream_t st, const int *d_n) {
-    if (n <= 0) return;
-    isect_map_kernel<<<(n + 255) / 256, 256, 0, st>>>(sorted_e, n, emit_gid, isect_gid, inv, d_n);
-}
-
-// Device-side intersection count for capacity-bounded (graph-capturable) steps:
-// d_n = total when it fits the capacity, else 0 with *overflow set (the step then
-// renders nothing and updates nothing; the host grows the buffers and repeats it).
-__global__ void clamp_count_kernel(const int64_t *total, int64_t cap, int *d_n, int *overflow) {
-    const int64_t t = *total;
-    const bool over = t > cap;
-    *d_n = over ? 0 : (int)t;
-    if (over) *overflow = 1;
-}
-
-void launch_clamp_count(const int64_t *total, int64_t cap, int *d_n, int *overflow, cudaStream_t st) {
-    clamp_count_kernel<<<1, 1, 0, st>>>(total, cap, d_n, overflow);
 }
 
 }  // namespace msplat

@@ -36,15 +36,17 @@ namespace {
 
 // Offsets of the descriptor blob (device copy and pinned staging share the layout).
 struct BlobLayout {
-    size_t proj, ras, rbwd, ssim, inst, toff, tx, ty, boff, imd, adam, bytes;
+    size_t proj, ras, rbwd, ssim, cnt, inst, toff, chk, tx, ty, boff, imd, adam, bytes;
     BlobLayout(int nv) {
         proj = 0;
         ras = align_up(proj + nv * sizeof(ProjectArgs), 256);
         rbwd = align_up(ras + nv * sizeof(RasterArgs), 256);
         ssim = align_up(rbwd + nv * sizeof(RasterBwdArgs), 256);
-        inst = align_up(ssim + nv * sizeof(SsimArgs), 256);
+        cnt = align_up(ssim + nv * sizeof(SsimArgs), 256);
+        inst = cnt + nv * sizeof(int64_t);
         toff = inst + (nv + 1) * sizeof(int);
-        tx = toff + (nv + 1) * sizeof(int);
+        chk = toff + (nv + 1) * sizeof(int);
+        tx = chk + (nv + 1) * sizeof(int);
         ty = tx + nv * sizeof(int);
         boff = ty + nv * sizeof(int);
         imd = boff + (nv + 1) * sizeof(int);
@@ -83,17 +85,15 @@ struct StepPtrs {
     float *aabb;
     int64_t *offsets, *scan_part, *total;
     int32_t *tile_start, *tile_end;
-    uint32_t *k[2];
-    uint32_t *v[2];
-    int32_t *emit_gid, *isect_gid, *inv;
+    int32_t *isect_gid, *inv;
     float *slots;
-    void *rscratch;
     float *img, *T, *v_img;
     int32_t *idx;
     double *partials;
     float *losses;
     int *counters;
     DepthScratch depth;  // depth order of the instances
+    BinArgs bin;
 };
 
 struct Sizes {
@@ -156,15 +156,9 @@ int ensure_buffers(msplat_cuda_ctx *ctx, const Sizes &sz, int64_t isect_cap, int
     ENSURE(ctx->total, 1, int64_t, total);
     ENSURE(ctx->tile_start, sz.tiles, int32_t, tile_start);
     ENSURE(ctx->tile_end, sz.tiles, int32_t, tile_end);
-    ENSURE(ctx->keys[0], isect_cap, uint32_t, k0);
-    ENSURE(ctx->keys[1], isect_cap, uint32_t, k1);
-    ENSURE(ctx->vals[0], isect_cap, uint32_t, v0);
-    ENSURE(ctx->vals[1], isect_cap, uint32_t, v1);
-    ENSURE(ctx->emit_gid, isect_cap, int32_t, emit_gid);
     ENSURE(ctx->isect_gid, isect_cap, int32_t, isect_gid);
     ENSURE(ctx->inv, isect_cap, int32_t, inv);
     ENSURE(ctx->slots, isect_cap * 9, float, slots);
-    ENSURE(ctx->radix_scratch, radix_scratch_bytes((int)isect_cap), unsigned char, rscratch);
     ENSURE(tb.pix_img, 3 * sz.pix, float, img);
     ENSURE(tb.pix_T, sz.pix, float, T);
     ENSURE(tb.pix_idx, sz.pix, int32_t, idx);
@@ -172,21 +166,35 @@ int ensure_buffers(msplat_cuda_ctx *ctx, const Sizes &sz, int64_t isect_cap, int
     ENSURE(tb.partials, sz.blocks, double, partials);
     ENSURE(tb.losses, nv, float, losses);
     ENSURE(tb.counters, N_COUNTERS, int, counters);
-    P = StepPtrs{desc, splats, radii, n_tiles, aabb, offsets, scan_part, total, tile_start, tile_end, {k0, k1},
-                 {v0, v1}, emit_gid, isect_gid, inv, slots, rscratch, img, T, v_img, idx, partials, losses, counters,
-                 {}};
+    P = StepPtrs{desc, splats, radii, n_tiles, aabb, offsets, scan_part, total, tile_start, tile_end, isect_gid, inv,
+                 slots, img, T, v_img, idx, partials, losses, counters, {}, {}};
     // capacities as the buffers now stand (ENSURE keeps headroom)
-    const int64_t cap_k = (int64_t)std::min({ctx->keys[0].bytes / 4, ctx->keys[1].bytes / 4, ctx->vals[0].bytes / 4,
-                                             ctx->vals[1].bytes / 4, ctx->emit_gid.bytes / 4,
-                                             ctx->isect_gid.bytes / 4, ctx->inv.bytes / 4, ctx->slots.bytes / 36});
+    const int64_t cap_k = (int64_t)std::min({ctx->isect_gid.bytes / 4, ctx->inv.bytes / 4, ctx->slots.bytes / 36});
     tb.isect_cap = std::min<int64_t>(cap_k, INT32_MAX / 2);
-    // one sort scratch serves the depth sort and the tile sort, so it covers both sizes
-    // (no reallocation when it already does)
-    if (int r = ensure_depth_scratch(ctx, inst, P.depth)) return r;
-    ENSURE(ctx->radix_scratch, radix_scratch_bytes((int)std::max<int64_t>(tb.isect_cap, inst)), unsigned char, rs2);
-    P.rscratch = rs2;
-    P.depth.radix_scratch = rs2;
     tb.tile_cap = (int)std::min<size_t>(std::min(ctx->tile_start.bytes, ctx->tile_end.bytes) / 4, INT32_MAX);
+    BinArgs &B = P.bin;
+    B.n = (int)inst;
+    B.chunks = nv * bin_chunks((int)(inst / nv), bin_chunk_len(inst, (tb.tile_cap + nv - 1) / nv));
+    B.tile_cap = tb.tile_cap;
+    // every view has the same Gaussians, so the same chunks
+    if (int r = ensure_bin_scratch(ctx, inst, (int64_t)(B.chunks / nv) * tb.tile_cap, P.depth, B)) return r;
+    B.splats = splats;
+    B.aabb = aabb;
+    B.n_tiles = n_tiles;
+    B.total = total;
+    B.tile_start = tile_start;
+    B.tile_end = tile_end;
+    const BlobLayout L(nv);
+    B.d.n_views = nv;
+    B.d.inst_off = reinterpret_cast<const int *>(desc + L.inst);
+    B.d.tile_off = reinterpret_cast<const int *>(desc + L.toff);
+    B.d.tiles_x = reinterpret_cast<const int *>(desc + L.tx);
+    B.d.tiles_y = reinterpret_cast<const int *>(desc + L.ty);
+    B.d.chunk_off = reinterpret_cast<const int *>(desc + L.chk);
+    B.d.count_off = reinterpret_cast<const int64_t *>(desc + L.cnt);
+    B.d.proj = reinterpret_cast<const ProjectArgs *>(desc + L.proj);
+    B.d.raster = reinterpret_cast<const RasterArgs *>(desc + L.ras);
+    bin_plan(B);
     return MSPLAT_CUDA_OK;
 }
 
@@ -199,7 +207,9 @@ void fill_blob(unsigned char *h, const StepArgs &a, const StepPtrs &P) {
     SsimArgs *sa = reinterpret_cast<SsimArgs *>(h + L.ssim);
     int *inst = reinterpret_cast<int *>(h + L.inst), *toff = reinterpret_cast<int *>(h + L.toff);
     int *tx = reinterpret_cast<int *>(h + L.tx), *ty = reinterpret_cast<int *>(h + L.ty);
-    int *boff = reinterpret_cast<int *>(h + L.boff);
+    int *boff = reinterpret_cast<int *>(h + L.boff), *chk = reinterpret_cast<int *>(h + L.chk);
+    int64_t *cnt = reinterpret_cast<int64_t *>(h + L.cnt);
+    const int view_chunks = P.bin.chunks / a.nv;
     float *imd = reinterpret_cast<float *>(h + L.imd), *adam = reinterpret_cast<float *>(h + L.adam);
     int to = 0, bo = 0;
     int64_t po = 0;
@@ -223,6 +233,8 @@ void fill_blob(unsigned char *h, const StepArgs &a, const StepPtrs &P) {
         p.radii = P.radii;
         p.aabb = P.aabb;
         p.n_tiles = P.n_tiles;
+        p.depth_keys = P.depth.keys[0];
+        p.depth_vals = P.depth.vals[0];
 
         RasterArgs &r = ra[v];
         r.W = W;
@@ -271,6 +283,8 @@ void fill_blob(unsigned char *h, const StepArgs &a, const StepPtrs &P) {
 
         inst[v] = v * a.n;
         toff[v] = to;
+        chk[v] = v * view_chunks;
+        cnt[v] = (int64_t)view_chunks * to;
         tx[v] = tX;
         ty[v] = tY;
         boff[v] = bo;
@@ -281,6 +295,7 @@ void fill_blob(unsigned char *h, const StepArgs &a, const StepPtrs &P) {
     }
     inst[a.nv] = a.nv * a.n;
     toff[a.nv] = to;
+    chk[a.nv] = a.nv * view_chunks;
     boff[a.nv] = bo;
     for (int g = 0; g < 6; g++) {
         adam[g] = a.ss ? a.ss[g] : 0.f;
@@ -288,48 +303,26 @@ void fill_blob(unsigned char *h, const StepArgs &a, const StepPtrs &P) {
     }
 }
 
-BatchDesc batch_desc(const StepPtrs &P, int nv) {
-    const BlobLayout L(nv);
-    BatchDesc d;
-    d.n_views = nv;
-    d.inst_off = reinterpret_cast<const int *>(P.desc + L.inst);
-    d.tile_off = reinterpret_cast<const int *>(P.desc + L.toff);
-    d.tiles_x = reinterpret_cast<const int *>(P.desc + L.tx);
-    d.tiles_y = reinterpret_cast<const int *>(P.desc + L.ty);
-    d.proj = reinterpret_cast<const ProjectArgs *>(P.desc + L.proj);
-    d.raster = reinterpret_cast<const RasterArgs *>(P.desc + L.ras);
-    return d;
-}
-
-// Projection, the instances' depth order and the scan of their tile counts in that
-// order (emission offsets; total -> P.total).
-void enqueue_count(const StepArgs &a, const StepPtrs &P, cudaStream_t st) {
-    const BatchDesc d = batch_desc(P, a.nv);
+// Projection, the instances' depth order and emission offsets (the total -> P.total),
+// and every tile's count and place.
+void enqueue_count(const StepArgs &a, StepPtrs &P, cudaStream_t st) {
     const int inst = a.nv * a.n;
-    launch_project_batch(d, inst, st);
-    DepthScratch ds = P.depth;
-    launch_depth_offsets(inst, P.splats, P.n_tiles, ds, P.offsets, P.total, P.scan_part, st);
+    launch_project_batch(P.bin.d, inst, st);
+    launch_depth_order(P.bin, P.depth, P.scan_part, P.total, st);
+    launch_bin_count(P.bin, P.offsets, st);
 }
 
-// Everything after the count: capacity check, emission, sort, ranges, forward,
-// loss, backward and Adam. tiles_hint / isect_hint: host-known counts (0 = device).
+// Everything after the count: capacity check, the tiles' lists, forward, loss, backward
+// and Adam. tiles_hint: the host-known tile count (0 = device).
 // tm: stage timer (eager steps only; null while capturing).
-void enqueue_rest(const StepArgs &a, const StepPtrs &P, int64_t isect_cap, int tile_cap, int tiles_hint,
+void enqueue_rest(const StepArgs &a, const StepPtrs &P, int64_t isect_cap, int tiles_hint,
                   cudaStream_t st, StageTimer *tm) {
     const BlobLayout L(a.nv);
-    const BatchDesc d = batch_desc(P, a.nv);
-    const int inst = a.nv * a.n;
+    const BatchDesc &d = P.bin.d;
     int *d_n = P.counters + C_NISECT, *d_over = P.counters + C_OVERFLOW;
     cudaMemsetAsync(P.counters, 0, N_COUNTERS * sizeof(int), st);
-    launch_clamp_count(P.total, isect_cap, d_n, d_over, st);
-    launch_emit_keys_batch(inst, P.splats, P.aabb, P.n_tiles, P.offsets, nullptr, d, P.k[0], P.v[0], P.emit_gid, st,
-                           isect_cap);
-    uint32_t *kk[2] = {P.k[0], P.k[1]};
-    uint32_t *vv[2] = {P.v[0], P.v[1]};
-    const int cap = (int)isect_cap;
-    const int cur = radix_sort_pairs32(kk, vv, cap, ceil_log2(std::max(tile_cap, 1)), P.rscratch, st, d_n);
-    launch_tile_ranges(kk[cur], cap, tile_cap, P.tile_start, P.tile_end, st, d_n, d.tile_off + a.nv);
-    launch_isect_map(vv[cur], cap, P.emit_gid, P.isect_gid, P.inv, st, d_n);
+    launch_bin_clamp(P.bin, isect_cap, d_n, d_over, st);
+    launch_bin_emit(P.bin, P.isect_gid, P.inv, isect_cap, st);
     if (tm) tm->mark(2, st);
     launch_raster_fwd_batch(d, tiles_hint, P.counters + C_RAS, st, a.variant, a.shape);
     if (tm) tm->mark(3, st);
@@ -394,10 +387,10 @@ std::vector<uint64_t> graph_key(const StepArgs &a, const StepPtrs &P, int64_t is
     }
     u((uintptr_t)a.vis), u((uintptr_t)a.gn), u((uintptr_t)a.ms);
     const void *ptrs[] = {P.desc, P.splats, P.radii, P.n_tiles, P.aabb, P.offsets, P.scan_part, P.total,
-                          P.tile_start, P.tile_end, P.k[0], P.k[1], P.v[0], P.v[1], P.emit_gid, P.isect_gid, P.inv,
-                          P.slots, P.rscratch, P.img, P.T, P.v_img, P.idx, P.partials, P.losses, P.counters,
-                          P.depth.keys[0], P.depth.keys[1], P.depth.vals[0], P.depth.vals[1], P.depth.counts,
-                          P.depth.off_sorted};
+                          P.tile_start, P.tile_end, P.isect_gid, P.inv, P.slots, P.img, P.T, P.v_img, P.idx, P.partials, P.losses, P.counters,
+                          P.depth.keys[0], P.depth.keys[1], P.depth.vals[0], P.depth.vals[1], P.depth.radix_scratch,
+                          P.bin.rects, P.bin.rect_tiles, P.bin.offsets_sorted, P.bin.bounds,
+                          P.bin.counts};
     for (const void *p : ptrs) u((uintptr_t)p);
     return k;
 }
@@ -470,13 +463,15 @@ int step_eager(msplat_cuda_ctx *ctx, const StepArgs &a, const Sizes &sz, float *
     ctx->n_isect = total;
     if (total > tb.isect_cap) {
         // grow (with headroom for later steps) and describe the new buffers
+        const uint32_t *order = P.bin.order;  // its buffers do not depend on the intersections
         if (int r = ensure_buffers(ctx, sz, total + total / 4 + 1024, a.nv, P)) return r;
+        P.bin.order = order;
         if (int r = stage_slot(tb, L.bytes, &h)) return r;
         fill_blob(h, a, P);
         if (int r = upload_blob(tb, h, P.desc, L.bytes, st)) return r;
     }
     ctx->timer.mark(1, st);
-    enqueue_rest(a, P, tb.isect_cap, tb.tile_cap, (int)sz.tiles, st, &ctx->timer);
+    enqueue_rest(a, P, tb.isect_cap, (int)sz.tiles, st, &ctx->timer);
     CUDA_TRY(cudaGetLastError());
     if (losses_out) {
         CUDA_TRY(cudaMemcpyAsync(losses_out, P.losses, a.nv * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -511,7 +506,7 @@ int step_graph(msplat_cuda_ctx *ctx, const StepArgs &a, const Sizes &sz, float *
         cudaGraph_t g = nullptr;
         CUDA_TRY(cudaStreamBeginCapture(gs, cudaStreamCaptureModeThreadLocal));
         enqueue_count(a, P, gs);
-        enqueue_rest(a, P, tb.isect_cap, tb.tile_cap, 0, gs, nullptr);
+        enqueue_rest(a, P, tb.isect_cap, 0, gs, nullptr);
         cudaError_t e = cudaStreamEndCapture(gs, &g);
         if (e != cudaSuccess) return fail(MSPLAT_CUDA_ECUDA, "graph capture: %s", cudaGetErrorString(e));
         e = cudaGraphInstantiate(&tb.exec, g, 0);
