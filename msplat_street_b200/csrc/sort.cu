@@ -3,6 +3,8 @@
 // The radix sort is reduce-then-scan per 8-bit digit: a histogram kernel, a device
 // scan of the digit-major counts, and a scatter kernel that ranks keys stably inside
 // each 2048-key block with warp ballots and popc. No block waits on another block.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <atomic>
 
@@ -153,7 +155,7 @@ constexpr int RADIX = 256;
 // keys, 256 x 8 (2048 keys a block) keeps enough blocks to fill the GPU; 64-bit keys
 // take 2048-key blocks too (4096 would need 48 KB of staging per block). Measured and
 // not kept: 512 x 8 and 1024 x 4 blocks for the large 32-bit sort (two and one blocks
-// per SM: the 46 M-key tile sort of a 1080p frame 1.06 and 1.51 ms against 1.02), and
+// per SM: a sort of 46 M keys of 13 bits 1.06 and 1.51 ms against 1.02), and
 // the largest shared-memory carveout (1.06 ms: the scatter's loads and stores want
 // the L1). The scatter is bound by its integer pipe (ALU 64 % of peak, issue 54 %):
 // the ranking's ballots, not DRAM, set its pace.
@@ -327,6 +329,134 @@ __global__ void __launch_bounds__(THREADS, sizeof(K) == 8 ? 1024 / THREADS : 512
     }
 }
 
+// Sorts of at most CLUSTER_SORT 32-bit keys (the depth order of a small scene): one
+// cluster of eight blocks keeps them in registers and distributed shared memory through
+// all the passes. A block ranks its part as the scatter does, the blocks exchange their
+// digit counts, and every key goes straight to its place in the shared memory of the
+// block that holds it next. In place; one launch where the histogram and scatter kernels
+// take two a pass, few blocks each: 10 k keys of 32 bits, 30 -> 21 us.
+constexpr int CLUSTER_BLOCKS = 8, CLUSTER_THREADS = 1024;
+constexpr int CLUSTER_MAX_ITEMS = 8, CLUSTER_SORT = CLUSTER_BLOCKS * CLUSTER_THREADS * CLUSTER_MAX_ITEMS;
+
+// per: keys a block holds, a multiple of 32, at most CLUSTER_THREADS * KEYS.
+template <int KEYS>
+__global__ void __cluster_dims__(CLUSTER_BLOCKS, 1, 1) __launch_bounds__(CLUSTER_THREADS)
+    radix_cluster_kernel(uint32_t *keys, uint32_t *vals, int n, int key_bits, int per) {
+    namespace cg = cooperative_groups;
+    constexpr int WARPS = CLUSTER_THREADS / 32;
+    __shared__ uint32_t wcnt[WARPS][RADIX];
+    __shared__ uint32_t counts[CLUSTER_BLOCKS][RADIX];  // every block's, by digit
+    __shared__ uint32_t start[RADIX], ws[33];
+    extern __shared__ __align__(16) unsigned char sort_smem[];  // per keys, per values
+    uint32_t *skey = reinterpret_cast<uint32_t *>(sort_smem), *sval = skey + per;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int me = (int)cluster.block_rank();
+    const int lo = min(n, me * per), m = min(n, lo + per) - lo;  // this block's part
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int base = warp * KEYS * 32;  // the warp's keys lie side by side
+    const unsigned lt = (1u << lane) - 1u;
+    uint32_t key[KEYS], val[KEYS], rank[KEYS];
+    cluster.sync();  // every block runs before its shared memory is written to
+#pragma unroll
+    for (int r = 0; r < KEYS; r++) {
+        const int k = base + r * 32 + lane;
+        if (k < m) {
+            key[r] = keys[lo + k];
+            val[r] = vals[lo + k];
+        }
+    }
+    for (int shift = 0; shift < key_bits; shift += 8) {
+        const uint32_t mask = key_bits - shift < 8 ? (1u << (key_bits - shift)) - 1u : 255u;
+        for (int i = threadIdx.x; i < WARPS * RADIX; i += CLUSTER_THREADS) (&wcnt[0][0])[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < KEYS; r++) {
+            const int k0 = base + r * 32;
+            if (k0 >= m) continue;  // warp-uniform
+            const bool ok = k0 + lane < m;
+            const int d = ok ? (int)((key[r] >> shift) & mask) : RADIX;
+            const unsigned peers = digit_peers(d, mask, k0 + 32 <= m);
+            const uint32_t before = ok ? wcnt[warp][d] : 0u;
+            rank[r] = before + (uint32_t)__popc(peers & lt);
+            __syncwarp();
+            if (ok && lane == __ffs(peers) - 1) wcnt[warp][d] = before + (uint32_t)__popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        if (threadIdx.x < RADIX) {  // the warps' counts become prefixes; the sum goes to every block
+            uint32_t c[WARPS], tot = 0;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) c[w] = wcnt[w][threadIdx.x];
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) {
+                wcnt[w][threadIdx.x] = tot;
+                tot += c[w];
+            }
+            for (int q = 0; q < CLUSTER_BLOCKS; q++) *cluster.map_shared_rank(&counts[me][threadIdx.x], q) = tot;
+        }
+        cluster.sync();
+        uint32_t all = 0, before = 0;
+        if (threadIdx.x < RADIX)
+            for (int q = 0; q < CLUSTER_BLOCKS; q++) {
+                const uint32_t c = counts[q][threadIdx.x];
+                all += c;
+                if (q < me) before += c;
+            }
+        uint32_t total;
+        const uint32_t ex = block_exclusive_scan<uint32_t>(all, ws, total) + before;
+        if (threadIdx.x < RADIX) start[threadIdx.x] = ex;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < KEYS; r++) {
+            if (base + r * 32 + lane >= m) continue;
+            const int d = (int)((key[r] >> shift) & mask);
+            const uint32_t p = start[d] + wcnt[warp][d] + rank[r];
+            const uint32_t q = p / (uint32_t)per, i = p - q * (uint32_t)per;
+            *cluster.map_shared_rank(skey + i, q) = key[r];
+            *cluster.map_shared_rank(sval + i, q) = val[r];
+        }
+        cluster.sync();  // all keys have arrived; all blocks have read the counts
+#pragma unroll
+        for (int r = 0; r < KEYS; r++) {
+            const int k = base + r * 32 + lane;
+            if (k < m) {
+                key[r] = skey[k];
+                val[r] = sval[k];
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < KEYS; r++) {
+        const int k = base + r * 32 + lane;
+        if (k < m) {
+            keys[lo + k] = key[r];
+            vals[lo + k] = val[r];
+        }
+    }
+}
+
+template <int KEYS>
+void radix_cluster_launch(uint32_t *keys, uint32_t *vals, int n, int key_bits, int per, cudaStream_t st) {
+    static std::atomic<uint64_t> done{0};  // once per device: room for the largest part
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(done.load() & bit)) {
+        cudaFuncSetAttribute(radix_cluster_kernel<KEYS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             CLUSTER_THREADS * KEYS * 8);
+        done.fetch_or(bit);
+    }
+    radix_cluster_kernel<KEYS><<<CLUSTER_BLOCKS, CLUSTER_THREADS, (size_t)per * 8, st>>>(keys, vals, n, key_bits, per);
+}
+
+// Sorts (keys, vals) in place.
+void radix_cluster_sort(uint32_t *keys, uint32_t *vals, int n, int key_bits, cudaStream_t st) {
+    const int per = ((n + CLUSTER_BLOCKS - 1) / CLUSTER_BLOCKS + 31) / 32 * 32;
+    if (per <= CLUSTER_THREADS * 2) radix_cluster_launch<2>(keys, vals, n, key_bits, per, st);
+    else if (per <= CLUSTER_THREADS * 4) radix_cluster_launch<4>(keys, vals, n, key_bits, per, st);
+    else radix_cluster_launch<CLUSTER_MAX_ITEMS>(keys, vals, n, key_bits, per, st);
+}
+
 template <typename K, int THREADS, int ITEMS>
 constexpr size_t radix_scatter_smem() {
     return (size_t)THREADS * ITEMS * (sizeof(K) + sizeof(uint32_t));
@@ -381,6 +511,10 @@ template <typename K>
 int radix_sort_dispatch(K *k[2], uint32_t *v[2], int n, int key_bits, void *scratch, cudaStream_t st, const int *d_n) {
     if ((!d_n && n <= 1) || n <= 0 || key_bits <= 0) return 0;
     if constexpr (sizeof(K) == 4) {
+        if (!d_n && n <= CLUSTER_SORT) {
+            radix_cluster_sort(k[0], v[0], n, key_bits, st);
+            return 0;
+        }
         if (n >= LARGE_SORT) return radix_sort_impl<K, 256, 16>(k, v, n, key_bits, scratch, st, d_n);
     }
     return radix_sort_impl<K, 256, 8>(k, v, n, key_bits, scratch, st, d_n);
