@@ -15,7 +15,8 @@
 //     quaternion, colour and opacity rows and zeroes the moments, coalesced;
 //  4. cull (:1432-1448) over the N_new rows and order-preserving compaction of all 18
 //     buffers (6 parameters, 6 first moments, 6 second moments) through a scratch
-//     buffer, one buffer at a time (:1449-1464).
+//     buffer (:1449-1464): the 15 narrow ones together, then the SH rest and its moments
+//     one at a time.
 // A Gaussian can be both split (large on screen) and cloned (small in the world), so
 // the rows after step 3 number up to 4N, not 3N as the reference's capacity check
 // assumes (its CPU port would then write past its buffers). Here every kernel from
@@ -120,23 +121,33 @@ __global__ void densify_dup_kernel(DensifyArgs a, const int32_t *dup, const int3
     row_parent[r] = i;
 }
 
-// The new rows a.n .. total - 1 (split children, then clones), one thread per element:
-// quaternion, DC, SH rest and opacity copied from the row's parent, every moment
-// zeroed. Consecutive threads write consecutive floats of consecutive rows.
-__global__ void densify_rows_kernel(DensifyArgs a, const int32_t *n_split, const int32_t *n_dup,
-                                    const int32_t *row_parent, int g) {
+// The new rows a.n .. total - 1 (split children, then clones): quaternion, DC, SH rest
+// and opacity copied from the row's parent, every moment zeroed. blockIdx.y: the group;
+// a block takes ROWS new rows at a time as one flat range, consecutive threads
+// consecutive floats, with the rows' parents in shared memory. 84 -> 41 us for 137 k new
+// rows, against one launch a group with a 64-bit division a float.
+constexpr int ROWS = 256, ROW_THREADS = 256;
+
+__global__ void __launch_bounds__(ROW_THREADS) densify_rows_kernel(DensifyArgs a, const int32_t *n_split,
+                                                                   const int32_t *n_dup, const int32_t *row_parent) {
+    __shared__ int32_t parent[ROWS];
     int64_t total;
     if (!rows_fit(a, n_split, n_dup, total)) return;
-    const int st = a.stride[g];
-    const int64_t elems = (total - a.n) * st;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < elems;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / st;
-        const int col = (int)(t - r * st);
-        const int64_t dst = ((int64_t)a.n + r) * st + col;
-        if (g >= 2) a.buf[g][dst] = a.buf[g][(int64_t)row_parent[r] * st + col];
-        a.m1[g][dst] = 0.f;
-        a.m2[g][dst] = 0.f;
+    const int g = blockIdx.y, st = a.stride[g];
+    if (st <= 0) return;
+    const int64_t rows = total - a.n;
+    for (int64_t r0 = (int64_t)blockIdx.x * ROWS; r0 < rows; r0 += (int64_t)gridDim.x * ROWS) {  // block-uniform
+        const int here = (int)min((int64_t)ROWS, rows - r0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < here; i += ROW_THREADS) parent[i] = row_parent[r0 + i];
+        __syncthreads();
+        const int64_t dst = ((int64_t)a.n + r0) * st;
+        for (int j = threadIdx.x; j < here * st; j += ROW_THREADS) {
+            const int row = j / st;
+            if (g >= 2) a.buf[g][dst + j] = a.buf[g][(int64_t)parent[row] * st + j - row * st];
+            a.m1[g][dst + j] = 0.f;
+            a.m2[g][dst + j] = 0.f;
+        }
     }
 }
 
@@ -163,43 +174,82 @@ __global__ void densify_cull_kernel(DensifyArgs a, const int32_t *split, const i
     keep[i] = cull ? 0 : 1;
 }
 
-// one buffer: kept rows to scratch at their ordinal, then back. Grid-stride loops with
-// several elements per thread keep more loads in flight; the copy back moves float4s
-// when both arrays are 16-byte aligned.
-constexpr int COMPACT_ITEMS = 4;
+// Compaction of several buffers at once (blockIdx.y): kept rows to scratch at their
+// ordinal, then back. A block takes ROWS source rows as one flat range, four floats a
+// thread and load, with the rows' destinations in shared memory; the rows kept lie side
+// by side in the scratch, so the stores of neighbouring threads do too. The copy back
+// moves float4s when both arrays are 16-byte aligned. 300 k Gaussians at SH degree 3 (437 k
+// rows before, 357 k after): gather 343 -> 207 us and copy 152 -> 112 us against one
+// thread a float with a 64-bit division and two look-ups each, a launch pair per buffer.
+constexpr int MAX_COMPACT = 15;
+struct CompactArgs {
+    float *buf[MAX_COMPACT];
+    int64_t at[MAX_COMPACT];  // its place in the scratch, floats
+    int stride[MAX_COMPACT];
+};
 
-__global__ void compact_gather_kernel(const float *src, float *scratch, int stride, const int32_t *keep,
-                                      const int32_t *keep_ord, const int32_t *n_new) {
-    const int64_t elems = (int64_t)(*n_new) * stride;
-    const int64_t step = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; base < elems; base += step * COMPACT_ITEMS) {
+__global__ void __launch_bounds__(ROW_THREADS) compact_gather_kernel(const CompactArgs c, float *scratch,
+                                                                     const int32_t *keep, const int32_t *keep_ord,
+                                                                     const int32_t *n_new) {
+    __shared__ int32_t to[ROWS];
+    const int64_t rows = *n_new;
+    const int st = c.stride[blockIdx.y];
+    const float *src = c.buf[blockIdx.y];
+    float *dst = scratch + c.at[blockIdx.y];
+    const bool vec4 = (reinterpret_cast<uintptr_t>(src) & 15) == 0;  // a block's first float is a multiple of 256
+    for (int64_t r0 = (int64_t)blockIdx.x * ROWS; r0 < rows; r0 += (int64_t)gridDim.x * ROWS) {  // block-uniform
+        const int here = (int)min((int64_t)ROWS, rows - r0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < here; i += ROW_THREADS) to[i] = keep[r0 + i] ? keep_ord[r0 + i] : -1;
+        __syncthreads();
+        const float *from = src + r0 * st;
+        const int floats = here * st, n4 = vec4 ? floats / 4 : 0;
+        constexpr int AHEAD = 4;  // loads before the first store
+        for (int q0 = threadIdx.x; q0 < n4; q0 += AHEAD * ROW_THREADS) {
+            float4 v[AHEAD];
 #pragma unroll
-        for (int u = 0; u < COMPACT_ITEMS; u++) {
-            const int64_t t = base + u * step;
-            if (t >= elems) break;
-            const int64_t row = t / stride;
-            if (!keep[row]) continue;
-            const int col = (int)(t - row * stride);
-            scratch[(int64_t)keep_ord[row] * stride + col] = src[t];
+            for (int h = 0; h < AHEAD; h++) {
+                const int q = q0 + h * ROW_THREADS;
+                if (q < n4) v[h] = reinterpret_cast<const float4 *>(from)[q];
+            }
+#pragma unroll
+            for (int h = 0; h < AHEAD; h++) {
+                const int q = q0 + h * ROW_THREADS;
+                if (q >= n4) break;
+                const float f[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+                int row = 4 * q / st, col = 4 * q - row * st;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int o = to[row];
+                    if (o >= 0) dst[(int64_t)o * st + col] = f[u];
+                    if (++col == st) {
+                        col = 0;
+                        if (++row == here) break;  // past the last float
+                    }
+                }
+            }
+        }
+        for (int j = 4 * n4 + threadIdx.x; j < floats; j += ROW_THREADS) {
+            const int row = j / st, o = to[row];
+            if (o >= 0) dst[(int64_t)o * st + j - row * st] = from[j];
         }
     }
 }
 
-__global__ void compact_copy_back_kernel(float *dst, const float *scratch, int stride, const int32_t *new_count,
-                                         const int32_t *overflow, int vec4) {
+__global__ void compact_copy_back_kernel(const CompactArgs c, const float *scratch, const int32_t *new_count,
+                                         const int32_t *overflow) {
     if (*overflow) return;
-    const int64_t elems = (int64_t)(*new_count) * stride;
+    float *dst = c.buf[blockIdx.y];
+    const float *src = scratch + c.at[blockIdx.y];
+    const int64_t elems = (int64_t)(*new_count) * c.stride[blockIdx.y];
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (vec4) {
-        const int64_t n4 = elems / 4;
-        float4 *d4 = reinterpret_cast<float4 *>(dst);
-        const float4 *s4 = reinterpret_cast<const float4 *>(scratch);
-        for (int64_t t = t0; t < n4; t += step) d4[t] = s4[t];
-        for (int64_t t = 4 * n4 + t0; t < elems; t += step) dst[t] = scratch[t];
-    } else {
-        for (int64_t t = t0; t < elems; t += step) dst[t] = scratch[t];
-    }
+    const bool vec4 = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
+    const int64_t n4 = vec4 ? elems / 4 : 0;
+    float4 *d4 = reinterpret_cast<float4 *>(dst);
+    const float4 *s4 = reinterpret_cast<const float4 *>(src);
+    for (int64_t t = t0; t < n4; t += step) d4[t] = s4[t];
+    for (int64_t t = 4 * n4 + t0; t < elems; t += step) dst[t] = src[t];
 }
 
 __global__ void opacity_reset_kernel(float *o, float *m1, float *m2, int n, float reset_logit) {
@@ -225,27 +275,39 @@ void launch_densify(const DensifyArgs &a, DensifyScratch &s, cudaStream_t st) {
     densify_split_kernel<<<gb, bs, 0, st>>>(a, s.split, s.split_ord, s.n_split, s.n_dup, s.overflow, s.row_parent);
     densify_dup_kernel<<<gb, bs, 0, st>>>(a, s.dup, s.dup_ord, s.n_split, s.n_dup, s.row_parent);
     const int64_t rows = 4 * (int64_t)n;  // at most N + 2 N splits + N clones
-    for (int g = 0; g < 6; g++) {
-        if (a.stride[g] <= 0) continue;
-        const int64_t most = 3 * (int64_t)n * a.stride[g];  // new rows are at most 3 N
-        const unsigned grid = (unsigned)std::min<int64_t>((most + bs - 1) / bs, 148 * 64);
-        densify_rows_kernel<<<grid, bs, 0, st>>>(a, s.n_split, s.n_dup, s.row_parent, g);
-    }
+    const unsigned row_blocks = (unsigned)std::min<int64_t>((rows + ROWS - 1) / ROWS, 148 * 16);
+    densify_rows_kernel<<<dim3(row_blocks, 6), ROW_THREADS, 0, st>>>(a, s.n_split, s.n_dup, s.row_parent);
     densify_cull_kernel<<<(unsigned)((rows + bs - 1) / bs), bs, 0, st>>>(a, s.split, s.n_split, s.n_dup, s.keep,
                                                                        s.n_new);
     scan_exclusive<int32_t>(s.keep, s.keep_ord, (int)rows, s.new_count, s.scan_part, st);
-    const int sms_blocks = 148 * 8;  // enough resident blocks for the grid-stride loops
-    for (int b = 0; b < 18; b++) {
-        const int g = b % 6;
-        float *buf = b < 6 ? a.buf[g] : (b < 12 ? a.m1[g] : a.m2[g]);
-        const int stride = a.stride[g];
-        if (stride <= 0) continue;  // e.g. no SH rest at degree 0
-        const int64_t elems = rows * stride;
-        const unsigned grid =
-            (unsigned)std::max<int64_t>(1, std::min<int64_t>((elems / COMPACT_ITEMS + bs - 1) / bs, sms_blocks));
-        compact_gather_kernel<<<grid, bs, 0, st>>>(buf, s.scratch, stride, s.keep, s.keep_ord, s.n_new);
-        const int vec4 = ((reinterpret_cast<uintptr_t>(buf) | reinterpret_cast<uintptr_t>(s.scratch)) & 15) == 0;
-        compact_copy_back_kernel<<<grid, bs, 0, st>>>(buf, s.scratch, stride, s.new_count, s.overflow, vec4);
+    // the narrow groups' 15 buffers side by side in the scratch, then each SH-rest buffer
+    CompactArgs c;
+    int k = 0;
+    int64_t at = 0;
+    auto flush = [&] {
+        if (k > 0) {
+            compact_gather_kernel<<<dim3(row_blocks, (unsigned)k), ROW_THREADS, 0, st>>>(c, s.scratch, s.keep,
+                                                                                         s.keep_ord, s.n_new);
+            compact_copy_back_kernel<<<dim3(148 * 4, (unsigned)k), bs, 0, st>>>(c, s.scratch, s.new_count, s.overflow);
+        }
+        k = 0;
+        at = 0;
+    };
+    auto add = [&](float *buf, int stride) {
+        if (stride <= 0) return;  // e.g. no SH rest at degree 0
+        c.buf[k] = buf;
+        c.at[k] = at;
+        c.stride[k++] = stride;
+        at += (rows * stride + 3) / 4 * 4;
+    };
+    for (int g = 0; g < 6; g++) {
+        if (g == 4) continue;
+        for (float *buf : {a.buf[g], a.m1[g], a.m2[g]}) add(buf, a.stride[g]);
+    }
+    flush();
+    for (float *buf : {a.buf[4], a.m1[4], a.m2[4]}) {
+        add(buf, a.stride[4]);
+        flush();
     }
 }
 

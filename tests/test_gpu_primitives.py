@@ -152,6 +152,34 @@ def test_gpu_densify_matches_oracle(n, check_screen, check_huge):
         assert np.array_equal(t2[g].cpu().numpy()[:new_n], o2[g][:new_n]), g
 
 
+@pytest.mark.parametrize("n,rest,shift", [(64, 0, 0), (85, 9, 1), (127, 24, 0), (128, 72, 1), (129, 45, 1),
+                                          (257, 72, 0), (513, 9, 3)])
+def test_gpu_densify_row_blocks(n, rest, shift):
+    """Row counts around the compaction's 256-row blocks, every SH-rest width and buffers
+    that start off a 16-byte boundary, against the oracle, with the tolerance of the
+    larger cases above (a child's offset is one ulp off at most); moments exactly."""
+    cap = 4 * n
+    bufs, m1, m2, stats = _densify_inputs(n, cap, 90 + n)
+    rng = np.random.default_rng(n)
+    for arrays in (bufs, m1, m2):
+        arrays[4] = rng.random((cap, rest)).astype(np.float32)
+
+    def upload(a):
+        flat = torch.zeros(a.size + shift, dtype=torch.float32, device="cuda")
+        flat[shift:] = torch.from_numpy(a).reshape(-1).cuda()
+        return flat[shift:].view(a.shape)
+
+    ob, o1, o2 = [b.copy() for b in bufs], [b.copy() for b in m1], [b.copy() for b in m2]
+    new_o = Oracle("restatement").densify(n, cap, ob, o1, o2, stats, 60.0, 31)
+    tb, t1, t2 = ([upload(a) for a in arrays] for arrays in (bufs, m1, m2))
+    st = [torch.from_numpy(stats[k]).cuda() for k in ("gn", "vis", "ms")]
+    assert Context().densify(n, tb, t1, t2, st[0], st[1], st[2], 60.0, 31) == new_o
+    for g in range(6):
+        np.testing.assert_allclose(tb[g].cpu().numpy()[:new_o], ob[g][:new_o], rtol=1e-6, atol=1e-7, err_msg=str(g))
+        assert np.array_equal(t1[g].cpu().numpy()[:new_o], o1[g][:new_o]), g
+        assert np.array_equal(t2[g].cpu().numpy()[:new_o], o2[g][:new_o]), g
+
+
 def _split_and_clone_inputs(n, cap, seed):
     """Small Gaussians (world scale below size_thresh) that are large on screen and
     have high gradients: each one is both split and cloned, 4 n rows in all."""
