@@ -747,15 +747,14 @@ class TargetPrefetch:
 
 
 def launches_per_step(n_isect: float, n_gauss: float = 1e5) -> float:
-    """Kernels one plain training step launches: project, depth keys, the depth sort
-    (4 passes of hist + scatter, plus a 3-kernel scan per pass above 131,072
-    Gaussians), tile counts gathered, their 3-kernel scan, offsets scattered, emission,
-    the tile sort (2 passes of hist + 3-kernel scan + scatter for 2048 tiles), ranges,
-    map, raster forward, SSIM, loss finalize, raster backward, backward/Adam."""
-    tiles_bits = 11  # 1024x512 -> 2048 tiles
-    tile_passes = (tiles_bits + 7) // 8
-    depth_sort = 4 * (2 if n_gauss <= 131072 else 5)
-    return 1 + 1 + depth_sort + 1 + 3 + 1 + 1 + tile_passes * 5 + 1 + 1 + 1 + 1 + 1 + 1 + 1
+    """Kernels one plain training step launches: project, the depth sort (one cluster
+    launch up to 65,536 Gaussians, else 4 passes of hist + scatter, plus a 3-kernel scan
+    per pass above 131,072), tile rectangles, the scan of their counts (3 kernels, one up
+    to 16,384 Gaussians), the binning's count, prefix, list starts and emission, raster
+    forward, SSIM, loss finalize, raster backward, backward/Adam."""
+    depth_sort = 1 if n_gauss <= 65536 else 4 * (2 if n_gauss <= 131072 else 5)
+    scan = 1 if n_gauss <= 16384 else 3
+    return 1 + depth_sort + 1 + scan + 4 + 1 + 1 + 1 + 1 + 1
 
 
 # DRAM bytes read + written by one launch of the rasterizer backward, from an ncu
@@ -776,8 +775,9 @@ def stage_bytes(n_isects: float, n_gauss: float) -> dict:
     written once):
      proj_sh_fwd: 236 B of parameters read + 48 B splat record, radius, box, tile
        count (76 B) written per Gaussian;
-     bin_sort: key emission 12 B per intersection, the tile sort's passes 24 B per
-       intersection per pass (2 passes for 2048 tiles), ranges and map 8 + 8 B;
+     bin_sort: 4 B id and 4 B map entry written per intersection, the tile rectangle
+       and offset read twice (48 B) per Gaussian (the depth order counts under
+       proj_sh_fwd);
      rast_fwd: splat record 48 B + id 4 B per intersection, 20 B per pixel written;
      loss_fwd_bwd: 36 B per pixel (render + target read, gradient written);
      rast_bwd: 48 + 4 B per intersection read + 36 B slot written, 32 B per pixel read;
@@ -785,7 +785,7 @@ def stage_bytes(n_isects: float, n_gauss: float) -> dict:
        (264 B) + SH 48 x 3 x 2 (1152 B), 36 B slot per intersection read."""
     return {
         "proj_sh_fwd": n_gauss * (236 + 76),
-        "bin_sort": n_isects * (12 + 2 * 24 + 16),
+        "bin_sort": n_isects * 8 + n_gauss * 48,
         "rast_fwd": n_isects * 52 + NPIX * 20,
         "loss_fwd_bwd": NPIX * 36,
         "rast_bwd": n_isects * 88 + NPIX * 32,

@@ -75,15 +75,51 @@ __device__ __forceinline__ int exp_index(double x, double &k) {
     return __double2loint(shifted);
 }
 
-// v 2^m, exactly, for v in [1, 2) and m in [-1020, 0]: the exponent field moved
+// v 2^m, exactly, where v and the result are normal: the exponent field moved
 __device__ __forceinline__ double exp_scale(double v, int m) {
     return __hiloint2double(__double2hiint(v) + m * (1 << 20), __double2loint(v));
 }
 
+// 2^(j/128), rounded to double
+static __device__ const double EXP2_TABLE[EXP_TABLE] = {
+    0x1.0000000000000p+0, 0x1.0163da9fb3335p+0, 0x1.02c9a3e778061p+0, 0x1.04315e86e7f85p+0,
+    0x1.059b0d3158574p+0, 0x1.0706b29ddf6dep+0, 0x1.0874518759bc8p+0, 0x1.09e3ecac6f383p+0,
+    0x1.0b5586cf9890fp+0, 0x1.0cc922b7247f7p+0, 0x1.0e3ec32d3d1a2p+0, 0x1.0fb66affed31bp+0,
+    0x1.11301d0125b51p+0, 0x1.12abdc06c31ccp+0, 0x1.1429aaea92de0p+0, 0x1.15a98c8a58e51p+0,
+    0x1.172b83c7d517bp+0, 0x1.18af9388c8deap+0, 0x1.1a35beb6fcb75p+0, 0x1.1bbe084045cd4p+0,
+    0x1.1d4873168b9aap+0, 0x1.1ed5022fcd91dp+0, 0x1.2063b88628cd6p+0, 0x1.21f49917ddc96p+0,
+    0x1.2387a6e756238p+0, 0x1.251ce4fb2a63fp+0, 0x1.26b4565e27cddp+0, 0x1.284dfe1f56381p+0,
+    0x1.29e9df51fdee1p+0, 0x1.2b87fd0dad990p+0, 0x1.2d285a6e4030bp+0, 0x1.2ecafa93e2f56p+0,
+    0x1.306fe0a31b715p+0, 0x1.32170fc4cd831p+0, 0x1.33c08b26416ffp+0, 0x1.356c55f929ff1p+0,
+    0x1.371a7373aa9cbp+0, 0x1.38cae6d05d866p+0, 0x1.3a7db34e59ff7p+0, 0x1.3c32dc313a8e5p+0,
+    0x1.3dea64c123422p+0, 0x1.3fa4504ac801cp+0, 0x1.4160a21f72e2ap+0, 0x1.431f5d950a897p+0,
+    0x1.44e086061892dp+0, 0x1.46a41ed1d0057p+0, 0x1.486a2b5c13cd0p+0, 0x1.4a32af0d7d3dep+0,
+    0x1.4bfdad5362a27p+0, 0x1.4dcb299fddd0dp+0, 0x1.4f9b2769d2ca7p+0, 0x1.516daa2cf6642p+0,
+    0x1.5342b569d4f82p+0, 0x1.551a4ca5d920fp+0, 0x1.56f4736b527dap+0, 0x1.58d12d497c7fdp+0,
+    0x1.5ab07dd485429p+0, 0x1.5c9268a5946b7p+0, 0x1.5e76f15ad2148p+0, 0x1.605e1b976dc09p+0,
+    0x1.6247eb03a5585p+0, 0x1.6434634ccc320p+0, 0x1.6623882552225p+0, 0x1.68155d44ca973p+0,
+    0x1.6a09e667f3bcdp+0, 0x1.6c012750bdabfp+0, 0x1.6dfb23c651a2fp+0, 0x1.6ff7df9519484p+0,
+    0x1.71f75e8ec5f74p+0, 0x1.73f9a48a58174p+0, 0x1.75feb564267c9p+0, 0x1.780694fde5d3fp+0,
+    0x1.7a11473eb0187p+0, 0x1.7c1ed0130c132p+0, 0x1.7e2f336cf4e62p+0, 0x1.80427543e1a12p+0,
+    0x1.82589994cce13p+0, 0x1.8471a4623c7adp+0, 0x1.868d99b4492edp+0, 0x1.88ac7d98a6699p+0,
+    0x1.8ace5422aa0dbp+0, 0x1.8cf3216b5448cp+0, 0x1.8f1ae99157736p+0, 0x1.9145b0b91ffc6p+0,
+    0x1.93737b0cdc5e5p+0, 0x1.95a44cbc8520fp+0, 0x1.97d829fde4e50p+0, 0x1.9a0f170ca07bap+0,
+    0x1.9c49182a3f090p+0, 0x1.9e86319e32323p+0, 0x1.a0c667b5de565p+0, 0x1.a309bec4a2d33p+0,
+    0x1.a5503b23e255dp+0, 0x1.a799e1330b358p+0, 0x1.a9e6b5579fdbfp+0, 0x1.ac36bbfd3f37ap+0,
+    0x1.ae89f995ad3adp+0, 0x1.b0e07298db666p+0, 0x1.b33a2b84f15fbp+0, 0x1.b59728de5593ap+0,
+    0x1.b7f76f2fb5e47p+0, 0x1.ba5b030a1064ap+0, 0x1.bcc1e904bc1d2p+0, 0x1.bf2c25bd71e09p+0,
+    0x1.c199bdd85529cp+0, 0x1.c40ab5fffd07ap+0, 0x1.c67f12e57d14bp+0, 0x1.c8f6d9406e7b5p+0,
+    0x1.cb720dcef9069p+0, 0x1.cdf0b555dc3fap+0, 0x1.d072d4a07897cp+0, 0x1.d2f87080d89f2p+0,
+    0x1.d5818dcfba487p+0, 0x1.d80e316c98398p+0, 0x1.da9e603db3285p+0, 0x1.dd321f301b460p+0,
+    0x1.dfc97337b9b5fp+0, 0x1.e264614f5a129p+0, 0x1.e502ee78b3ff6p+0, 0x1.e7a51fbc74c83p+0,
+    0x1.ea4afa2a490dap+0, 0x1.ecf482d8e67f1p+0, 0x1.efa1bee615a27p+0, 0x1.f252b376bba97p+0,
+    0x1.f50765b6e4540p+0, 0x1.f7bfdad9cbe14p+0, 0x1.fa7c1819e90d8p+0, 0x1.fd3c22b8f71f1p+0,
+};
+
 // Every thread of the block calls each; the span is ready after the barrier that follows
 // init_b. t: EXP_TABLE doubles of scratch, read by init_b.
 __device__ __forceinline__ void exp_span_init_a(double *t) {
-    for (int j = threadIdx.x; j < EXP_TABLE; j += blockDim.x) t[j] = exp2((double)j * (1.0 / EXP_TABLE));
+    for (int j = threadIdx.x; j < EXP_TABLE; j += blockDim.x) t[j] = EXP2_TABLE[j];
 }
 __device__ __forceinline__ void exp_span_init_b(double *span, const double *t) {
     for (int i = threadIdx.x; i < EXP_SPAN; i += blockDim.x) span[i] = exp_scale(t[-i & (EXP_TABLE - 1)], -i >> EXP_BITS);
@@ -106,7 +142,20 @@ __device__ __noinline__ float exp_once(float xf) {
     double k;
     const int ki = exp_index(x, k);
     const double r = FAR ? fma(-k, EXP_LN2_T_LO, fma(-k, EXP_LN2_T_HI, x)) : fma(-k, EXP_LN2_T, x);
-    return (float)(exp_scale(exp2((double)(ki & (EXP_TABLE - 1)) * (1.0 / EXP_TABLE)), ki >> EXP_BITS) * exp_poly(r));
+    return (float)(exp_scale(EXP2_TABLE[ki & (EXP_TABLE - 1)], ki >> EXP_BITS) * exp_poly(r));
+}
+
+// exp(x) in double, rounded once to float, for any x: the same method with the power of
+// two applied to the exponent and the reduction in two steps (within about 1e-15 of
+// exp(x) over the range where the float result is neither 0 nor infinite). t: the
+// EXP_TABLE entries 2^(j/128) of exp_span_init_a.
+__device__ __forceinline__ float exp_wide(float xf, const double *t) {
+    if (xf != xf) return xf;
+    const double x = (double)fminf(fmaxf(xf, -110.f), 100.f);  // 0 and infinity beyond, as floats
+    double k;
+    const int ki = exp_index(x, k);
+    const double r = fma(-k, EXP_LN2_T_LO, fma(-k, EXP_LN2_T_HI, x));
+    return (float)exp_scale(t[ki & (EXP_TABLE - 1)] * exp_poly(r), ki >> EXP_BITS);
 }
 
 // Two float32 values in one 64-bit register pair, for sm_100's packed FP32

@@ -29,8 +29,9 @@ using proj_detail::xform43;
 // row makes every load instruction of the warp touch 32 sectors; when the warp's 32
 // lanes project Gaussians whose rows lie back to back in one array (row0, row0 + 45,
 // ...), the warp instead copies the 32 rows (1440 contiguous floats) into shared
-// memory with asynchronous 4-byte copies whose addresses are consecutive across the
-// lanes (4 sectors an instruction), which complete while the geometry runs. Every
+// memory with asynchronous copies (16 bytes each where the rows start on 16 bytes, else
+// 4) whose addresses are consecutive across the lanes, which complete while the geometry
+// runs. Every
 // lane of the warp must call issue_rest_rows; it returns whether the copies were
 // issued (warp-uniform). The caller then has every lane call rest_rows_wait before
 // any lane reads its row at buf + 45 * lane (stride 45 words: no bank conflicts).
@@ -42,6 +43,19 @@ __device__ __forceinline__ bool issue_rest_rows(const float *row, bool use, floa
         __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(row), 0));
     if (!__all_sync(0xffffffffu, use && row == row0 + PROJ_REST3 * lane)) return false;
     const unsigned dst = (unsigned)__cvta_generic_to_shared(buf);
+    if ((reinterpret_cast<uintptr_t>(row0) & 15) == 0) {  // warp-uniform
+        constexpr int N4 = 32 * PROJ_REST3 / 4;
+#pragma unroll
+        for (int k = 0; k < (N4 + 31) / 32; k++) {
+            const int e = k * 32 + lane;
+            if (e < N4)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16u * (unsigned)e),
+                             "l"(row0 + 4 * e)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        return true;
+    }
 #pragma unroll 9
     for (int k = 0; k < PROJ_REST3; k++) {
         const int e = k * 32 + lane;  // < 1440: inside the 32 rows
@@ -77,8 +91,9 @@ struct ProjState {
 
 // Geometry of Gaussian i (output slot o): cull, covariance, EWA, conic, radius, tile
 // rectangle, opacity and the pixel-reach extents. Returns false where the Gaussian
-// is culled (its radius and tile count left at zero).
-__device__ __forceinline__ bool project_geom(const ProjectArgs &a, int i, int64_t o, ProjState &st) {
+// is culled (its radius and tile count left at zero). exp_t: exp_wide's table.
+__device__ __forceinline__ bool project_geom(const ProjectArgs &a, int i, int64_t o, const double *exp_t,
+                                             ProjState &st) {
     a.radii[o] = 0;
     a.n_tiles[o] = 0;
     const float *vm = a.cam.viewmat;
@@ -86,7 +101,7 @@ __device__ __forceinline__ bool project_geom(const ProjectArgs &a, int i, int64_
     V3 pv = xform43(vm, pw);
     if (pv.z <= a.cam.clip) return false;
     V3 ls = ld3(a.scales, i);
-    V3 s{exp_ref(ls.x), exp_ref(ls.y), exp_ref(ls.z)};
+    V3 s{exp_wide(ls.x, exp_t), exp_wide(ls.y, exp_t), exp_wide(ls.z, exp_t)};
     const float4 qq = reinterpret_cast<const float4 *>(a.quats)[i];
     Q4 q{qq.x, qq.y, qq.z, qq.w};
     float cov[6];
@@ -140,38 +155,38 @@ __device__ __forceinline__ bool project_geom(const ProjectArgs &a, int i, int64_
     a.aabb[2 * o + 1] = ay;
 
     // sigmoid opacity as the pack step computes it (core/cpu/msplat_cpu.cpp:560)
-    const float op = 1.f / (1.f + exp_ref(-a.opacities[i]));
+    const float op = 1.f / (1.f + exp_wide(-a.opacities[i], exp_t));
     // Half-extents of the region a pixel can be composited in: sigma < 5.55 and
     // op * exp(-sigma) >= 1/255, i.e. 0.5 d^T conic d <= L. Its bounding box has
-    // half-widths sqrt(2 L conic_c / det) and sqrt(2 L conic_a / det), evaluated in
-    // double with margins, so the rasterizers may skip pixel blocks outside it without
-    // changing any result. An empty box marks a Gaussian that never reaches 1/255.
+    // half-widths sqrt(2 L conic_c / det) and sqrt(2 L conic_a / det), with margins far
+    // above the roundings, so the rasterizers may skip pixel blocks outside it without
+    // changing any result. An empty box marks a Gaussian that never reaches 1/255. The
+    // determinant and the sums below cancel for elongated splats and are taken in double;
+    // what follows them is single precision (its 1e-6 against margins of 1e-3; a
+    // determinant that a float could not hold counts as not positive definite).
     float ex = -1e30f, ey = -1e30f;
-    const double lg = log(255.0 * (double)op);
-    const double L = fmin(5.55, lg + 1e-4);
-    if (L > 0.0) {
-        const double ca = conic.x, cb = conic.y, cc = conic.z;
-        const double cdet = ca * cc - cb * cb;
-        if (cdet > 0.0 && ca > 0.0 && cc > 0.0) {
-            ex = (float)(sqrt(2.0 * L * cc / cdet) * 1.001 + 0.5);
-            ey = (float)(sqrt(2.0 * L * ca / cdet) * 1.001 + 0.5);
-        } else {
-            ex = ey = 1e30f;  // not positive definite: never skip
-        }
-    }
-    // The same region's half-extents along the diagonals, sqrt(2 L u^T C^-1 u) for
+    // the same region's half-extents along the diagonals, sqrt(2 L u^T C^-1 u) for
     // u = (1, 1) and (1, -1), with a wider margin on L: the rasterizers test each
     // warp's 8x4 pixel block against them (separating axes; rotated, elongated splats
     // have boxes much larger than themselves). Infinite: the box test alone.
     float hp = __int_as_float(0x7f800000), hm = hp;
-    {
-        const double ca = conic.x, cb = conic.y, cc = conic.z;
-        const double det2 = ca * cc - cb * cb;
-        const double Ld = fmin(5.55, lg) + 1e-2;
-        if (det2 > 0.0 && ca > 0.0 && cc > 0.0 && Ld > 0.0) {
-            hp = (float)(sqrt(2.0 * Ld * fmax(ca + cc - 2.0 * cb, 0.0) / det2) * 1.001 + 0.5);
-            hm = (float)(sqrt(2.0 * Ld * fmax(ca + cc + 2.0 * cb, 0.0) / det2) * 1.001 + 0.5);
+    const float lg = logf(255.f * op);
+    const float L = fminf(5.55f, lg + 1e-4f), Ld = fminf(5.55f, lg) + 1e-2f;
+    const double ca = conic.x, cb = conic.y, cc = conic.z;
+    const double cdet = ca * cc - cb * cb;
+    const bool definite = cdet > 1e-37 && ca > 0.0 && cc > 0.0;
+    const float idet = 2.f / (float)cdet;
+    if (L > 0.f) {
+        if (definite) {
+            ex = sqrtf(L * conic.z * idet) * 1.001f + 0.5f;
+            ey = sqrtf(L * conic.x * idet) * 1.001f + 0.5f;
+        } else {
+            ex = ey = 1e30f;  // not positive definite: never skip
         }
+    }
+    if (definite && Ld > 0.f) {
+        hp = sqrtf(Ld * (float)fmax(ca + cc - 2.0 * cb, 0.0) * idet) * 1.001f + 0.5f;
+        hm = sqrtf(Ld * (float)fmax(ca + cc + 2.0 * cb, 0.0) * idet) * 1.001f + 0.5f;
     }
     if (ex < -1e29f) ex = ey = -__int_as_float(0x7f800000);  // never reaches 1/255
     st.pw = pw;
