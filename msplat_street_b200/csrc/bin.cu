@@ -284,8 +284,28 @@ __global__ void __launch_bounds__(BIN_THREADS) bin_prefix_kernel(const BinArgs a
 // length. One block: a 1080p frame's 8160 tiles are one round.
 constexpr int SCAN_THREADS = 1024, SCAN_PER = 8;
 
-__global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(int T, int32_t *tile_start, int32_t *tile_end) {
+// order (ORDER; T <= BIN_ORDER_MAX): the tiles for the rasterizers' blocks, by the
+// length of their lists, the longest first, so that the last blocks to start are short
+// ones (a tile of the frame's last rows may hold its longest list). A counting sort over
+// eighths of each power of two; tiles of one step in no particular order, which changes
+// no tile's result. It costs 2.6 us for 2048 tiles; ball views at 1024 x 768 composite in
+// 120 instead of 132 us and their backward in 222 instead of 267 where the long lists come
+// late. Street steps at 1024 x 512 gain 3 % (852 -> 824 us), renders there 2.5 %; at 1600 x
+// 1060, eight rounds of blocks, nothing either way. Frames of up to BIN_ORDER_MIN tiles
+// start them all at once: ordering them made a 256 x 256 step 1.5 % slower.
+constexpr int ORDER_STEPS = 256;
+static_assert(BIN_ORDER_MAX <= SCAN_THREADS * SCAN_PER, "one round");
+
+__device__ __forceinline__ int order_step(int len) {
+    return len > 0 ? ORDER_STEPS - 2 - (int)((__float_as_uint((float)len) >> 20) - (127u << 3)) : ORDER_STEPS - 1;
+}
+
+template <bool ORDER>
+__global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(int T, int32_t *tile_start, int32_t *tile_end,
+                                                                  int32_t *order) {
     __shared__ long long ws[32];
+    __shared__ int step[ORDER ? ORDER_STEPS : 1], wsum[ORDER_STEPS / 32];
+    if (ORDER && threadIdx.x < ORDER_STEPS) step[threadIdx.x] = 0;  // read after the scan's barriers
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     long long carry = 0;
     for (int b0 = 0; b0 < T; b0 += SCAN_THREADS * SCAN_PER) {
@@ -343,6 +363,40 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(int T, int32_t
         }
         carry += all;
         __syncthreads();
+        if constexpr (!ORDER) continue;
+#pragma unroll
+        for (int j = 0; j < SCAN_PER; j++) {
+            v[j] = i0 + j < T ? order_step(v[j] - first[j]) : -1;
+            const unsigned none = __ballot_sync(0xffffffffu, v[j] == ORDER_STEPS - 1);  // often most of a frame
+            if (v[j] >= 0 && v[j] < ORDER_STEPS - 1) atomicAdd(&step[v[j]], 1);
+            if (lane == 0 && none) atomicAdd(&step[ORDER_STEPS - 1], __popc(none));
+        }
+        __syncthreads();
+        int c = 0, incl = 0;
+        if (threadIdx.x < ORDER_STEPS) {  // whole warps
+            c = incl = step[threadIdx.x];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += u;
+            }
+            if (lane == 31) wsum[warp] = incl;
+        }
+        __syncthreads();
+        if (threadIdx.x < ORDER_STEPS) {
+            for (int w = 0; w < warp; w++) incl += wsum[w];
+            step[threadIdx.x] = incl - c;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < SCAN_PER; j++) {
+            const unsigned none = __ballot_sync(0xffffffffu, v[j] == ORDER_STEPS - 1);
+            int at = 0;
+            if (lane == 0 && none) at = atomicAdd(&step[ORDER_STEPS - 1], __popc(none));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(none & ((1u << lane) - 1u));
+            if (v[j] >= 0 && v[j] < ORDER_STEPS - 1) at = atomicAdd(&step[v[j]], 1);
+            if (v[j] >= 0) order[at] = i0 + j;
+        }
     }
 }
 
@@ -567,7 +621,8 @@ void launch_bin_count(const BinArgs &a, int64_t *offsets, cudaStream_t st) {
     const int blocks = (a.tile_cap + 31) / 32;
     if (batch) bin_prefix_kernel<true><<<blocks, BIN_THREADS, 0, st>>>(a);
     else bin_prefix_kernel<false><<<blocks, BIN_THREADS, 0, st>>>(a);
-    bin_starts_kernel<<<1, SCAN_THREADS, 0, st>>>(a.tile_cap, a.tile_start, a.tile_end);
+    if (a.tile_order) bin_starts_kernel<true><<<1, SCAN_THREADS, 0, st>>>(a.tile_cap, a.tile_start, a.tile_end, a.tile_order);
+    else bin_starts_kernel<false><<<1, SCAN_THREADS, 0, st>>>(a.tile_cap, a.tile_start, a.tile_end, nullptr);
 }
 
 void launch_bin_emit(const BinArgs &a, int32_t *gids, int32_t *inv, int64_t cap, cudaStream_t st) {

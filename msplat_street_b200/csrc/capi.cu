@@ -90,6 +90,12 @@ SkyArgs sky_args(const msplat_cuda_prior &p, const CamParams &cam) {
     return s;
 }
 
+// The single-view frame's tile order, where it has one.
+const int32_t *frame_tile_order(const msplat_cuda_ctx *ctx, int tiles_x, int tiles_y) {
+    if (!ctx->ordered_frame || ctx->tiles_x != tiles_x || ctx->tiles_y != tiles_y) return nullptr;
+    return reinterpret_cast<const int32_t *>(ctx->tile_order.ptr);
+}
+
 // Projection, binning and forward rasterization: the shared forward of render and
 // train (core/cpu/msplat_cpu.cpp:629-657). One host synchronisation reads the
 // intersection count, which sizes the lists. With a prior whose aux flag is set, the
@@ -146,6 +152,11 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ENSURE(ctx->total, 1, int64_t, d_total);
     ENSURE(ctx->tile_start, T, int32_t, tile_start);
     ENSURE(ctx->tile_end, T, int32_t, tile_end);
+    int32_t *tile_order = nullptr;
+    if (T > BIN_ORDER_MIN && T <= BIN_ORDER_MAX) {
+        ENSURE(ctx->tile_order, T, int32_t, to);
+        tile_order = to;
+    }
     const size_t npix = (size_t)cam.width * cam.height;
     ENSURE(ctx->out_img, npix * 3, float, out_img);
     ENSURE(ctx->final_T, npix, float, final_T);
@@ -177,6 +188,7 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ba.n_tiles = n_tiles;
     ba.tile_start = tile_start;
     ba.tile_end = tile_end;
+    ba.tile_order = tile_order;
 
     ProjectArgs pa;
     pa.n = n;
@@ -223,6 +235,7 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ENSURE(ctx->isect_gid, n_isect, int32_t, isect_gid);
     ENSURE(ctx->inv, n_isect, int32_t, inv);
     if (!emitted) launch_bin_emit(ba, isect_gid, inv, n_isect, st);
+    ctx->ordered_frame = tile_order != nullptr;
 
     RasterArgs ra{};
     ra.W = (int)cam.width;
@@ -232,6 +245,7 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ra.tile_start = tile_start;
     ra.tile_end = tile_end;
     ra.isect_gid = isect_gid;
+    ra.tile_order = ctx->ordered_frame ? tile_order : nullptr;
     ra.n_isect = n_isect;
     ra.splats = splats;
     for (int c = 0; c < 3; c++) ra.bg[c] = bg[c];
@@ -457,6 +471,7 @@ int forward_batch(msplat_cuda_ctx *ctx, int nv, const msplat_cuda_view *views) {
         ra.tile_start = tile_start;
         ra.tile_end = tile_end;
         ra.isect_gid = isect_gid;
+        ra.tile_order = nullptr;
         ra.splats = splats;
         for (int c = 0; c < 3; c++) ra.bg[c] = w.background[c];
         ra.out_img = w.out_img;
@@ -845,6 +860,7 @@ int msplat_cuda_train_step(msplat_cuda_ctx *ctx, int num_points, float *means3d,
     rb.tile_start = reinterpret_cast<const int32_t *>(ctx->tile_start.ptr);
     rb.tile_end = reinterpret_cast<const int32_t *>(ctx->tile_end.ptr);
     rb.isect_gid = reinterpret_cast<const int32_t *>(ctx->isect_gid.ptr);
+    rb.tile_order = frame_tile_order(ctx, tiles_x, tiles_y);
     rb.splats = reinterpret_cast<const Splat *>(ctx->splats.ptr);
     for (int c = 0; c < 3; c++) rb.bg[c] = background[c];
     rb.final_T = reinterpret_cast<const float *>(ctx->final_T.ptr);
@@ -976,6 +992,7 @@ int msplat_cuda_render_backward(msplat_cuda_ctx *ctx, int num_points, const floa
     rb.tile_start = reinterpret_cast<const int32_t *>(ctx->tile_start.ptr);
     rb.tile_end = reinterpret_cast<const int32_t *>(ctx->tile_end.ptr);
     rb.isect_gid = reinterpret_cast<const int32_t *>(ctx->isect_gid.ptr);
+    rb.tile_order = frame_tile_order(ctx, tiles_x, tiles_y);
     rb.splats = reinterpret_cast<const Splat *>(ctx->splats.ptr);
     for (int c = 0; c < 3; c++) rb.bg[c] = background[c];
     rb.final_T = reinterpret_cast<const float *>(ctx->final_T.ptr);
@@ -1342,7 +1359,7 @@ int64_t msplat_cuda_ctx_device_bytes(msplat_cuda_ctx *ctx) {
                         &ctx->total, &ctx->v_xy, &ctx->v_conic, &ctx->v_rgb, &ctx->v_opacity, &ctx->v_mean3d,
                         &ctx->v_scale, &ctx->v_quat, &ctx->keys[0], &ctx->keys[1], &ctx->vals[0], &ctx->vals[1],
                         &ctx->isect_gid, &ctx->inv, &ctx->slots, &ctx->radix_scratch,
-                        &ctx->tile_start, &ctx->tile_end, &ctx->out_img, &ctx->final_T, &ctx->final_idx,
+                        &ctx->tile_start, &ctx->tile_end, &ctx->tile_order, &ctx->out_img, &ctx->final_T, &ctx->final_idx,
                         &ctx->v_rendered, &ctx->loss_part, &ctx->loss, &ctx->d_flags, &ctx->d_counts,
                         &ctx->d_scratch, &ctx->k_bounds, &ctx->k_sorted, &ctx->k_box, &ctx->k_md, &ctx->tstore,
                         &ctx->tcount, &ctx->bdesc, &ctx->bcounter, &ctx->tb.desc, &ctx->tb.pix_img,

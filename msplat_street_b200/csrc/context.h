@@ -191,12 +191,13 @@ struct msplat_cuda_ctx {
     // key / value buffers of the sort and kNN primitives, and the radix sorts' scratch
     Buf keys[2], vals[2], radix_scratch;
     // per tile / pixel
-    Buf tile_start, tile_end, out_img, final_T, final_idx, v_rendered, loss_part, loss;
+    Buf tile_start, tile_end, tile_order, out_img, final_T, final_idx, v_rendered, loss_part, loss;
     // densification and primitive scratch
     Buf d_flags, d_counts, d_scratch, k_bounds, k_sorted, k_box, k_md, k_evals;
     // stored-transmittance mode (option "store_transmittance" = per-pixel capacity)
     int tstore_cap = 0;
     Buf tstore, tcount;
+    bool ordered_frame = false;  // whether tile_order is the single-view frame's
     Buf pairs;  // the frame's pair counts (msplat_cuda_frame_pair_counts)
     // depth-chunked compositing: option "chunked_raster" (0 off, 1 frames of fewer
     // than CHUNK_AUTO_TILES tiles, 2 every frame) and "chunk_len"; whether the last
@@ -234,7 +235,7 @@ struct msplat_cuda_ctx {
     void release() {
         Buf *all[] = {&splats, &radii, &aabb, &n_tiles, &offsets, &scan_part, &total, &v_xy, &v_conic, &v_rgb,
                       &v_opacity, &v_mean3d, &v_scale, &v_quat, &keys[0], &keys[1], &vals[0], &vals[1],
-                      &isect_gid, &inv, &slots, &radix_scratch, &tile_start, &tile_end, &out_img, &final_T,
+                      &isect_gid, &inv, &slots, &radix_scratch, &tile_start, &tile_end, &tile_order, &out_img, &final_T,
                       &final_idx, &v_rendered, &loss_part, &loss, &d_flags, &d_counts, &d_scratch, &k_bounds,
                       &k_sorted, &k_box, &k_md, &k_evals, &tstore, &tcount, &pairs, &bdesc, &bcounter, &dkeys[0], &dkeys[1],
                       &dvals[0], &dvals[1], &rects, &rect_tiles, &off_sorted, &bin_bounds, &bin_counts, &img[0], &img[1], &img[2]};

@@ -52,6 +52,7 @@ int radix_sort_pairs32(uint32_t *k[2], uint32_t *v[2], int n, int key_bits, void
 struct RasterArgs {
     int W, H, tiles_x, tiles_y;
     const int32_t *tile_start, *tile_end, *isect_gid;
+    const int32_t *tile_order;  // single-view frames: the blocks' tiles (null: by index)
     int64_t n_isect;  // single-view frames: all entries, where the host knows them
     const Splat *splats;
     float bg[3];
@@ -176,7 +177,11 @@ struct BinArgs {
     int2 *bounds;             // per chunk: its positions
     int32_t *counts;          // per chunk, the tiles of its view
     int32_t *tile_start, *tile_end;
+    int32_t *tile_order;  // single views, may be null: the tiles, longest lists first
 };
+// A frame of more tiles than the GPU holds blocks of the rasterizers (148 SMs x 4), and
+// of no more than the scan of the list starts takes in one round, has its tiles ordered.
+constexpr int BIN_ORDER_MIN = 592, BIN_ORDER_MAX = 8192;
 int bin_chunk_len(int64_t n, int64_t tiles);
 int bin_chunks(int n, int len);
 void bin_plan(BinArgs &a);
@@ -192,6 +197,7 @@ void launch_raster_fwd_batch(const BatchDesc &d, int tiles_hint, int *d_counter,
 struct RasterBwdArgs {
     int W, H, tiles_x, tiles_y;
     const int32_t *tile_start, *tile_end, *isect_gid;
+    const int32_t *tile_order;  // single-view frames: the blocks' tiles (null: by index)
     const Splat *splats;
     float bg[3];
     const float *final_T;

@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_kernel(Ra
     extern __shared__ __align__(16) unsigned char fwd_smem[];
     FwdStage<FB, LINES> &s = *reinterpret_cast<FwdStage<FB, LINES> *>(fwd_smem);
     s.init();  // ready after the tile's first barrier
-    const int tile = blockIdx.x / SUB;
+    const int at = blockIdx.x / SUB, tile = a.tile_order ? a.tile_order[at] : at;
     raster_fwd_tile<FB, AUX, false, TS, NT, LINES>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s, nullptr, 0, 0,
                                                    blockIdx.x % SUB);
 }
@@ -764,7 +764,7 @@ template <int BB, int SB, bool AUX = false, bool TS = false>
 __global__ void __launch_bounds__(BWD_THREADS, BB <= 64 ? 6 : 5) raster_bwd_kernel(RasterBwdArgs a) {
     extern __shared__ __align__(16) float4 smem4[];
     __shared__ int kmax;
-    const int tile = blockIdx.x;
+    const int tile = a.tile_order ? a.tile_order[blockIdx.x] : blockIdx.x;
     raster_bwd_tile<BB, SB, AUX, false, TS>(a, tile, tile % a.tiles_x, tile / a.tiles_x, smem4, kmax);
 }
 

@@ -244,6 +244,7 @@ void fill_blob(unsigned char *h, const StepArgs &a, const StepPtrs &P) {
         r.tile_start = P.tile_start;
         r.tile_end = P.tile_end;
         r.isect_gid = P.isect_gid;
+        r.tile_order = nullptr;
         r.splats = P.splats;
         for (int c = 0; c < 3; c++) r.bg[c] = a.bg[c];
         r.out_img = P.img + 3 * po;
@@ -261,6 +262,7 @@ void fill_blob(unsigned char *h, const StepArgs &a, const StepPtrs &P) {
         b.tile_start = P.tile_start;
         b.tile_end = P.tile_end;
         b.isect_gid = P.isect_gid;
+        b.tile_order = nullptr;
         b.splats = P.splats;
         for (int c = 0; c < 3; c++) b.bg[c] = a.bg[c];
         b.final_T = P.T + po;

@@ -108,3 +108,29 @@ def test_batched_step_lists(nv):
         total = [a + b for a, b in zip(total, one)]
     for a, b in zip(grads, total):
         assert torch.equal(a, b)  # added view by view in both
+
+
+@pytest.mark.parametrize("n,w,h", [(3000, 592, 256), (3000, 9488, 16), (1, 1000, 500), (4000, 2048, 1024),
+                                   (4000, 2064, 1024)])
+def test_ordered_tiles_change_no_step(n, w, h):
+    """Frames around the tile counts whose blocks take the tiles by list length (593 to
+    8192; 592 and 8256 go by index; the one of a single Gaussian is mostly empty): two
+    steps equal the batched step's, whose tiles go by index, bit for bit."""
+    g = scenes.random_gaussians(n, 3 * n + w, log_scale_mean=-2.5)
+    cam = prepare_cam(look_at((0.2, 0.1, 2.6), (0, 0, 0)), w, h, 0.8 * h + 64, 0.8 * h + 64, w / 3.0, h / 2.0)
+    gt = torch.rand((h, w, 3), generator=torch.Generator().manual_seed(n)).cuda()
+    sides = []
+    for batch in (False, True):
+        p = GaussianParams.from_numpy(g)
+        adam = AdamState.zeros_like(p, C1_LRS)
+        stats = tuple(torch.zeros(n, device="cuda") for _ in range(3))
+        ctx = Context()
+        for _ in range(2):
+            if batch:
+                loss = float(ctx.train_batch(p, adam, [(cam, gt)], BACKGROUND, stats)[0])
+            else:
+                loss = ctx.train_step(p, adam, cam, BACKGROUND, gt, stats, sync_loss=True)
+        sides.append((loss, p.tensors() + adam.exp_avg + adam.exp_avg_sq + list(stats)))
+    assert sides[0][0] == sides[1][0]
+    for x, y in zip(sides[0][1], sides[1][1]):
+        assert torch.equal(x, y)
