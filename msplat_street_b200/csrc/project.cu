@@ -3,7 +3,7 @@
 // Follows project_and_sh (core/cpu/msplat_cpu.cpp:452-500) and its helpers
 // (:63-190). The output per visible Gaussian is one 48-byte Splat record (read by
 // both rasterizer passes), its depth, radius, pixel AABB half-extent and the number
-// of 16x16 tiles its AABB covers (the input of the key-emission scan). Compiled with
+// of 16x16 tiles its AABB covers (what the binning deals out). Compiled with
 // -fmad=false: tile rectangles and depth keys must equal the reference's bit for bit.
 #include "project_impl.cuh"
 

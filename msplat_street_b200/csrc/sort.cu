@@ -2,7 +2,8 @@
 //
 // The radix sort is reduce-then-scan per 8-bit digit: a histogram kernel, a device
 // scan of the digit-major counts, and a scatter kernel that ranks keys stably inside
-// each 2048-key block with warp ballots and popc. No block waits on another block.
+// each 2048-key block with warp ballots and popc, no block waiting on another; small
+// sorts of 32-bit keys run in one cluster of eight blocks instead.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -61,15 +61,22 @@ __device__ __forceinline__ void ssim_block(const SsimArgs &a, int bx, int by, in
     const int x0 = bx * ST, y0 = by * ST;
     const float w = a.ssim_weight;
     // 1. inputs, zero outside the image
-    for (int i = threadIdx.x; i < SH_IN * SH_IN; i += SSIM_THREADS) {
-        const int r = i / SH_IN, q = i - r * SH_IN;
+    constexpr int PER = (SH_IN * SH_IN + SSIM_THREADS - 1) / SSIM_THREADS;
+    float2 v[PER];  // all loads before the first store
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int i = threadIdx.x + k * SSIM_THREADS, r = i / SH_IN, q = i - r * SH_IN;
         const int gy = y0 - 10 + r, gx = x0 - 10 + q;
-        float2 v = make_float2(0.f, 0.f);
-        if (gy >= 0 && gy < H && gx >= 0 && gx < W) {
+        v[k] = make_float2(0.f, 0.f);
+        if (i < SH_IN * SH_IN && gy >= 0 && gy < H && gx >= 0 && gx < W) {
             const size_t idx = ((size_t)gy * W + gx) * 3 + c;
-            v = make_float2(a.gt[idx], a.img[idx]);
+            v[k] = make_float2(a.gt[idx], a.img[idx]);
         }
-        s.in[r * P_IN + q] = v;
+    }
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int i = threadIdx.x + k * SSIM_THREADS, r = i / SH_IN, q = i - r * SH_IN;
+        if (i < SH_IN * SH_IN) s.in[r * P_IN + q] = v[k];
     }
     __syncthreads();
     // this thread's output pixels (pass 5): column ox, rows oy .. oy + RUN_O - 1
@@ -165,10 +172,12 @@ __device__ __forceinline__ void ssim_block(const SsimArgs &a, int bx, int by, in
 // Block b of an image: tile b / 3, channel b % 3.
 //
 // Bound by FP32 issue: about 640 separately rounded operations a pixel and channel,
-// halo included. 1024 x 512: 92 -> 58 us, 256 x 256: 33 -> 15 us against the form that
+// halo included. 1024 x 512: 92 -> 55 us, 256 x 256: 33 -> 14 us against the form that
 // computed one output a thread and step (two shared loads a tap) with a tile's channels
 // one after another; the channels as blocks of their own triple the blocks of a small
-// frame.
+// frame, and the inputs' loads all start before the first is stored (58 and 15.5 us where
+// they did not). A packed instruction holds the FMA pipe as long as its two scalars:
+// packing the window sums' third value as well left the time where it was.
 __global__ void __launch_bounds__(SSIM_THREADS, 3) ssim_loss_kernel(SsimArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SsimSmem &s = *reinterpret_cast<SsimSmem *>(smem_raw);

@@ -11,8 +11,8 @@
 //
 // Work is numbered globally: instance v * N + i is Gaussian i seen by view v, tiles
 // and pixels run view after view. Each stage is one launch over the whole batch:
-// projection, scan, key emission, one stable radix sort of all (view, tile) keys,
-// tile ranges, and persistent rasterizer / SSIM / raster-backward kernels that pull
+// projection, the view-major depth order, binning by counting (every (view, tile)'s
+// list), and persistent rasterizer / SSIM / raster-backward kernels that pull
 // (view, tile) or (view, block) work items from counters, then the multi-view
 // backward + Adam kernel.
 //
