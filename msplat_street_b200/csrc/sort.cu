@@ -98,32 +98,56 @@ __global__ void scan_apply_kernel(const int32_t *in, int n, const TO *partials, 
 
 int scan_blocks(int n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
 
-// Small inputs: one 1024-thread block walks the array in chunks of 4096 with a
-// running carry (one launch instead of three).
-constexpr int SCAN_SMALL = 16384, SMALL_ITEMS = 4;
+// Small inputs: one 1024-thread block, 16 consecutive elements a thread (one launch
+// instead of three). Bound by latency: loads and stores of 16 bytes, one block-wide scan.
+// 10 k elements into 64 bits: 9.1 -> 5.7 us against rounds of four elements a thread.
+constexpr int SMALL_ITEMS = 16, SCAN_SMALL = 1024 * SMALL_ITEMS;
 
 template <typename TO>
 __global__ void __launch_bounds__(1024) scan_small_kernel(const int32_t *in, int n, TO *out, TO *total) {
     __shared__ TO ws[33];
-    TO carry = 0;
-    for (int base = 0; base < n; base += 1024 * SMALL_ITEMS) {
-        const int i0 = base + threadIdx.x * SMALL_ITEMS;
-        TO v[SMALL_ITEMS], s = 0;
+    const int i0 = threadIdx.x * SMALL_ITEMS;
+    // 16-byte accesses: the thread's first element lies on 64 bytes where the arrays do on 16
+    const bool wide = i0 + SMALL_ITEMS <= n &&
+                      ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    int32_t v[SMALL_ITEMS];
+    if (wide) {
 #pragma unroll
-        for (int j = 0; j < SMALL_ITEMS; j++) {
-            v[j] = i0 + j < n ? (TO)in[i0 + j] : TO(0);
-            s += v[j];
+        for (int j = 0; j < SMALL_ITEMS; j += 4) {
+            const int4 q = *reinterpret_cast<const int4 *>(in + i0 + j);
+            v[j] = q.x, v[j + 1] = q.y, v[j + 2] = q.z, v[j + 3] = q.w;
         }
-        TO tot;
-        TO ex = block_exclusive_scan<TO>(s, ws, tot) + carry;
+    } else {
+#pragma unroll
+        for (int j = 0; j < SMALL_ITEMS; j++) v[j] = i0 + j < n ? in[i0 + j] : 0;
+    }
+    TO s = 0, tot;
+#pragma unroll
+    for (int j = 0; j < SMALL_ITEMS; j++) s += (TO)v[j];
+    TO ex = block_exclusive_scan<TO>(s, ws, tot);
+    if (wide) {
+        constexpr int PER = 16 / sizeof(TO);
+        struct alignas(16) Pack {
+            TO e[PER];
+        };
+#pragma unroll
+        for (int j = 0; j < SMALL_ITEMS; j += PER) {
+            Pack p;
+#pragma unroll
+            for (int u = 0; u < PER; u++) {
+                p.e[u] = ex;
+                ex += (TO)v[j + u];
+            }
+            *reinterpret_cast<Pack *>(out + i0 + j) = p;
+        }
+    } else {
 #pragma unroll
         for (int j = 0; j < SMALL_ITEMS; j++) {
             if (i0 + j < n) out[i0 + j] = ex;
-            ex += v[j];
+            ex += (TO)v[j];
         }
-        carry += tot;
     }
-    if (threadIdx.x == 0 && total) *total = carry;
+    if (threadIdx.x == 0 && total) *total = tot;
 }
 
 template <typename TO>
