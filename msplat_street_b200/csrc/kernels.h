@@ -83,7 +83,7 @@ inline int variant_index(int v) { return (v >= 0 && v < N_RASTER_VARIANTS) ? v :
 
 // Block shapes of the batched forward rasterizer (pixels a block composites; every
 // shape walks the 16 x 16 tile's list, so all give the same bits): 16 x 16 (the
-// default), 16 x 8 and 8 x 8 (the reference's Metal thread-group shape).
+// default; a single view's launch may halve it), 16 x 8 and 8 x 8 (the reference's Metal thread-group shape).
 struct RasterShape {
     int w, h;
 };
