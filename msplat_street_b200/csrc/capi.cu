@@ -136,13 +136,10 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
             const float *bg) {
     cudaStream_t st = ctx->stream;
     const int T = cam.tiles_x * cam.tiles_y;
-    ctx->n = n;
-    ctx->W = (int)cam.width;
-    ctx->H = (int)cam.height;
-    ctx->tiles_x = cam.tiles_x;
-    ctx->tiles_y = cam.tiles_y;
     if (n > 0 && (!means || !scales || !quats || !dc || !opac || (cam.degree > 0 && !rest)))
         return fail(MSPLAT_CUDA_EINVAL, "null Gaussian parameter pointer");
+    ctx->drop_frame();
+    ctx->aux_frame = ctx->chunk_frame = false;
     ENSURE(ctx->splats, n, Splat, splats);
     ENSURE(ctx->radii, n, int32_t, radii);
     ENSURE(ctx->aabb, 2 * (size_t)n, float, aabb);
@@ -165,7 +162,6 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     const msplat_cuda_prior *pr = ctx->has_prior ? &ctx->prior : nullptr;
     const bool aux = pr && pr->aux;
     const bool sky = aux && pr->sky && pr->sky_tex;
-    ctx->aux_frame = aux;
     float *out_depth = nullptr, *bg_img = nullptr;
     if (aux) {
         ENSURE(ctx->pri[PB_DEPTH], npix, float, od);
@@ -235,7 +231,6 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ENSURE(ctx->isect_gid, n_isect, int32_t, isect_gid);
     ENSURE(ctx->inv, n_isect, int32_t, inv);
     if (!emitted) launch_bin_emit(ba, isect_gid, inv, n_isect, st);
-    ctx->ordered_frame = tile_order != nullptr;
 
     RasterArgs ra{};
     ra.W = (int)cam.width;
@@ -245,7 +240,7 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ra.tile_start = tile_start;
     ra.tile_end = tile_end;
     ra.isect_gid = isect_gid;
-    ra.tile_order = ctx->ordered_frame ? tile_order : nullptr;
+    ra.tile_order = tile_order;
     ra.n_isect = n_isect;
     ra.splats = splats;
     for (int c = 0; c < 3; c++) ra.bg[c] = bg[c];
@@ -269,7 +264,6 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     // rasterizer is one-pass only, as in core/metal/msplat_metal.mm:1103-1106)
     const bool chunked =
         !aux && T > 0 && (ctx->chunk_mode == 2 || (ctx->chunk_mode == 1 && T < CHUNK_AUTO_TILES));
-    ctx->chunk_frame = chunked;
     ChunkArgs ck{};
     if (chunked) {
         if (int r = chunk_buffers(ctx, T, false, ck)) return r;
@@ -290,6 +284,14 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     }
     ctx->timer.mark(3, st);
     CUDA_TRY(cudaGetLastError());
+    ctx->n = n;
+    ctx->W = (int)cam.width;
+    ctx->H = (int)cam.height;
+    ctx->tiles_x = cam.tiles_x;
+    ctx->tiles_y = cam.tiles_y;
+    ctx->ordered_frame = tile_order != nullptr;
+    ctx->aux_frame = aux;
+    ctx->chunk_frame = chunked;
     return MSPLAT_CUDA_OK;
 }
 
@@ -344,6 +346,7 @@ int forward_batch(msplat_cuda_ctx *ctx, int nv, const msplat_cuda_view *views) {
         ba.chunks += c;
         counts_len += (int64_t)c * ((w.img_width + TILE - 1) / TILE) * ((w.img_height + TILE - 1) / TILE);
     }
+    ctx->drop_frame();
     if (ctx->bdesc_pending) {  // the previous batch's raster upload still reads the staging
         CUDA_TRY(cudaEventSynchronize(ctx->bdesc_ev));
         ctx->bdesc_pending = false;
@@ -426,7 +429,6 @@ int forward_batch(msplat_cuda_ctx *ctx, int nv, const msplat_cuda_view *views) {
     d.raster = reinterpret_cast<const RasterArgs *>(d_desc + o_ras);
 
     ctx->n = n;
-    ctx->W = ctx->H = ctx->tiles_x = ctx->tiles_y = 0;  // no single-view frame to inspect
     ctx->timer.reset_marks();
     ctx->timer.mark(0, st);
     CUDA_TRY(cudaMemcpyAsync(d_desc, h, o_ras, cudaMemcpyHostToDevice, st));

@@ -232,7 +232,16 @@ struct msplat_cuda_ctx {
         release();
         timer.destroy();
     }
+    // No frame to inspect or to run a backward over. A call that replaces the frame's
+    // buffers drops it before it touches them and publishes its own when that is
+    // complete, so that a call that fails in between leaves none.
+    void drop_frame() {
+        n = W = H = tiles_x = tiles_y = 0;
+        n_isect = 0;
+        ordered_frame = false;
+    }
     void release() {
+        drop_frame();
         Buf *all[] = {&splats, &radii, &aabb, &n_tiles, &offsets, &scan_part, &total, &v_xy, &v_conic, &v_rgb,
                       &v_opacity, &v_mean3d, &v_scale, &v_quat, &keys[0], &keys[1], &vals[0], &vals[1],
                       &isect_gid, &inv, &slots, &radix_scratch, &tile_start, &tile_end, &tile_order, &out_img, &final_T,

@@ -583,8 +583,8 @@ extern "C" int msplat_cuda_train_batch(msplat_cuda_ctx *ctx, int num_points, flo
     if (sz.inst >= (int64_t)INT32_MAX || sz.tiles >= (int64_t)INT32_MAX || sz.pix >= (int64_t)INT32_MAX)
         return fail(MSPLAT_CUDA_EOVERFLOW, "batch too large: %lld instances, %lld tiles, %lld pixels",
                     (long long)sz.inst, (long long)sz.tiles, (long long)sz.pix);
+    ctx->drop_frame();
     ctx->n = (int)sz.inst;
-    ctx->W = ctx->H = ctx->tiles_x = ctx->tiles_y = 0;  // no single-view frame to inspect
     TrainBatchState &tb = ctx->tb;
     const bool use_graph = tb.graph && tb.isect_cap > 0 && sz.tiles <= tb.tile_cap;
     if (use_graph) {

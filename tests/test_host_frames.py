@@ -1,0 +1,72 @@
+"""What the C-ABI launches and leaves behind, on a recorded CUDA runtime (fake_cuda.py;
+no GPU): a call that fails leaves no frame that a later call would walk."""
+import pytest
+
+import fake_cuda
+
+N, W, H = 1000, 640, 480  # 1200 tiles
+
+
+def _frame_kernels(cuda):
+    return [k for k in cuda.launches() if "raster" in k[0] or "backward" in k[0] or "pair_count" in k[0]]
+
+
+def _fails_at_every_allocation(cuda):
+    """A larger frame after a good one, its allocations failing one after another."""
+    k, seen = 0, []
+    while True:
+        ctx = cuda.context()
+        cuda.allocs_left(-1)
+        cuda.readback(5000)
+        assert cuda.render(ctx, N, W, H) == 0 and cuda.lib.msplat_cuda_num_isects(ctx) == 5000
+        assert cuda.render_backward(ctx, N, W, H) == 0
+        cuda.readback(50_000_000)
+        cuda.allocs_left(k)
+        status = cuda.render(ctx, 20 * N, 2 * W, 2 * H)
+        cuda.allocs_left(-1)
+        if status == 0:
+            assert k > 10  # it does allocate
+            return seen
+        cuda.launches()
+        after = [cuda.render_backward(ctx, n, w, h) for n, w, h in ((20 * N, 2 * W, 2 * H), (N, W, H))]
+        seen.append((status, after, cuda.pair_counts(ctx), _frame_kernels(cuda)))
+        cuda.lib.msplat_cuda_ctx_destroy(ctx)
+        k += 1
+
+
+def test_failed_allocation_leaves_no_frame():
+    for k, (status, after, counts, launched) in enumerate(fake_cuda.run(_fails_at_every_allocation)):
+        assert status != 0
+        assert after == [1, 1], k  # EINVAL: no render of that scene and camera to follow
+        assert counts == 0 and launched == [], k
+
+
+def _too_many_entries(cuda, w, h):
+    ctx = cuda.context()
+    cuda.readback(5000)
+    assert cuda.render(ctx, N, W, H) == 0
+    cuda.readback(1 << 31)
+    status = cuda.render(ctx, N, w, h)
+    cuda.launches()
+    after = [cuda.render_backward(ctx, N, *s) for s in ((w, h), (W, H))]
+    return status, after, cuda.pair_counts(ctx), _frame_kernels(cuda), cuda.lib.msplat_cuda_num_isects(ctx)
+
+
+@pytest.mark.parametrize("size", [(W, H), (256, 256), (1920, 1088)])
+def test_too_many_intersections_leave_no_frame(size):
+    status, after, counts, launched, isects = fake_cuda.run(_too_many_entries, *size)
+    assert status == 4 and after == [1, 1] and counts == 0 and launched == [] and isects == 0
+
+
+def _refused(cuda):
+    ctx = cuda.context()
+    cuda.readback(5000)
+    assert cuda.render(ctx, N, W, H) == 0
+    view = list(cuda._view(2 * N, W, H, 0))
+    view[1] = None  # no means
+    status = cuda.lib.msplat_cuda_render(ctx, *view, 64, 64, 64, view[-1], None)
+    return status, cuda.render_backward(ctx, N, W, H)
+
+
+def test_refused_render_keeps_the_frame():
+    assert fake_cuda.run(_refused) == (1, 0)
