@@ -19,10 +19,10 @@ __device__ __forceinline__ void depth_key(const ProjectArgs &a, int o, bool kept
 
 // With SH degree 3 in use the warp stages its SH-rest rows while the geometry runs
 // (issue_rest_rows); no lane leaves before the wait that every lane of the warp takes.
-// Bound by the 236 bytes a Gaussian reads and by double-precision issue: the general exp
-// and log and four double square roots a Gaussian gave way to the table exponential and
-// single-precision extents, and 45 four-byte copies a lane to 12 of 16 bytes. 12 million
-// Gaussians over eight views 826 -> 751 us, 500 k in one 39 -> 37 us.
+// Bound by the 236 bytes a Gaussian reads and by double-precision issue: the general
+// exp gave way to the table exponential, three of the skip extents' four divisions to one
+// reciprocal, and 45 four-byte copies a lane to 12 of 16 bytes. 12 million Gaussians over
+// eight views 826 -> 775 us.
 __global__ void __launch_bounds__(PROJ_THREADS) project_kernel(ProjectArgs a) {
     __shared__ __align__(16) float rest_buf[PROJ_THREADS / 32][32 * PROJ_REST3];
     __shared__ double exp_t[EXP_TABLE];

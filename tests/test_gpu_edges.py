@@ -149,3 +149,35 @@ def test_slot_sums_of_every_size(n, scale, degree):
     ctx.train_batch(q, aq, [(cam, gt_t)], BACKGROUND, degrees_to_use=degree)
     for a, b in zip(p.tensors() + ap.exp_avg + ap.exp_avg_sq, q.tensors() + aq.exp_avg + aq.exp_avg_sq):
         assert torch.equal(a, b)
+
+
+def _half_up(x):
+    """float64 -> float32 (nearest) -> half (toward +infinity), as the record is packed."""
+    f = x.astype(np.float32)
+    with np.errstate(over="ignore"):
+        h = f.astype(np.float16)
+    return np.where(h.astype(np.float32) < f, np.nextafter(h, np.float16(np.inf)), h)
+
+
+def test_skip_extents_in_64_bits():
+    """The four extents of every visible Gaussian's record are the 64-bit ones of its conic
+    and opacity (a Gaussian that can reach no pixel has an empty box)."""
+    g = scenes.random_gaussians(200_000, 9, log_scale_mean=-4.0, log_scale_std=1.0)
+    g.opacities[:] = np.random.default_rng(9).normal(-4.0, 2.0, g.opacities.shape)
+    ctx = Context()
+    ctx.render(GaussianParams.from_numpy(g), scenes.small_camera(512, 384, 400.0), BACKGROUND)
+    rec = ctx.frame("splats").cpu().numpy().reshape(g.n, 12)[ctx.frame("radii").cpu().numpy() > 0]
+    a, b, c, op = (rec[:, k].astype(np.float64) for k in (2, 3, 4, 5))
+    got = np.ascontiguousarray(rec[:, 10:12]).view(np.float16)
+    lg, det = np.log(255.0 * op), a * c - b * b
+    reach, diag = np.minimum(5.55, lg + 1e-4), np.minimum(5.55, lg) + 1e-2
+    assert (det > 0).all() and (reach <= 0).any() and (diag <= 0).any()
+
+    def extent(level, num, none):
+        return np.where(level > 0, np.sqrt(np.maximum(2.0 * level * num / det, 0.0)) * 1.001 + 0.5, none)
+
+    want = [extent(reach, c, -np.inf), extent(reach, a, -np.inf), extent(diag, np.maximum(a + c - 2 * b, 0), np.inf),
+            extent(diag, np.maximum(a + c + 2 * b, 0), np.inf)]
+    assert len(rec) > 100_000
+    for k, w in enumerate(want):
+        assert np.array_equal(got[:, k], _half_up(w)), k
