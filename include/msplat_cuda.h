@@ -104,6 +104,9 @@ int msplat_cuda_frame_pair_counts_device(msplat_cuda_ctx *ctx, uint64_t *d_sum);
  * and the backward's 128-entry table with the power of two applied to the exponent)
  * and writes NaN wherever they differ. */
 int msplat_cuda_rasterizer_exp(msplat_cuda_ctx *ctx, const float *x, int64_t n, float *out);
+/* No counterpart in the reference (test hook). The projection's exponential (scales and
+ * sigmoid opacities), for any x. */
+int msplat_cuda_projection_exp(msplat_cuda_ctx *ctx, const float *x, int64_t n, float *out);
 /* Bytes of device memory the context's caches hold. */
 int64_t msplat_cuda_ctx_device_bytes(msplat_cuda_ctx *ctx);
 

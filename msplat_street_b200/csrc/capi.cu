@@ -1299,6 +1299,13 @@ int msplat_cuda_rasterizer_exp(msplat_cuda_ctx *ctx, const float *x, int64_t n, 
     return MSPLAT_CUDA_OK;
 }
 
+int msplat_cuda_projection_exp(msplat_cuda_ctx *ctx, const float *x, int64_t n, float *out) {
+    if (!ctx || (n > 0 && (!x || !out))) return fail(MSPLAT_CUDA_EINVAL, "null argument");
+    launch_exp_wide(x, n, out, ctx->stream);
+    CUDA_TRY(cudaGetLastError());
+    return MSPLAT_CUDA_OK;
+}
+
 namespace {
 // The pair counter's view of the context's last single-view frame.
 RasterArgs pair_count_args(const msplat_cuda_ctx *ctx) {

@@ -49,9 +49,10 @@ __device__ __forceinline__ float exp_ref(float x) { return (float)exp((double)x)
 // 1.6e-16), and 2^m 2^(j/128) comes from a table over the range that the block fills
 // once (exp_span_init_a, a barrier, exp_span_init_b). The reduction is one fused step:
 // k times the rounding of ln2 / 128 stays below 4.5e-16 for |k| <= 1026. The double
-// result is within about 1e-15 of exp(x), so the float it rounds to equals exp_ref's
-// unless exp(x) lies that close to a float rounding boundary. (A 64-entry table needs a
-// degree 5 and two reduction steps for the same: two operations more of fifteen.)
+// result is within about 1e-15 of exp(x); no float of [-5.55, 0] has its exponential that
+// close to a float rounding boundary: evaluated for all of them, the float is the
+// correctly rounded one, as that of a degree 5 with two reduction steps over 64 entries
+// is (two operations more of fifteen). A change to any constant here needs that check.
 constexpr double EXP_INV_LN2_T = 0x1.71547652b82fep+7;    // 128 / ln 2
 constexpr double EXP_LN2_T = 0x1.62e42fefa39efp-8;     // ln 2 / 128
 constexpr double EXP_LN2_T_HI = 0x1.62e42fefa2000p-8;  // its upper 40 bits: k * HI is exact
@@ -59,7 +60,7 @@ constexpr double EXP_LN2_T_LO = 0x1.9ef35793c7673p-48;  // ln 2 / 128 - HI
 constexpr int EXP_TABLE = 128, EXP_BITS = 7;
 constexpr int EXP_SPAN = 1040;  // covers k down to -1039 (x >= -5.62)
 
-// exp(r) - 1 over r, |r| <= ln2 / 256
+// exp(r), |r| <= ln2 / 256
 __device__ __forceinline__ double exp_poly(double r) {
     double p = fma(r, 0x1.55555acd08c2ep-5, 0x1.55555d88e27efp-3);
     p = fma(p, r, 0x1.fffffffffff58p-2);
@@ -146,9 +147,9 @@ __device__ __noinline__ float exp_once(float xf) {
 }
 
 // exp(x) in double, rounded once to float, for any x: the same method with the power of
-// two applied to the exponent and the reduction in two steps (within about 1e-15 of
-// exp(x) over the range where the float result is neither 0 nor infinite). t: the
-// EXP_TABLE entries 2^(j/128) of exp_span_init_a.
+// two applied to the exponent and the reduction in two steps (within about 5e-16 of
+// exp(x)). Evaluated for every float: the correctly rounded result, 0 and infinity
+// included. t: the EXP_TABLE entries 2^(j/128) of exp_span_init_a.
 __device__ __forceinline__ float exp_wide(float xf, const double *t) {
     if (xf != xf) return xf;
     const double x = (double)fminf(fmaxf(xf, -110.f), 100.f);  // 0 and infinity beyond, as floats

@@ -97,6 +97,8 @@ void launch_raster_fwd(const RasterArgs &a, cudaStream_t st, int variant = 0, in
 void launch_pair_counts(const RasterArgs &a, unsigned long long *d_out, cudaStream_t st, bool accumulate = false);
 // the rasterizers' exponential (exp_tab) of n device inputs
 void launch_exp_tab(const float *x, int64_t n, float *out, cudaStream_t st);
+// the projection's (exp_wide)
+void launch_exp_wide(const float *x, int64_t n, float *out, cudaStream_t st);
 void launch_raster_fwd_aux(const RasterArgs &a, cudaStream_t st, int shape = 0);
 
 struct RasterBwdArgs;

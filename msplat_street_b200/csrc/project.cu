@@ -5,6 +5,8 @@
 // both rasterizer passes), its depth, radius, pixel AABB half-extent and the number
 // of 16x16 tiles its AABB covers (what the binning deals out). Compiled with
 // -fmad=false: tile rectangles and depth keys must equal the reference's bit for bit.
+#include <algorithm>
+
 #include "project_impl.cuh"
 
 namespace msplat {
@@ -72,6 +74,20 @@ __global__ void __launch_bounds__(PROJ_THREADS) project_batch_kernel(const Batch
 void launch_project_batch(const BatchDesc &d, int total, cudaStream_t st) {
     if (total <= 0) return;
     project_batch_kernel<<<(total + PROJ_THREADS - 1) / PROJ_THREADS, PROJ_THREADS, 0, st>>>(d, total);
+}
+
+// The scales' and opacities' exponential over n inputs (test hook).
+__global__ void exp_wide_kernel(const float *x, int64_t n, float *out) {
+    __shared__ double t[EXP_TABLE];
+    exp_span_init_a(t);
+    __syncthreads();
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = exp_wide(x[i], t);
+}
+
+void launch_exp_wide(const float *x, int64_t n, float *out, cudaStream_t st) {
+    if (n <= 0) return;
+    exp_wide_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, st>>>(x, n, out);
 }
 
 }  // namespace msplat

@@ -262,3 +262,50 @@ def test_rasterizer_exponential_matches_double_exp():
         total += xt.numel()
     assert worst <= 1
     assert differ <= max(4, total // 10_000_000), (differ, total)
+
+
+def _nearest_to_exp(x, y):
+    """Whether float32 y is a float32 nearest to exp(x) (of a finite positive result)."""
+    import decimal
+    with decimal.localcontext() as dc:
+        dc.prec = 60
+        e = decimal.Decimal(float(x)).exp()
+        near = [np.nextafter(np.float32(y), np.float32(s)) for s in (0.0, np.inf)]
+        off = [abs(decimal.Decimal(float(v)) - e) for v in near if np.isfinite(v)]
+        return all(abs(decimal.Decimal(float(y)) - e) <= o for o in off)
+
+
+@pytest.mark.parametrize("hook,spans", [
+    ("rasterizer", [(-5.55, -2.0 ** -31)]),  # below 2^-31 in magnitude every exponential is 1
+    ("projection", [(2.0 ** -31, 101.0), (-112.0, -2.0 ** -31)]),
+])
+def test_exponentials_are_correctly_rounded(hook, spans):
+    """Every float of the ranges: the rasterizers' exponential over theirs, the projection's
+    over all whose result is neither 0, 1 nor infinite by magnitude alone. CUDA's double
+    exponential rounded to float stands for the exact value; where the two differ, the
+    exact value decides."""
+    import ctypes as C
+    from msplat_street_b200 import _lib
+    ctx = Context()
+    f = getattr(_lib.lib(), f"msplat_cuda_{hook}_exp")
+
+    def run(x):
+        got = torch.empty_like(x)
+        _lib.check(f(ctx.handle, C.c_void_p(x.data_ptr()), x.numel(), C.c_void_p(got.data_ptr())))
+        return got
+
+    for a, b in spans:
+        lo, hi = sorted(int(np.float32(abs(v)).view(np.int32)) for v in (a, b))
+        for s in range(lo, hi + 1, 1 << 25):
+            x = torch.arange(s, min(s + (1 << 25), hi + 1), dtype=torch.int32, device="cuda").view(torch.float32)
+            x = -x if a < 0 else x
+            got, ref = run(x), torch.exp(x.double()).float()
+            off = got != ref
+            assert int(off.sum()) < 1000
+            for xi, yi in zip(x[off].tolist(), got[off].tolist()):
+                assert _nearest_to_exp(xi, yi), (xi, yi)
+    if hook == "projection":
+        inf = float("inf")
+        x = torch.tensor([0.0, -0.0, 1e-45, -1e-45, -103.0, -104.0, -110.0, -1e9, -inf, 88.7, 88.73, 100.0, 3e38, inf,
+                          float("nan")], device="cuda")
+        assert torch.equal(run(x)[:-1], torch.exp(x.double()).float()[:-1]) and bool(run(x)[-1].isnan())
