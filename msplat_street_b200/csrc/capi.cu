@@ -241,7 +241,6 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ra.tile_end = tile_end;
     ra.isect_gid = isect_gid;
     ra.tile_order = tile_order;
-    ra.n_isect = n_isect;
     ra.splats = splats;
     for (int c = 0; c < 3; c++) ra.bg[c] = bg[c];
     ra.out_img = out_img;

@@ -53,7 +53,6 @@ struct RasterArgs {
     int W, H, tiles_x, tiles_y;
     const int32_t *tile_start, *tile_end, *isect_gid;
     const int32_t *tile_order;  // single-view frames: the blocks' tiles (null: by index)
-    int64_t n_isect;  // single-view frames: all entries, where the host knows them
     const Splat *splats;
     float bg[3];
     float *out_img, *final_T;

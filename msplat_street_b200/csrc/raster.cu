@@ -118,42 +118,20 @@ __device__ __forceinline__ float sigma_cut(float o) { return fminf(logf(255.f * 
 // A forward block's shared memory: one round of FB staged splats, and the exponential's
 // table.
 //
-// LINES: with each splat's terms of sigma per column and per row of the tile (32 pairs)
-// instead of its centre and conic, so that a visit costs three operations and two loads
-// for sigma instead of eleven and one. The forward is bound by instruction issue, and a
-// splat that reaches a tile is visited by most of its eight warps: 228 -> 185 warp
-// instructions an intersection with the exponential's shorter form, an early street view
-// 271 -> 257 us, eight mixed ones 3224 -> 3060. Whole-tile blocks of up to 128 staged
-// splats take it (42 KB a block, four blocks per SM); smaller blocks have fewer warps to
-// share the terms, and their occupancy would pay for the space. Two kinds of frames do
-// without as well (fwd_lines): those of fewer tiles than the GPU has places for, where a
-// block's own latency counts, which the terms' extra step lengthens (256 tiles: 40
-// against 43 us); and those of long lists, whose small splats reach few of a tile's warps
-// before its pixels are done (1600 entries a tile at 800 x 600: the frame 3 us slower
-// with the terms; 575 a tile: the 14 us faster of above).
-template <int FB, bool LINES>
-struct FwdGeom {
-    float4 axis[2][FB];   // (x, a / 2, b), (y, c / 2, 1)
-    float2 line[FB][32];  // columns (a/2 dx dx, b dx), then rows (c/2 dy dy, dy)
-};
+// Measured and not kept: each splat's terms of sigma per column and per row of the tile
+// in place of its centre and conic (three operations and two loads a visit for sigma
+// instead of eleven and one, 42 more stores a splat and 47 KB a block). Against these
+// blocks it lost in every frame and batch tried, from 300 to 14400 tiles and 120 to 6500
+// entries a tile: 100 k to 3 M Gaussians at 1024 x 768 2 to 5 %, 580 to 700 tiles 2 to 8 %,
+// an early street step 0.1 %, batches 1 to 3 %.
 template <int FB>
-struct FwdGeom<FB, false> {
-    float4 geom[FB];  // x, y, a / 2, b
-    float cz[FB];     // c / 2
-};
-template <int FB, int NT>
-constexpr bool can_lines = NT == FWD_THREADS && FB <= 128;
-constexpr int LINES_MIN_TILES = 4 * 148, LINES_MAX_LIST = 1024;
-inline bool fwd_lines(int tiles, int64_t isects) {
-    return tiles >= LINES_MIN_TILES && isects <= (int64_t)LINES_MAX_LIST * tiles;
-}
-template <int FB, bool LINES>
-struct FwdStage : FwdGeom<FB, LINES> {
+struct FwdStage {
+    float4 geom[FB];    // x, y, a / 2, b
     float4 colour[FB];  // colours as staged_colour leaves them, depth
     float2 cut[FB];     // opacity, sigma_cut
+    float cz[FB];       // c / 2
     double espan[EXP_SPAN];
     uint8_t mask[FB];   // warp_block_mask
-    unsigned alive;     // the warps with unfinished pixels (LINES)
     // the exponential's table; ready after the next block barrier
     __device__ __forceinline__ void init() {
         static_assert(sizeof(colour) >= EXP_TABLE * sizeof(double), "scratch for the table's first octave");
@@ -174,12 +152,11 @@ struct FwdStage : FwdGeom<FB, LINES> {
 // (rasterize_forward_aux, core/cpu/msplat_cpu.cpp:574-626 with f.aux).
 // CHUNK: composite only piece `chunk` of the list (ck->chunk_len long) from T = 1 and
 // write the piece's transmittance, colour and last contributor to item `item`.
-template <int FB, bool AUX, bool CHUNK, bool TS, int NT, bool LINES>
-__device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, int tx, int ty, FwdStage<FB, LINES> &s,
+template <int FB, bool AUX, bool CHUNK, bool TS, int NT>
+__device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, int tx, int ty, FwdStage<FB> &s,
                                                 const ChunkArgs *ck = nullptr, int item = 0, int chunk = 0,
                                                 int q = 0) {
     static_assert(!CHUNK || NT == FWD_THREADS, "depth pieces are composited by whole-tile blocks");
-    static_assert(!LINES || can_lines<FB, NT>, "a warp stages FB / 8 splats, a lane each");
     const int g = sub_tile_thread<NT>(threadIdx.x, q);  // this thread's place in the tile
     int lx, ly;
     tile_pixel(g, lx, ly);
@@ -198,58 +175,20 @@ __device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, i
     const size_t npix = (size_t)a.W * a.H;
     const size_t pid = inside ? (size_t)py * a.W + px : 0;
     int stored = 0;  // contributions seen (stored-transmittance mode)
-    // LINES: a warp whose pixels are all done leaves s.alive, and splats get their terms
-    // for the others only (a stale s.alive costs the terms of a splat nobody visits).
-    bool left = false;
-    if (LINES && threadIdx.x == 0) s.alive = 0xffu;
     for (int b0 = start; b0 < end; b0 += FB) {
-        if (LINES && b0 > start && !left && __all_sync(0xffffffffu, done)) {  // warp-uniform
-            if (lane == 0) atomicAnd(&s.alive, ~(1u << w));
-            left = true;
-        }
         if (__syncthreads_count(done) == NT) break;
-        if constexpr (LINES) {
-            // a warp stages FB / 8 splats: their records, then each one's 16 column and
-            // 16 row terms of sigma, a lane each
-            constexpr int PER = FB / (NT / 32);
-            const int wl = threadIdx.x >> 5, si = wl * PER + lane, k = b0 + si;
-            bool live = false;
-            if (lane < PER && k < end) {
-                const float4 *rec = reinterpret_cast<const float4 *>(a.splats + a.isect_gid[k]);
-                const float4 A = rec[0], B = rec[1], C = rec[2];
-                s.axis[0][si] = make_float4(A.x, 0.5f * A.z, A.w, 0.f);
-                s.axis[1][si] = make_float4(A.y, 0.5f * B.x, 1.f, 0.f);
-                s.cut[si] = make_float2(B.y, sigma_cut(B.y));
-                s.colour[si] = make_float4(staged_colour(B.z), staged_colour(B.w), staged_colour(C.x), C.y);
-                const uint32_t m = warp_block_mask(A, C, tx, ty) & s.alive;
-                s.mask[si] = (uint8_t)m;
-                live = m != 0u;
-            }
-            unsigned todo = __ballot_sync(0xffffffffu, live);
-            __syncwarp();
-            const int axis = lane >> 4;
-            const float origin = (float)((axis ? ty : tx) * TILE + (lane & 15));
-            while (todo) {  // warp-uniform
-                const int j = wl * PER + __ffs(todo) - 1;
-                todo &= todo - 1u;
-                const float4 p = s.axis[axis][j];
-                const float d = p.x - origin;
-                s.line[j][lane] = make_float2(p.y * d * d, p.z * d);
-            }
-        } else {
-            for (int si = threadIdx.x; si < FB; si += NT) {
-                const int k = b0 + si;
-                if (k >= end) break;
-                const float4 *rec = reinterpret_cast<const float4 *>(a.splats + a.isect_gid[k]);
-                const float4 A = rec[0], B = rec[1], C = rec[2];
-                // the conic's diagonal halved: 0.5 (a dx dx + c dy dy) == (a/2) dx dx +
-                // (c/2) dy dy bit for bit (scaling by 2^-1 commutes with each rounding)
-                s.geom[si] = make_float4(A.x, A.y, 0.5f * A.z, A.w);
-                s.cz[si] = 0.5f * B.x;
-                s.cut[si] = make_float2(B.y, sigma_cut(B.y));
-                s.colour[si] = make_float4(staged_colour(B.z), staged_colour(B.w), staged_colour(C.x), C.y);
-                s.mask[si] = (uint8_t)warp_block_mask(A, C, tx, ty);
-            }
+        for (int si = threadIdx.x; si < FB; si += NT) {
+            const int k = b0 + si;
+            if (k >= end) break;
+            const float4 *rec = reinterpret_cast<const float4 *>(a.splats + a.isect_gid[k]);
+            const float4 A = rec[0], B = rec[1], C = rec[2];
+            // the conic's diagonal halved: 0.5 (a dx dx + c dy dy) == (a/2) dx dx +
+            // (c/2) dy dy bit for bit (scaling by 2^-1 commutes with each rounding)
+            s.geom[si] = make_float4(A.x, A.y, 0.5f * A.z, A.w);
+            s.cz[si] = 0.5f * B.x;
+            s.cut[si] = make_float2(B.y, sigma_cut(B.y));
+            s.colour[si] = make_float4(staged_colour(B.z), staged_colour(B.w), staged_colour(C.x), C.y);
+            s.mask[si] = (uint8_t)warp_block_mask(A, C, tx, ty);
         }
         __syncthreads();
         const int cnt = min(FB, end - b0);
@@ -260,17 +199,9 @@ __device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, i
             while (bits && !done) {
                 const int j = base + __ffs(bits) - 1;
                 bits &= bits - 1u;
-                // sigma = (a/2 dx dx + c/2 dy dy) + b dx dy in the reference's roundings; a
-                // column's pixels share a/2 dx dx and b dx, a row's c/2 dy dy and dy
-                float sigma;
-                if constexpr (LINES) {
-                    const float2 cx = s.line[j][lx], cy = s.line[j][TILE + ly];
-                    sigma = (cx.x + cy.x) + cx.y * cy.y;
-                } else {
-                    const float4 A = s.geom[j];
-                    const float dx = A.x - fpx, dy = A.y - fpy;
-                    sigma = (A.z * dx * dx + s.cz[j] * dy * dy) + A.w * dx * dy;
-                }
+                const float4 A = s.geom[j];
+                const float dx = A.x - fpx, dy = A.y - fpy;
+                const float sigma = (A.z * dx * dx + s.cz[j] * dy * dy) + A.w * dx * dy;
                 const float2 cut = s.cut[j];
                 if (sigma < 0.f || sigma > cut.y) continue;
                 const float alpha = fminf(0.999f, cut.x * exp_span(-sigma, s.espan));
@@ -335,15 +266,14 @@ __device__ __forceinline__ void raster_fwd_tile(const RasterArgs &a, int tile, i
 
 // One block per sub-block of a tile (NT threads: the whole 16 x 16 tile, a 16 x 8
 // half or an 8 x 8 quarter; blocks SUB * t .. SUB * t + SUB - 1 share tile t's list).
-template <int FB, bool AUX, bool TS, int NT, bool LINES>
+template <int FB, bool AUX, bool TS, int NT>
 __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_kernel(RasterArgs a) {
     constexpr int SUB = FWD_THREADS / NT;
-    extern __shared__ __align__(16) unsigned char fwd_smem[];
-    FwdStage<FB, LINES> &s = *reinterpret_cast<FwdStage<FB, LINES> *>(fwd_smem);
+    __shared__ FwdStage<FB> s;
     s.init();  // ready after the tile's first barrier
     const int at = blockIdx.x / SUB, tile = a.tile_order ? a.tile_order[at] : at;
-    raster_fwd_tile<FB, AUX, false, TS, NT, LINES>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s, nullptr, 0, 0,
-                                                   blockIdx.x % SUB);
+    raster_fwd_tile<FB, AUX, false, TS, NT>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s, nullptr, 0, 0,
+                                            blockIdx.x % SUB);
 }
 
 // Persistent forward over the tiles of a batch of views (each with its own scene,
@@ -356,9 +286,7 @@ __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_kernel(Ra
 template <int FB, int NT>
 __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_batch_kernel(const BatchDesc d, int *counter) {
     constexpr int SUB = FWD_THREADS / NT;
-    constexpr bool LINES = can_lines<FB, NT>;
-    extern __shared__ __align__(16) unsigned char fwd_smem[];
-    FwdStage<FB, LINES> &s = *reinterpret_cast<FwdStage<FB, LINES> *>(fwd_smem);
+    __shared__ FwdStage<FB> s;
     __shared__ int s_item, s_lt;
     __shared__ RasterArgs s_args;  // the tile's view, read from shared memory (keeps registers down)
     s.init();  // ready after the loop's first barrier
@@ -378,8 +306,8 @@ __global__ void __launch_bounds__(NT, 4 * FWD_THREADS / NT) raster_fwd_batch_ker
         __syncthreads();
         const int it = s_item, lt = s_lt;
         if (it >= total_items) break;
-        raster_fwd_tile<FB, false, false, false, NT, LINES>(s_args, it / SUB, lt % s_args.tiles_x,
-                                                            lt / s_args.tiles_x, s, nullptr, 0, 0, it % SUB);
+        raster_fwd_tile<FB, false, false, false, NT>(s_args, it / SUB, lt % s_args.tiles_x, lt / s_args.tiles_x, s,
+                                                     nullptr, 0, 0, it % SUB);
     }
 }
 
@@ -395,14 +323,11 @@ int resident_grid(K kernel, size_t smem, int threads = TILE_PIX) {
 
 template <int FB, int NT>
 void fwd_batch_launch(const BatchDesc &d, int tiles_hint, int *d_counter, cudaStream_t st) {
-    constexpr size_t smem = sizeof(FwdStage<FB, can_lines<FB, NT>>);
-    static const int grid = [] {  // once per variant and shape, thread-safe
-        cudaFuncSetAttribute(raster_fwd_batch_kernel<FB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return resident_grid(raster_fwd_batch_kernel<FB, NT>, smem, NT);
-    }();
+    // once per variant and shape, thread-safe
+    static const int grid = resident_grid(raster_fwd_batch_kernel<FB, NT>, 0, NT);
     const int items = tiles_hint * (FWD_THREADS / NT);
     const int g = tiles_hint > 0 ? std::min(grid, items) : grid;
-    raster_fwd_batch_kernel<FB, NT><<<g, NT, smem, st>>>(d, d_counter);
+    raster_fwd_batch_kernel<FB, NT><<<g, NT, 0, st>>>(d, d_counter);
 }
 
 template <int NT>
@@ -796,33 +721,19 @@ __global__ void __launch_bounds__(BWD_THREADS, 5) raster_bwd_batch_kernel(const 
     }
 }
 
-template <int FB, bool AUX, bool TS, int NT, bool LINES = false>
+template <int FB, bool AUX, bool TS, int NT>
 void fwd_launch(const RasterArgs &a, int T, cudaStream_t st) {
-    constexpr size_t smem = sizeof(FwdStage<FB, LINES>);
-    static const bool attr = [] {  // once per instance, thread-safe
-        cudaFuncSetAttribute(raster_fwd_kernel<FB, AUX, TS, NT, LINES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-        return true;
-    }();
-    (void)attr;
-    raster_fwd_kernel<FB, AUX, TS, NT, LINES><<<T * (FWD_THREADS / NT), NT, smem, st>>>(a);
+    raster_fwd_kernel<FB, AUX, TS, NT><<<T * (FWD_THREADS / NT), NT, 0, st>>>(a);
 }
 
-// Shape 0 is whole tiles where the blocks take the sigma terms by column and row, halves
-// elsewhere: a half retires with its own pixels, and twice the blocks fill a small frame
-// better. 10 k to 300 k Gaussians at 256 x 256: 39 -> 36, 87 -> 82 and 238 -> 191 us, 100 k at
-// 400 x 320 93 -> 75, a 1 M-Gaussian 1080p frame 1073 -> 1054 us in all; 480 x 300 of the
-// street 88 -> 89, 800 x 600 of long lists the same.
+// Shape 0 of a single view is halves: a half retires with its own pixels, and twice the
+// blocks fill a small frame better. 10 k to 300 k Gaussians at 256 x 256: 39 -> 36, 87 -> 82
+// and 238 -> 191 us, 100 k at 400 x 320 93 -> 75, a 1 M-Gaussian 1080p frame 1073 -> 1054 us
+// in all; 480 x 300 of the street 88 -> 89, 800 x 600 of long lists the same.
 template <int FB, bool AUX, bool TS>
 void fwd_launch_shape(const RasterArgs &a, int T, cudaStream_t st, int shape) {
-    switch (shape_index(shape)) {
-        case 1: fwd_launch<FB, AUX, TS, FWD_THREADS / 2>(a, T, st); break;
-        case 2: fwd_launch<FB, AUX, TS, FWD_THREADS / 4>(a, T, st); break;
-        default:
-            if (fwd_lines(T, a.n_isect)) fwd_launch<FB, AUX, TS, FWD_THREADS, can_lines<FB, FWD_THREADS>>(a, T, st);
-            else fwd_launch<FB, AUX, TS, FWD_THREADS / 2>(a, T, st);
-            break;
-    }
+    if (shape_index(shape) == 2) fwd_launch<FB, AUX, TS, FWD_THREADS / 4>(a, T, st);
+    else fwd_launch<FB, AUX, TS, FWD_THREADS / 2>(a, T, st);
 }
 
 // The aux forward runs the default staging only (the reference too forces one
@@ -1027,15 +938,13 @@ __device__ __forceinline__ int chunk_tile(const int32_t *first, int T, int i) {
 
 template <int FB>
 __global__ void __launch_bounds__(FWD_THREADS, 4) raster_fwd_chunk_kernel(RasterArgs a, ChunkArgs c) {
-    extern __shared__ __align__(16) unsigned char fwd_smem[];
-    constexpr bool LINES = can_lines<FB, FWD_THREADS>;
-    FwdStage<FB, LINES> &s = *reinterpret_cast<FwdStage<FB, LINES> *>(fwd_smem);
+    __shared__ FwdStage<FB> s;
     const int T = a.tiles_x * a.tiles_y, item = blockIdx.x;
     if (item >= c.first[T]) return;  // block-uniform
     const int tile = chunk_tile(c.first, T, item);
     s.init();  // ready after the tile's first barrier
-    raster_fwd_tile<FB, false, true, false, FWD_THREADS, LINES>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s, &c,
-                                                                item, item - c.first[tile]);
+    raster_fwd_tile<FB, false, true, false, FWD_THREADS>(a, tile, tile % a.tiles_x, tile / a.tiles_x, s, &c, item,
+                                                         item - c.first[tile]);
 }
 
 // rasterize_forward_merge_kernel (.metal:2741-2808): per pixel, the tile's pieces front
@@ -1076,13 +985,7 @@ __global__ void __launch_bounds__(TILE_PIX) chunk_merge_kernel(RasterArgs a, Chu
 
 template <int FB>
 void fwd_chunk_launch(const RasterArgs &a, const ChunkArgs &c, int64_t items, cudaStream_t st) {
-    constexpr size_t smem = sizeof(FwdStage<FB, can_lines<FB, FWD_THREADS>>);
-    static const bool attr = [] {
-        cudaFuncSetAttribute(raster_fwd_chunk_kernel<FB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return true;
-    }();
-    (void)attr;
-    raster_fwd_chunk_kernel<FB><<<(unsigned)items, FWD_THREADS, smem, st>>>(a, c);
+    raster_fwd_chunk_kernel<FB><<<(unsigned)items, FWD_THREADS, 0, st>>>(a, c);
 }
 
 void launch_raster_fwd_chunked(const RasterArgs &a, const ChunkArgs &c, int64_t item_cap, cudaStream_t st,
