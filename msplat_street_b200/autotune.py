@@ -1,4 +1,4 @@
-"""Autotuner for the rasterizer's staging sizes and the batched forward's block shape.
+"""Autotuner for the rasterizer's staging sizes and the forward's block shape.
 
 The forward and backward rasterizers stage each tile's depth-sorted Gaussians in
 shared memory in rounds; the backward also reduces its per-pixel gradients in
@@ -10,7 +10,7 @@ every variant computes the same images and gradients, so the tuner only times th
 it runs the caller's step on each variant, interleaved over several rounds to share
 out drift (training changes the scene as it goes), and keeps the fastest.
 
-The batched forward also has a block shape (msplat_cuda_raster_shape): a block
+The forward also has a block shape (msplat_cuda_raster_shape): a block
 composites a whole 16 x 16 tile, a 16 x 8 half or an 8 x 8 quarter of it, the last
 being the reference Metal rasterizer's thread group inside its 16 x 16 bins
 (core/metal/msplat_metal.mm:1187-1197). Every shape walks the tile's whole list, so
@@ -43,7 +43,7 @@ def raster_variants() -> List[dict]:
 
 
 def raster_shapes() -> List[dict]:
-    """The batched forward's block shapes: pixels a block composites."""
+    """The forward's block shapes: pixels a block composites."""
     w, h = C.c_int32(), C.c_int32()
     n = lib().msplat_cuda_raster_shape(0, C.byref(w), C.byref(h))
     out = []

@@ -408,8 +408,9 @@ class Context:
         self.raster_variant = int(v)
 
     def set_raster_shape(self, s: int) -> None:
-        """Block shape of the batched forward rasterizer (see autotune.raster_shapes());
-        results do not depend on it."""
+        """Block shape of the forward rasterizers (see autotune.raster_shapes()); results do
+        not depend on it. Never set, single views composite in 16 x 8 blocks and batches
+        in 16 x 16."""
         check(self._lib.msplat_cuda_ctx_set_option(self.handle, b"raster_shape", int(s)))
         self.raster_shape = int(s)
 

@@ -176,7 +176,7 @@ constexpr int CHUNK_AUTO_TILES = 400;  // core/metal/msplat_metal.mm:1103
 struct msplat_cuda_ctx {
     cudaStream_t stream = nullptr;
     int raster_variant = 0;  // option "raster_variant": index into RASTER_VARIANTS
-    int raster_shape = 0;    // option "raster_shape": index into RASTER_SHAPES (forward rasterizers)
+    int raster_shape = -1;   // option "raster_shape": index into RASTER_SHAPES (forward rasterizers); -1: never set
     TrainBatchState tb;
     bool keep_grads = false;
     StageTimer timer;

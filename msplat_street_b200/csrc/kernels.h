@@ -80,17 +80,20 @@ constexpr RasterVariant RASTER_VARIANTS[N_RASTER_VARIANTS] = {
     {128, 128, 3}, {128, 64, 3}, {128, 64, 4}, {256, 128, 3}, {64, 128, 3}, {256, 64, 4}, {128, 32, 4}, {256, 128, 4}};
 inline int variant_index(int v) { return (v >= 0 && v < N_RASTER_VARIANTS) ? v : 0; }
 
-// Block shapes of the batched forward rasterizer (pixels a block composites; every
-// shape walks the 16 x 16 tile's list, so all give the same bits): 16 x 16 (the
-// default; a single view's launch may halve it), 16 x 8 and 8 x 8 (the reference's Metal thread-group shape).
+// Block shapes of the forward rasterizers (pixels a block composites; every shape walks
+// the 16 x 16 tile's list, so all give the same bits): 16 x 16 (the default of the
+// batched one), 16 x 8 (of a single view's) and 8 x 8 (the reference's Metal thread-group
+// shape).
 struct RasterShape {
     int w, h;
 };
 constexpr int N_RASTER_SHAPES = 3;
 constexpr RasterShape RASTER_SHAPES[N_RASTER_SHAPES] = {{16, 16}, {16, 8}, {8, 8}};
-inline int shape_index(int s) { return (s >= 0 && s < N_RASTER_SHAPES) ? s : 0; }
+constexpr int SINGLE_SHAPE = 1, BATCH_SHAPE = 0;  // the defaults
+inline int shape_index(int s, int fallback) { return (s >= 0 && s < N_RASTER_SHAPES) ? s : fallback; }
 
-void launch_raster_fwd(const RasterArgs &a, cudaStream_t st, int variant = 0, int shape = 0);
+// shape: an index into RASTER_SHAPES, or -1 for the default (here and below)
+void launch_raster_fwd(const RasterArgs &a, cudaStream_t st, int variant = 0, int shape = -1);
 // (pixel, Gaussian) pairs the reference's forward / backward loops evaluate over the
 // frame (out[0], out[1]; device counters, zeroed first unless accumulate)
 void launch_pair_counts(const RasterArgs &a, unsigned long long *d_out, cudaStream_t st, bool accumulate = false);
@@ -98,7 +101,7 @@ void launch_pair_counts(const RasterArgs &a, unsigned long long *d_out, cudaStre
 void launch_exp_tab(const float *x, int64_t n, float *out, cudaStream_t st);
 // the projection's (exp_wide)
 void launch_exp_wide(const float *x, int64_t n, float *out, cudaStream_t st);
-void launch_raster_fwd_aux(const RasterArgs &a, cudaStream_t st, int shape = 0);
+void launch_raster_fwd_aux(const RasterArgs &a, cudaStream_t st, int shape = -1);
 
 struct RasterBwdArgs;
 // Depth-chunked compositing (core/metal/msplat_metal.metal:2641-3030): every tile's
@@ -193,7 +196,7 @@ void launch_bin_emit(const BinArgs &a, int32_t *gids, int32_t *inv, int64_t cap,
 void launch_bin_clamp(const BinArgs &a, int64_t cap, int *d_n, int *overflow, cudaStream_t st);
 
 void launch_raster_fwd_batch(const BatchDesc &d, int tiles_hint, int *d_counter, cudaStream_t st, int variant = 0,
-                             int shape = 0);
+                             int shape = -1);
 
 struct RasterBwdArgs {
     int W, H, tiles_x, tiles_y;

@@ -344,7 +344,7 @@ void fwd_batch_staging(const BatchDesc &d, int tiles_hint, int *d_counter, cudaS
 void launch_raster_fwd_batch(const BatchDesc &d, int tiles_hint, int *d_counter, cudaStream_t st, int variant,
                              int shape) {
     cudaMemsetAsync(d_counter, 0, sizeof(int), st);
-    switch (shape_index(shape)) {
+    switch (shape_index(shape, BATCH_SHAPE)) {
         case 1: fwd_batch_staging<FWD_THREADS / 2>(d, tiles_hint, d_counter, st, variant); break;
         case 2: fwd_batch_staging<FWD_THREADS / 4>(d, tiles_hint, d_counter, st, variant); break;
         default: fwd_batch_staging<FWD_THREADS>(d, tiles_hint, d_counter, st, variant); break;
@@ -726,14 +726,19 @@ void fwd_launch(const RasterArgs &a, int T, cudaStream_t st) {
     raster_fwd_kernel<FB, AUX, TS, NT><<<T * (FWD_THREADS / NT), NT, 0, st>>>(a);
 }
 
-// Shape 0 of a single view is halves: a half retires with its own pixels, and twice the
-// blocks fill a small frame better. 10 k to 300 k Gaussians at 256 x 256: 39 -> 36, 87 -> 82
-// and 238 -> 191 us, 100 k at 400 x 320 93 -> 75, a 1 M-Gaussian 1080p frame 1073 -> 1054 us
-// in all; 480 x 300 of the street 88 -> 89, 800 x 600 of long lists the same.
+// By default a single view composites in halves: a half retires with its own pixels, and
+// twice the blocks fill a small frame better. The forward against whole tiles: 43 -> 41,
+// 128 -> 99 and 243 -> 195 us for 10 k, 100 k and 300 k Gaussians at 256 x 256, 87 -> 75 for
+// 50 k at 464 x 320, 143 -> 138 and 486 -> 430 for 300 k and 3 M at 1024 x 768, 338 -> 322
+// for 1 M at 1920 x 1080; street views 0.5 us either way at 1024 x 512, 353 -> 357 at
+// 1600 x 1060.
 template <int FB, bool AUX, bool TS>
 void fwd_launch_shape(const RasterArgs &a, int T, cudaStream_t st, int shape) {
-    if (shape_index(shape) == 2) fwd_launch<FB, AUX, TS, FWD_THREADS / 4>(a, T, st);
-    else fwd_launch<FB, AUX, TS, FWD_THREADS / 2>(a, T, st);
+    switch (shape_index(shape, SINGLE_SHAPE)) {
+        case 1: fwd_launch<FB, AUX, TS, FWD_THREADS / 2>(a, T, st); break;
+        case 2: fwd_launch<FB, AUX, TS, FWD_THREADS / 4>(a, T, st); break;
+        default: fwd_launch<FB, AUX, TS, FWD_THREADS>(a, T, st); break;
+    }
 }
 
 // The aux forward runs the default staging only (the reference too forces one

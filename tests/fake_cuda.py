@@ -79,6 +79,14 @@ class FakeCuda:
     def render_backward(self, ctx, n, w, h, degree=0):
         return self.lib.msplat_cuda_render_backward(ctx, *self._view(n, w, h, degree), _BG.ctypes.data, *[64] * 7)
 
+    def render_batch(self, ctx, views, n, w, h):
+        vs = (_lib.View * views)()
+        for v in vs:
+            v.num_points, v.img_width, v.img_height = n, w, h
+            v.means3d = v.scales = v.quats = v.features_dc = v.opacities = v.out_img = 64
+            v.glob_scale = v.fx = v.fy = 1.0
+        return self.lib.msplat_cuda_render_batch(ctx, views, vs)
+
     def pair_counts(self, ctx):
         out = (C.c_int64 * 2)()
         return self.lib.msplat_cuda_frame_pair_counts(ctx, out)

@@ -1,5 +1,6 @@
 """What the C-ABI launches and leaves behind, on a recorded CUDA runtime (fake_cuda.py;
-no GPU): a call that fails leaves no frame that a later call would walk."""
+no GPU): a call that fails leaves no frame that a later call would walk, and the options
+that results do not show choose the launches they say."""
 import pytest
 
 import fake_cuda
@@ -70,3 +71,21 @@ def _refused(cuda):
 
 def test_refused_render_keeps_the_frame():
     assert fake_cuda.run(_refused) == (1, 0)
+
+
+def _forward_blocks(cuda, shape):
+    """(blocks, threads) of the single-view forward, and the batched one's threads."""
+    ctx = cuda.context()
+    if shape is not None:
+        assert cuda.lib.msplat_cuda_ctx_set_option(ctx, b"raster_shape", shape) == 0
+    cuda.readback(5000)
+    assert cuda.render(ctx, N, W, H) == 0 and cuda.render_batch(ctx, 2, N, W, H) == 0
+    fwd = [k for k in cuda.launches() if "raster_fwd" in k[0]]
+    assert len(fwd) == 2 and "batch" in fwd[1][0]
+    return fwd[0][1], fwd[0][3], fwd[1][3]
+
+
+@pytest.mark.parametrize("shape,blocks", [(None, (2400, 128, 256)), (0, (1200, 256, 256)), (1, (2400, 128, 128)),
+                                          (2, (4800, 64, 64))])
+def test_raster_shape_chooses_the_blocks(shape, blocks):
+    assert fake_cuda.run(_forward_blocks, shape) == blocks
