@@ -1095,7 +1095,7 @@ int msplat_cuda_densify(msplat_cuda_ctx *ctx, int N, int buf_capacity, float gra
     a.log_size_fac = std::log(1.6f);  // the host's logf, as the reference computes it (msplat_cpu.cpp:1348)
     a.seed = seed;
     const int strides[6] = {3, 3, 4, 3, fr_stride, 1};
-    int max_stride = 3 * (3 + 3 + 4 + 3 + 1);  // the narrow groups' rows, three buffers each, side by side
+    int max_stride = 1;
     for (int g = 0; g < 6; g++) {
         a.stride[g] = strides[g];
         max_stride = std::max(max_stride, strides[g]);
@@ -1112,7 +1112,8 @@ int msplat_cuda_densify(msplat_cuda_ctx *ctx, int N, int buf_capacity, float gra
     if (rows > (int64_t)INT32_MAX) return fail(MSPLAT_CUDA_EINVAL, "msplat_densify: N (%d) too large", N);
     ENSURE(ctx->d_flags, 7 * rows, int32_t, flags);
     ENSURE(ctx->d_counts, 8 + scan_blocks((int)rows) + 1, int32_t, counts);
-    ENSURE(ctx->d_scratch, rows * max_stride + 64, float, scratch);  // 64: each buffer starts on 16 bytes
+    const int64_t scratch_floats = densify_scratch_floats(rows, max_stride);
+    ENSURE(ctx->d_scratch, scratch_floats, float, scratch);
     if (!ctx->h_count) CUDA_TRY(cudaMallocHost(&ctx->h_count, sizeof(int32_t)));
     DensifyScratch s;
     s.split = flags;
@@ -1129,6 +1130,7 @@ int msplat_cuda_densify(msplat_cuda_ctx *ctx, int N, int buf_capacity, float gra
     s.overflow = counts + 4;
     s.scan_part = counts + 8;
     s.scratch = scratch;
+    s.scratch_floats = scratch_floats;
     launch_densify(a, s, st);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(ctx->h_count, s.new_count, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

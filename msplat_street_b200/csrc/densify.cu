@@ -260,6 +260,21 @@ __global__ void opacity_reset_kernel(float *o, float *m1, float *m2, int n, floa
     m2[i] = 0.f;
 }
 
+// A buffer's place in the scratch: each starts on 16 bytes.
+static int64_t align4(int64_t floats) { return (floats + 3) / 4 * 4; }
+
+// Room for the widest buffer's rows, as compacting one buffer at a time needs, and for
+// all 15 narrow ones at once (a launch pair instead of 15) where those take no more than
+// NARROW_FLOATS: at SH degree 3 the two are the same size, at degree 0 ten times apart,
+// and a large model's buffers are long enough to be compacted a few at a time. 2 M
+// Gaussians at degree 0: 874 us with 512 MB, 831 with the 1.3 GB of all at once, 943 with
+// 256 MB.
+constexpr int64_t NARROW_FLOATS = 1 << 27;  // 512 MB
+int64_t densify_scratch_floats(int64_t rows, int max_stride) {
+    const int64_t narrow = 3 * (3 * align4(3 * rows) + align4(4 * rows) + align4(rows));
+    return std::max(align4(rows * max_stride), std::min(narrow, NARROW_FLOATS));
+}
+
 void launch_densify(const DensifyArgs &a, DensifyScratch &s, cudaStream_t st) {
     const int n = a.n;
     if (n <= 0) {
@@ -280,7 +295,8 @@ void launch_densify(const DensifyArgs &a, DensifyScratch &s, cudaStream_t st) {
     densify_cull_kernel<<<(unsigned)((rows + bs - 1) / bs), bs, 0, st>>>(a, s.split, s.n_split, s.n_dup, s.keep,
                                                                        s.n_new);
     scan_exclusive<int32_t>(s.keep, s.keep_ord, (int)rows, s.new_count, s.scan_part, st);
-    // the narrow groups' 15 buffers side by side in the scratch, then each SH-rest buffer
+    // the narrow groups' 15 buffers side by side in the scratch, as many at a time as it
+    // holds, then each SH-rest buffer
     CompactArgs c;
     int k = 0;
     int64_t at = 0;
@@ -295,10 +311,12 @@ void launch_densify(const DensifyArgs &a, DensifyScratch &s, cudaStream_t st) {
     };
     auto add = [&](float *buf, int stride) {
         if (stride <= 0) return;  // e.g. no SH rest at degree 0
+        const int64_t size = align4(rows * stride);
+        if (at + size > s.scratch_floats) flush();
         c.buf[k] = buf;
         c.at[k] = at;
         c.stride[k++] = stride;
-        at += (rows * stride + 3) / 4 * 4;
+        at += size;
     };
     for (int g = 0; g < 6; g++) {
         if (g == 4) continue;

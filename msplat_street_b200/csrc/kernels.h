@@ -299,8 +299,10 @@ struct DensifyScratch {
     int32_t *n_split, *n_dup, *n_new, *new_count, *scan_part;
     int32_t *overflow;  // set when N + 2 splits + clones exceeds cap (nothing is written)
     int32_t *row_parent;  // 3N: the parent of each new row (split children, then clones)
-    float *scratch;     // 4N x max(3 x 14, SH-rest stride) + 64 floats
+    float *scratch;     // densify_scratch_floats(4N, widest stride)
+    int64_t scratch_floats;
 };
+int64_t densify_scratch_floats(int64_t rows, int max_stride);
 void launch_densify(const DensifyArgs &a, DensifyScratch &s, cudaStream_t st);
 void launch_opacity_reset(float *o, float *m1, float *m2, int n, float reset_logit, cudaStream_t st);
 

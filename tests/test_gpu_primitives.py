@@ -180,6 +180,27 @@ def test_gpu_densify_row_blocks(n, rest, shift):
         assert np.array_equal(t2[g].cpu().numpy()[:new_o], o2[g][:new_o]), g
 
 
+def test_gpu_densify_narrow_buffers_in_parts():
+    """A model of SH degree 0 whose narrow buffers do not fit the scratch side by side."""
+    n = 810_000
+    cap = 3 * n
+    rng = np.random.default_rng(8)
+    g = scenes.random_gaussians(n, 8, sh_degree=0, log_scale_mean=-4.0, log_scale_std=1.5)
+    strides = [3, 3, 4, 3, 0, 1]
+    bufs = [np.pad(a.reshape(n, s), ((0, cap - n), (0, 0))).astype(np.float32) for a, s in zip(g.arrays(), strides)]
+    m1, m2 = ([rng.random((cap, s), dtype=np.float32) for s in strides] for _ in range(2))
+    stats = {"vis": rng.integers(0, 4, n).astype(np.float32), "gn": (rng.random(n) * 2e-3).astype(np.float32),
+             "ms": (rng.random(n) * 0.3).astype(np.float32)}
+    tb, t1, t2 = ([torch.from_numpy(b).cuda() for b in arrays] for arrays in (bufs, m1, m2))
+    st = [torch.from_numpy(stats[k]).cuda() for k in ("gn", "vis", "ms")]
+    new_o = Oracle("restatement").densify(n, cap, bufs, m1, m2, stats, 60.0, 31)
+    assert Context().densify(n, tb, t1, t2, st[0], st[1], st[2], 60.0, 31) == new_o
+    for g in range(6):  # tolerance as above
+        np.testing.assert_allclose(tb[g].cpu().numpy()[:new_o], bufs[g][:new_o], rtol=1e-6, atol=1e-7, err_msg=str(g))
+        assert np.array_equal(t1[g].cpu().numpy()[:new_o], m1[g][:new_o]), g
+        assert np.array_equal(t2[g].cpu().numpy()[:new_o], m2[g][:new_o]), g
+
+
 def _split_and_clone_inputs(n, cap, seed):
     """Small Gaussians (world scale below size_thresh) that are large on screen and
     have high gradients: each one is both split and cloned, 4 n rows in all."""

@@ -1,6 +1,8 @@
 """What the C-ABI launches and leaves behind, on a recorded CUDA runtime (fake_cuda.py;
 no GPU): a call that fails leaves no frame that a later call would walk, and the options
 that results do not show choose the launches they say."""
+import ctypes as C
+
 import pytest
 
 import fake_cuda
@@ -89,3 +91,29 @@ def _forward_blocks(cuda, shape):
                                           (2, (4800, 64, 64))])
 def test_raster_shape_chooses_the_blocks(shape, blocks):
     assert fake_cuda.run(_forward_blocks, shape) == blocks
+
+
+def _densify(cuda, n, rest):
+    """Device bytes a densification holds, and its compaction launches."""
+    ctx = cuda.context()
+    six = (C.c_void_p * 6)(*[64] * 6)
+    count = C.c_int()
+    assert cuda.lib.msplat_cuda_densify(ctx, n, 4 * n, 2e-4, 0.01, 0.05, 0, 0.1, 0.5, 0.15, 0, 64, 64, 64, 256.0, six,
+                                        rest, six, six, 1, C.byref(count)) == 0
+    gathers = sum("compact_gather" in k[0] for k in cuda.launches())
+    return cuda.lib.msplat_cuda_ctx_device_bytes(ctx), gathers
+
+
+# per row of 4 n: seven flags, and the widest buffer's floats; a quarter more for growth
+@pytest.mark.parametrize("n,rest,widest", [(10_000_000, 0, 4), (10_000_000, 9, 9), (4_000_000, 24, 24),
+                                           (4_000_000, 45, 45), (1_000_000, 72, 72)])
+def test_densify_scratch_is_the_widest_buffer(n, rest, widest):
+    held, _ = fake_cuda.run(_densify, n, rest)
+    assert held <= 1.26 * 4 * n * 4 * (7 + widest)
+
+
+@pytest.mark.parametrize("n,rest,gathers", [(100_000, 0, 1), (100_000, 45, 4), (400_000, 45, 4)])
+def test_densify_compacts_narrow_buffers_together(n, rest, gathers):
+    held, launched = fake_cuda.run(_densify, n, rest)
+    assert launched == gathers
+    assert held <= 1.26 * (4 * n * 4 * (7 + rest) + (1 << 28))
