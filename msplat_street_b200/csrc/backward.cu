@@ -493,15 +493,51 @@ __device__ __forceinline__ int active_bases(uint32_t dtu) { return dtu < 1 ? 0 :
 // us).
 constexpr int NB = 128;
 
+// The gradient arrays of one Gaussian (those that are asked for).
+__device__ __forceinline__ void write_grads(const BackwardArgs &a, size_t i, const float s9[9], float depth,
+                                            const float gm[3], const float gsv[3], const float gq[4]) {
+    if (a.v_xy) {
+        a.v_xy[2 * i] = s9[0];
+        a.v_xy[2 * i + 1] = s9[1];
+    }
+    if (a.v_conic)
+        for (int c = 0; c < 3; c++) a.v_conic[3 * i + c] = s9[2 + c];
+    if (a.v_rgb)
+        for (int c = 0; c < 3; c++) a.v_rgb[3 * i + c] = s9[5 + c];
+    if (a.v_opacity) a.v_opacity[i] = s9[8];
+    if (a.v_depth) a.v_depth[i] = depth;
+    if (a.v_mean3d) {
+        for (int c = 0; c < 3; c++) {
+            a.v_mean3d[3 * i + c] = gm[c];
+            a.v_scale[3 * i + c] = gsv[c];
+        }
+        for (int c = 0; c < 4; c++) a.v_quat[4 * i + c] = gq[c];
+    }
+    if (a.g_dc)
+        for (int c = 0; c < 3; c++) a.g_dc[3 * i + c] = SH_C0 * s9[5 + c];
+}
+
+// The gradients on their way to the Adam steps.
+template <int NB>
+struct AdamGrads {
+    float mean[NB * 3], scale[NB * 3], quat[NB * 4], op[NB], dc[NB * 3];
+};
+
 // Bound by the latency of its chain of phases (radii; slot positions; slots; parameters;
 // three rounds of Adam loads) and, where most Gaussians are visible and SH degree 3 is in
 // use, by issue (Adam's exact square root and divisions). Against one thread a Gaussian
 // with its slots, VJPs and Adam in one lane (whose order of additions the slot sums
 // keep): a 1 M-Gaussian street step at 1600 x 1060 545 -> 345 us, an early 100 k street
-// view 100 -> 76 us, 200 k gradients with everything visible 65 -> 69 us.
+// view 100 -> 76 us.
+//
+// ADAM: the update step; else gradients (and statistics) only, which go to their arrays
+// from the thread that computed them: 63 us for 200 k Gaussians, all visible, and 176 for
+// 600 k, where passing them through shared memory as the update does took 70 and 201 and
+// one thread a Gaussian 66 and 185.
+template <bool ADAM>
 __global__ void __launch_bounds__(NB, 1024 / NB) backward_adam_kernel(BackwardArgs a) {
     __shared__ VisibleList<NB> L;
-    __shared__ float s_mean[NB * 3], s_scale[NB * 3], s_quat[NB * 4], s_op[NB], s_dc[NB * 3];
+    __shared__ AdamGrads<ADAM ? NB : 1> s;
     __shared__ float s_basis[NB][MAX_REST + 2];
     __shared__ uint8_t s_vis[NB];
     const int t = threadIdx.x;
@@ -509,17 +545,22 @@ __global__ void __launch_bounds__(NB, 1024 / NB) backward_adam_kernel(BackwardAr
     const int rows = (int)min((int64_t)NB, (int64_t)a.n - g0);
     const int active = active_bases(a.cam.degrees_to_use);
 
-    // 1. the visible Gaussians and their slot sums
+    // 1. the visible Gaussians and their slot sums; the others' gradients are zero
     const bool vis = list_instances<NB>(L, g0, rows, a.radii, a.offsets, a.n_tiles);
     if (!vis) {
+        if constexpr (ADAM) {
 #pragma unroll
-        for (int c = 0; c < 9; c++) L.s9[t * 9 + c] = 0.f;
-        L.depth[t] = 0.f;
+            for (int c = 0; c < 9; c++) L.s9[t * 9 + c] = 0.f;
+            L.depth[t] = 0.f;
 #pragma unroll
-        for (int c = 0; c < 3; c++) s_mean[t * 3 + c] = s_scale[t * 3 + c] = s_dc[t * 3 + c] = 0.f;
+            for (int c = 0; c < 3; c++) s.mean[t * 3 + c] = s.scale[t * 3 + c] = s.dc[t * 3 + c] = 0.f;
 #pragma unroll
-        for (int c = 0; c < 4; c++) s_quat[t * 4 + c] = 0.f;
-        s_op[t] = 0.f;
+            for (int c = 0; c < 4; c++) s.quat[t * 4 + c] = 0.f;
+            s.op[t] = 0.f;
+        } else if (t < rows) {
+            const float zero[9] = {};
+            write_grads(a, (size_t)g0 + t, zero, 0.f, zero, zero, zero);
+        }
     }
     s_vis[t] = vis;
     sum_slots<NB>(L, a.inv, a.slots, a.slots_depth);
@@ -531,18 +572,22 @@ __global__ void __launch_bounds__(NB, 1024 / NB) backward_adam_kernel(BackwardAr
         float s9[9], gm[3], gsv[3], gq[4];
 #pragma unroll
         for (int c = 0; c < 9; c++) s9[c] = L.s9[li * 9 + c];
+        const float depth = a.slots_depth ? L.depth[li] : 0.f;
         V3 dir;
-        projection_vjp(a.cam, a.means, a.scales, a.quats, a.glob_scale, a.splats + i, i, s9, gm, gsv, gq, dir,
-                       a.slots_depth ? L.depth[li] : 0.f);
+        projection_vjp(a.cam, a.means, a.scales, a.quats, a.glob_scale, a.splats + i, i, s9, gm, gsv, gq, dir, depth);
+        if constexpr (!ADAM) {
+            write_grads(a, (size_t)i, s9, depth, gm, gsv, gq);
+        } else {
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            s_mean[li * 3 + c] = gm[c];
-            s_scale[li * 3 + c] = gsv[c];
-            s_dc[li * 3 + c] = SH_C0 * s9[5 + c];
+            for (int c = 0; c < 3; c++) {
+                s.mean[li * 3 + c] = gm[c];
+                s.scale[li * 3 + c] = gsv[c];
+                s.dc[li * 3 + c] = SH_C0 * s9[5 + c];
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) s.quat[li * 4 + c] = gq[c];
+            s.op[li] = s9[8];
         }
-#pragma unroll
-        for (int c = 0; c < 4; c++) s_quat[li * 4 + c] = gq[c];
-        s_op[li] = s9[8];
         if (active > 0) sh_rest_basis(dir, s_basis[li]);
         if (a.vis_counts) {
             a.vis_counts[i] += 1.0f;
@@ -552,35 +597,20 @@ __global__ void __launch_bounds__(NB, 1024 / NB) backward_adam_kernel(BackwardAr
     }
     __syncthreads();
 
-    // 3. gradient outputs (zero for invisible Gaussians)
-    if (t < rows) {
-        const size_t i = (size_t)g0 + t;
-        const float *s9 = L.s9 + t * 9;
-        if (a.v_xy) {
-            a.v_xy[2 * i] = s9[0];
-            a.v_xy[2 * i + 1] = s9[1];
-        }
-        if (a.v_conic)
-            for (int c = 0; c < 3; c++) a.v_conic[3 * i + c] = s9[2 + c];
-        if (a.v_rgb)
-            for (int c = 0; c < 3; c++) a.v_rgb[3 * i + c] = s9[5 + c];
-        if (a.v_opacity) a.v_opacity[i] = s9[8];
-        if (a.v_depth) a.v_depth[i] = L.depth[t];
-        if (a.v_mean3d) {
-            for (int c = 0; c < 3; c++) {
-                a.v_mean3d[3 * i + c] = s_mean[t * 3 + c];
-                a.v_scale[3 * i + c] = s_scale[t * 3 + c];
-            }
-            for (int c = 0; c < 4; c++) a.v_quat[4 * i + c] = s_quat[t * 4 + c];
-        }
-        if (a.g_dc)
-            for (int c = 0; c < 3; c++) a.g_dc[3 * i + c] = s_dc[t * 3 + c];
-    }
-
-    // 4. Adam: means, scales, quats, opacity of all N; DC and the SH rest of the visible
     const float b1 = a.beta1, b2 = a.beta2, eps = a.eps;
-    if (a.do_adam) {
-        adam_groups<NB>(a.p, a.m1, a.m2, g0, rows, s_mean, s_scale, s_quat, s_op, s_dc, s_vis, a.ss, a.bc2, b1, b2,
+    const int stride = a.rest_stride, used = 3 * active;
+    auto grad = [&](int i, int base, int c, int) { return s_basis[i][base] * L.s9[i * 9 + 5 + c]; };
+    const size_t off = (size_t)g0 * (size_t)max(stride, 0);
+    if constexpr (!ADAM) {  // 3. the SH rest's gradient rows
+        if (stride > 0 && a.g_rest)
+            write_rest<NB>(a.g_rest + off, rows, stride, used,
+                           [&](int i, int base, int c, int e) { return s_vis[i] ? grad(i, base, c, e) : 0.f; });
+        return;
+    } else {
+        if (t < rows)
+            write_grads(a, (size_t)g0 + t, L.s9 + t * 9, L.depth[t], s.mean + t * 3, s.scale + t * 3, s.quat + t * 4);
+        // 3. Adam: means, scales, quats, opacity of all N; DC and the SH rest of the visible
+        adam_groups<NB>(a.p, a.m1, a.m2, g0, rows, s.mean, s.scale, s.quat, s.op, s.dc, s_vis, a.ss, a.bc2, b1, b2,
                         eps);
         // needle cap after the scale update (scale_ratio_cap, core/cpu/msplat_cpu.cpp:1295-1309)
         if (a.log_max_scale_ratio > 0.f) {  // grid-uniform
@@ -597,26 +627,17 @@ __global__ void __launch_bounds__(NB, 1024 / NB) backward_adam_kernel(BackwardAr
                 }
             }
         }
+        if (stride <= 0 || active == 0) return;
+        adam_rest<NB>(a.p[4] + off, a.m1[4] + off, a.m2[4] + off, L.count, stride, used,
+                      [&](int r) { return (int)L.idx[r]; }, grad, a.ss[4], b1, b2, a.bc2[4], eps);
     }
-
-    // 5. SH rest: its gradient rows, or Adam
-    const int stride = a.rest_stride, used = 3 * active;
-    if (stride <= 0) return;
-    auto grad = [&](int i, int base, int c, int) { return s_basis[i][base] * L.s9[i * 9 + 5 + c]; };
-    const size_t off = (size_t)g0 * stride;
-    if (a.g_rest) {
-        write_rest<NB>(a.g_rest + off, rows, stride, used,
-                       [&](int i, int base, int c, int e) { return s_vis[i] ? grad(i, base, c, e) : 0.f; });
-        return;
-    }
-    if (!a.do_adam || active == 0) return;
-    adam_rest<NB>(a.p[4] + off, a.m1[4] + off, a.m2[4] + off, L.count, stride, used,
-                  [&](int r) { return (int)L.idx[r]; }, grad, a.ss[4], b1, b2, a.bc2[4], eps);
 }
 
 void launch_backward_adam(const BackwardArgs &a, cudaStream_t st) {
     if (a.n <= 0) return;
-    backward_adam_kernel<<<(a.n + NB - 1) / NB, NB, 0, st>>>(a);
+    const int blocks = (a.n + NB - 1) / NB;
+    if (a.do_adam) backward_adam_kernel<true><<<blocks, NB, 0, st>>>(a);
+    else backward_adam_kernel<false><<<blocks, NB, 0, st>>>(a);
 }
 
 // The multi-view form: a block walks the batch's views in order, lists the Gaussians each

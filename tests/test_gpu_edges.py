@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from msplat_street_b200 import scenes
+from msplat_street_b200 import autograd, scenes
 from msplat_street_b200.backend import AdamState, Context, GaussianParams
 from msplat_street_b200.camera import look_at, prepare_cam
 from oracle_lib import Oracle, new_adam_state
@@ -149,6 +149,34 @@ def test_slot_sums_of_every_size(n, scale, degree):
     ctx.train_batch(q, aq, [(cam, gt_t)], BACKGROUND, degrees_to_use=degree)
     for a, b in zip(p.tensors() + ap.exp_avg + ap.exp_avg_sq, q.tensors() + aq.exp_avg + aq.exp_avg_sq):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n,degree,unseen", [(1, 3, 0.0), (127, 0, 0.5), (128, 3, 0.0), (129, 2, 0.5), (1000, 3, 0.9),
+                                             (1000, 1, 0.0)])
+def test_gradients_with_and_without_the_update(n, degree, unseen):
+    """The backward that writes gradients and the one that also updates are two kernels:
+    the same gradients bit for bit, in blocks all visible, mixed and ragged."""
+    g = scenes.random_gaussians(n, n, sh_degree=degree, log_scale_mean=-2.5)
+    g.means[np.random.default_rng(n).random(n) < unseen, 2] += 10.0  # behind the camera
+    cam = scenes.small_camera(160, 120, 130.0)
+    gt = torch.rand((120, 160, 3), device="cuda")
+    frames, moments = [], None
+    for update in (True, False):
+        ctx, p = Context(keep_grads=True), GaussianParams.from_numpy(g)
+        adam = AdamState.zeros_like(p, C1_LRS)
+        stats = [torch.zeros(n, device="cuda") for _ in range(3)]
+        ctx.train_step(p, adam, cam, BACKGROUND, gt, stats, num_adam_groups=6 if update else 0)
+        frames.append([ctx.frame(k).clone() for k in GRAD_KEYS] + stats)
+        moments = adam.exp_avg if update else moments
+    for a, b in zip(*frames):
+        assert torch.equal(a, b)
+    seen = frames[0][-3] > 0
+    assert bool(seen.any()) and (unseen == 0 or not bool(seen.all()))
+    p = GaussianParams(*[torch.from_numpy(a).cuda().requires_grad_(True) for a in g.arrays()])
+    autograd.ssim_l1_loss(autograd.render(p, cam, BACKGROUND), gt).backward()
+    for t, m in zip(p.tensors(), moments):  # the first moments of one step from zero
+        if t.numel():
+            assert torch.allclose(t.grad.reshape(m.shape) * np.float32(1.0 - np.float32(0.9)), m, rtol=1e-6, atol=0)
 
 
 def _half_up(x):
