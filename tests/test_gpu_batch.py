@@ -151,3 +151,24 @@ def test_server_small_budget_lru():
     assert store.resident_bytes <= store.budget
     _check_alone(res, reqs, store)
     srv.close()
+
+
+@pytest.mark.parametrize("before,shift", [(701, 0), (702, 0), (703, 0), (32, 1), (33, 2), (1, 3)])
+def test_degree_3_rows_off_16_bytes(before, shift):
+    """A scene whose SH-rest rows a warp cannot copy 16 bytes at a time: the scene before it
+    in the batch has a count that is no multiple of four, or its tensor starts off 16
+    bytes. The images of the aligned scene alone, and the oracle's."""
+    g = scenes.random_gaussians(900, 6)
+    cam = scenes.small_camera(200, 136, 180.0)
+    first, aligned = _dev(scenes.random_gaussians(before, 7)), _dev(g)
+    flat = torch.zeros(aligned.features_rest.numel() + shift, device="cuda")
+    flat[shift:] = aligned.features_rest.reshape(-1)
+    moved = aligned.clone()
+    moved.features_rest = flat[shift:].view(aligned.features_rest.shape)
+    assert moved.features_rest.data_ptr() % 16 == 4 * shift
+    ctx = Context()
+    alone = ctx.render(aligned, cam, BACKGROUND).clone()
+    assert torch.equal(ctx.render(moved, cam, BACKGROUND), alone)
+    got = ctx.render_batch([BatchItem(first, scenes.small_camera(64, 48), BACKGROUND), BatchItem(moved, cam, BACKGROUND)])
+    assert torch.equal(got[1], alone)
+    assert np.abs(alone.cpu().numpy() - Oracle().render(g, cam, BACKGROUND)).max() <= 1e-5
