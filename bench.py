@@ -401,7 +401,7 @@ def run_ours(args, world, rank, local):
                        "gaussians_end": final_n, "isects_mean": float(np.mean(n_isects)),
                        "l2": "256 MB write between timed steps", "parallelism": f"replicas x{world}"},
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 4},
-            "gpu_launches": int(args.steps * launches_per_step(np.mean(n_isects), final_n)),
+            "gpu_launches": int(args.steps * launches_per_step(final_n)),
             "roofline": roof,
             "throughput": thr,
             "schedule_sample": sched,
@@ -746,7 +746,7 @@ class TargetPrefetch:
         return t
 
 
-def launches_per_step(n_isect: float, n_gauss: float = 1e5) -> float:
+def launches_per_step(n_gauss: float = 1e5) -> float:
     """Kernels one plain training step launches: project, the depth sort (one cluster
     launch up to 65,536 Gaussians, else 4 passes of hist + scatter, plus a 3-kernel scan
     per pass above 131,072), tile rectangles, the scan of their counts (3 kernels, one up

@@ -556,17 +556,18 @@ __global__ void bin_view_keys_kernel(int n, const uint32_t *order, const BatchDe
     if (r < n) keys[r] = (uint32_t)find_view(d.inst_off, d.n_views, (int)order[r]);
 }
 
-// Gaussians to a chunk's block: so many that there are four blocks for every place of an
-// SM and the last round of blocks is a small share, but 64 to 2048. The upper end keeps
-// the writes of the lists in L2: the blocks at work at a time (some 600) then fill one
+// Gaussians to a chunk on average, which sets the number of chunks (each then takes an
+// equal share of the intersections, however many Gaussians that is): so many chunks that
+// there are four blocks an SM, but 64 to 2048 Gaussians each. The upper end keeps the
+// writes of the lists in L2: the blocks at work at a time (some 600) then fill one
 // stretch of every list, about 60 MB in all, line after line; with all chunks of a 100
 // M-entry batch at work at once half-filled lines went to memory (2.28 ms against 1.26).
 // Above it only where the per-tile counts (a row of the frame's tiles per chunk) would
-// take more than BIN_MAX_COUNTS. tiles: the view's, in a batch the largest view's. How
-// many chunks a view uses depends on its intersections (BIN_MIN_ENTRIES).
+// take more than BIN_MAX_COUNTS. tiles: the view's, in a batch the largest view's. A view
+// uses fewer chunks where they would hold less than BIN_MIN_ENTRIES intersections.
 constexpr int64_t BIN_MAX_COUNTS = 1 << 26;
 int bin_chunk_len(int64_t n, int64_t tiles) {
-    const int64_t len = std::min<int64_t>(2048, std::max<int64_t>(64, (n + 591) / 592));
+    const int64_t len = std::min<int64_t>(2048, std::max<int64_t>(64, (n + GPU_PLACES - 1) / GPU_PLACES));
     return (int)std::min<int64_t>(INT32_MAX, std::max(len, (n * tiles + BIN_MAX_COUNTS - 1) / BIN_MAX_COUNTS));
 }
 int bin_chunks(int n, int len) { return (int)(((int64_t)n + len - 1) / len); }
@@ -578,7 +579,7 @@ void bin_plan(BinArgs &a) {
     a.win_rows = BIN_MAX_TILES;
     a.grid_y = 2;
     if (a.d.n_views > 0) return;
-    const int split = std::min(8, std::max(1, 592 / std::max(1, a.chunks)));
+    const int split = std::min(8, std::max(1, GPU_PLACES / std::max(1, a.chunks)));
     if (split > 1) a.win_rows = std::max(BIN_WARPS, (a.tiles_y + split - 1) / split);
     const int w = std::min(a.tiles_x, BIN_MAX_TILES), h = std::max(1, std::min(BIN_MAX_TILES / w, a.win_rows));
     a.grid_y = std::min(8, ((a.tiles_x + w - 1) / w) * ((a.tiles_y + h - 1) / h));

@@ -401,7 +401,7 @@ int forward_batch(msplat_cuda_ctx *ctx, int nv, const msplat_cuda_view *views) {
         pa.n_tiles = n_tiles;
         pa.depth_keys = ds.keys[0];
         pa.depth_vals = ds.vals[0];
-            h_inst[v] = io;
+        h_inst[v] = io;
         h_toff[v] = to;
         h_tx[v] = tx;
         h_ty[v] = ty;

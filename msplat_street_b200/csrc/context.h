@@ -309,12 +309,6 @@ inline int ensure(Buf &b, size_t count, T **out) {
     type *var = nullptr;              \
     if (int _r = ensure<type>(buf, (size_t)(count), &var)) return _r;
 
-inline int ceil_log2(int v) {
-    int b = 0;
-    while ((1 << b) < v) b++;
-    return b;
-}
-
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 int check_camera(int num_points, unsigned H, unsigned W, int tx, int ty, unsigned degree, unsigned dtu,

@@ -44,7 +44,7 @@ template <typename TO>
 void scan_exclusive(const int32_t *in, TO *out, int n, TO *d_total, TO *partials, cudaStream_t st);
 
 size_t radix_scratch_bytes(int n);
-// d_n / d_T (optional): device-side counts capping the host-side capacities n / T
+// d_n (optional): a device-side count capping the host-side capacity n
 int radix_sort_pairs(uint64_t *k[2], uint32_t *v[2], int n, int key_bits, void *scratch, cudaStream_t st,
                      const int *d_n = nullptr);
 int radix_sort_pairs32(uint32_t *k[2], uint32_t *v[2], int n, int key_bits, void *scratch, cudaStream_t st,
@@ -183,9 +183,12 @@ struct BinArgs {
     int32_t *tile_start, *tile_end;
     int32_t *tile_order;  // single views, may be null: the tiles, longest lists first
 };
-// A frame of more tiles than the GPU holds blocks of the rasterizers (148 SMs x 4), and
-// of no more than the scan of the list starts takes in one round, has its tiles ordered.
-constexpr int BIN_ORDER_MIN = 592, BIN_ORDER_MAX = 8192;
+// Four blocks on each of the 148 SMs: whole-tile blocks of the rasterizers that run at a
+// time.
+constexpr int GPU_PLACES = 4 * 148;
+// A frame of more tiles than that, and of no more than the scan of the list starts takes
+// in one round, has its tiles ordered.
+constexpr int BIN_ORDER_MIN = GPU_PLACES, BIN_ORDER_MAX = 8192;
 int bin_chunk_len(int64_t n, int64_t tiles);
 int bin_chunks(int n, int len);
 void bin_plan(BinArgs &a);

@@ -176,14 +176,12 @@ constexpr int RADIX = 256;
 // Keys per block: THREADS x ITEMS. Large sorts of 32-bit keys take 256 threads x 16
 // items (4096 keys a block): each digit's run in a block then averages 16 entries, so
 // the scatter's stores come in runs of 64 bytes or more, and the per-block digit counts
-// (256 per block, scanned every pass) stay small next to the keys. Below LARGE_SORT
-// keys, 256 x 8 (2048 keys a block) keeps enough blocks to fill the GPU; 64-bit keys
-// take 2048-key blocks too (4096 would need 48 KB of staging per block). Measured and
-// not kept: 512 x 8 and 1024 x 4 blocks for the large 32-bit sort (two and one blocks
-// per SM: a sort of 46 M keys of 13 bits 1.06 and 1.51 ms against 1.02), and
-// the largest shared-memory carveout (1.06 ms: the scatter's loads and stores want
-// the L1). The scatter is bound by its integer pipe (ALU 64 % of peak, issue 54 %):
-// the ranking's ballots, not DRAM, set its pace.
+// (256 per block, scanned every pass) stay small next to the keys. The depth order of 12
+// million instances (32 bits): histograms 70, scatters 414 and scans 138 us against 89,
+// 420 and 155 in 2048-key blocks. Below LARGE_SORT keys, 256 x 8 (2048 keys a block) keeps
+// enough blocks to fill the GPU; 64-bit keys take 2048-key blocks too (4096 would need 48
+// KB of staging per block). The scatter is bound by its integer pipe: the ranking's
+// ballots, not DRAM, set its pace.
 constexpr int SORT_THREADS = 256;
 constexpr int LARGE_SORT = 4 << 20;
 constexpr int MAX_SORT_THREADS = 1024;
@@ -197,11 +195,10 @@ constexpr int DIRECT_SORT_BLOCKS = 64;
 // the smallest of every block shape below.
 int radix_max_blocks(int n) { return (n + 2047) / 2048; }
 
-// d_n (may be null): a device-side count that caps n (capacity-bounded launches)
 // The lanes of the warp whose digit equals this lane's (d in 0..RADIX, RADIX marking
 // a lane with no key): nine ballots, one per bit of d, each narrowing the set to the
 // lanes that agree on that bit. Constant cost whatever the number of distinct digits
-// in the warp (a warp of scattered tile ids holds up to 32).
+// in the warp (up to 32).
 // Only the bits a pass's digits can hold take a ballot (mask, uniform), and the no-key
 // bit only in a block that is not full (full: every lane holds a key).
 __device__ __forceinline__ unsigned digit_peers(int d, uint32_t mask, bool full) {
@@ -219,6 +216,7 @@ __device__ __forceinline__ unsigned digit_peers(int d, uint32_t mask, bool full)
 // Counting needs no ranks: each warp adds its keys' digits to its own shared-memory
 // histogram with one atomic per key (lanes of a warp that share a digit are resolved
 // by the shared-memory atomic unit), and the block sums the warps' histograms.
+// d_n (may be null): a device-side count that caps n (capacity-bounded launches).
 template <typename K, int THREADS, int SORT_ITEMS>
 __global__ void __launch_bounds__(THREADS) radix_hist_kernel(const K *keys, int n, const int *d_n, int shift,
                                                              uint32_t mask, uint32_t *counts, int nb) {

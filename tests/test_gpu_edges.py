@@ -125,7 +125,7 @@ def test_train_step_edge(oracle, name):
 @pytest.mark.parametrize("n,scale,degree", [(1, -1.0, 3), (127, -2.0, 1), (129, -1.0, 2), (300, 0.0, 3)])
 def test_slot_sums_of_every_size(n, scale, degree):
     """Screen-space gradients (the sums of the intersection slots) of scenes whose Gaussians
-    cover from one tile to the whole 40 x 30 tile frame (sums of one lane, of eight, of a
+    cover from one tile to the whole 40 x 30 tile frame (sums of one lane, of four, of a
     warp and of the block) and whose counts lie around the backward kernel's 128-Gaussian
     blocks, against the oracle within the gradient tolerance; the batched step's parameters
     and moments are the same bits. (The world-space gradients of such needles are no
