@@ -206,7 +206,11 @@ def test_server_small_budget_evicts_and_completes():
     srv = serving.RenderServer(st, [0.0] * 3, slots=2, max_batch=4, max_batch_pixels=4 * 64 * 48,
                                keep_images=True, renderer_factory=lambda: FakeRenderer(log, delay=0.001))
     reqs = _requests(50, 5, seed=3)
-    res = srv.run(reqs, realtime=False)
+    # in two runs: at most two scenes are resident between them, so at least three of the
+    # five are uploaded again whatever order the workers take the requests in
+    first, second = reqs[:25], reqs[25:]
+    assert len({r.scene_id for r in first}) == len({r.scene_id for r in second}) == 5
+    res = srv.run(first, realtime=False) + srv.run(second, realtime=False)
     assert len(res) == 50 and st.evictions > 0 and st.uploads > 5
     for r in res:
         assert torch.all(r.image == 20_000.0 + r.width / 1e4)
