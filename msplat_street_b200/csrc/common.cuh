@@ -135,10 +135,11 @@ __device__ __forceinline__ float exp_span(float xf, const double *span) {
 }
 
 // The same double without a table, for the few pairs a pass evaluates so (the backward's
-// near the cut-offs, the pair counter): the span's entry computed on the spot. FAR: for x
-// down to -700, with the reduction in two steps.
+// near the cut-offs, the pair counter): the span's entry computed on the spot. Inlined:
+// as a call it cost the backward 1.5 % (an early street view 434 -> 428 us, 200 k Gaussians
+// at 1024 x 768 258 -> 252). FAR: for x down to -700, with the reduction in two steps.
 template <bool FAR = false>
-__device__ __noinline__ float exp_once(float xf) {
+__device__ __forceinline__ float exp_once(float xf) {
     const double x = (double)xf;
     double k;
     const int ki = exp_index(x, k);
