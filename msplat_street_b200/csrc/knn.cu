@@ -191,6 +191,7 @@ __device__ __forceinline__ float gap2(const Bounds &q, const float4 lo, const fl
 // A warp's search state: its 32 queries (one per lane) and their three best distances.
 struct KnnSearch {
     const float4 *sp;
+    float4 *pts;  // shared memory of this warp: the points of the box being scanned
     int n;
     float4 q;
     uint32_t self;
@@ -209,13 +210,20 @@ struct KnnSearch {
         const float4 lo = mn[i], hi = mx[i];
         return lo.x <= hi.x && gap2(qb, lo, hi) < thr;
     }
-    // box c's points against every query; the loads are the same on every lane
-    __device__ __forceinline__ void scan_box(int c) {
+    // the lane's point of box c (none: a distance that is no number)
+    __device__ __forceinline__ float4 load_box(int c) const {
+        const int j = c * KNN_BOX + (threadIdx.x & 31);
+        return j < n ? sp[j] : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
+    }
+    // a box's points, a lane's each, against every query
+    __device__ __forceinline__ void scan_box(const float4 mine) {
         boxes++;
-        const int j0 = c * KNN_BOX, cnt = min(KNN_BOX, n - j0);
+        __syncwarp();  // the box before is read
+        pts[threadIdx.x & 31] = mine;
+        __syncwarp();
 #pragma unroll 8
-        for (int k = 0; k < cnt; k++) {
-            const float4 p = sp[j0 + k];
+        for (int k = 0; k < KNN_BOX; k++) {
+            const float4 p = pts[k];
             const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
             const float d = dx * dx + dy * dy + dz * dz;
             if (d < b2 && fin && __float_as_uint(p.w) != self) keep3(d, b0, b1, b2);
@@ -231,7 +239,7 @@ struct KnnSearch {
             m &= m - 1;
             const float4 lo = bmin[cb], hi = bmax[cb];
             const Bounds me{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
-            if (__ballot_sync(0xffffffffu, fin && gap2(me, lo, hi) < b2)) scan_box(cb);
+            if (__ballot_sync(0xffffffffu, fin && gap2(me, lo, hi) < b2)) scan_box(load_box(cb));
         }
     }
 };
@@ -240,9 +248,14 @@ struct KnnSearch {
 // box it reads) -- the search's work, for throughput reports.
 //
 // Bound by instruction issue: about 12 instructions a point of a box that is read. A
-// 400 k-point cloud: 4.34 -> 0.56 ms against the form in which every warp tested all
+// 400 k-point cloud: 4.34 -> 0.39 ms against the form in which every warp tested all
 // 12.5 k boxes, 32 at a time, and read all that passed the first test; the descent
-// through groups and supergroups leaves a few dozen node tests a warp.
+// through groups and supergroups leaves a few dozen node tests a warp. A box comes in one
+// load, a point a lane, and is read from shared memory: with a load a point, the same on
+// every lane, each box cost four cache misses one after another (0.56 ms; one outlier far
+// from 20 k points, which puts them all into one Morton cell, 2.46 against 1.01, and 1.41
+// in the form before). Loading the next box ahead reads many that the second test drops:
+// 0.58.
 __global__ void __launch_bounds__(128) knn_query_kernel(const float4 *sp, int n, int nboxes, const float4 *bmin,
                                                         const float4 *bmax, int ngroups, const float4 *gmin,
                                                         const float4 *gmax, int nsuper, const float4 *smin,
@@ -253,7 +266,9 @@ __global__ void __launch_bounds__(128) knn_query_kernel(const float4 *sp, int n,
     const int j = own * KNN_BOX + lane;
     const bool valid = j < n;
     KnnSearch s;
+    __shared__ float4 pts[128 / 32][KNN_BOX];
     s.sp = sp;
+    s.pts = pts[threadIdx.x >> 5];
     s.n = n;
     s.q = valid ? sp[j] : make_float4(0.f, 0.f, 0.f, 0.f);
     s.self = __float_as_uint(s.q.w);
@@ -270,7 +285,7 @@ __global__ void __launch_bounds__(128) knn_query_kernel(const float4 *sp, int n,
     const unsigned nq = __popc(__ballot_sync(0xffffffffu, s.fin));
     if (nq) {  // warp-uniform
         const int og = own / KNN_BOX, os = og / KNN_BOX;
-        s.scan_box(own);
+        s.scan_box(s.load_box(own));
         s.scan_group(og, own, bmin, bmax, nboxes);
         // supergroup 0 of the walk is the warp's own, then the others in order
         for (int i0 = 0; i0 < nsuper; i0 += 32) {

@@ -93,6 +93,15 @@ def test_gpu_knn_search_levels(n):
     np.testing.assert_array_equal(_core._gpu_knn3_mean_dist(pts), Oracle("restatement").knn3_mean_dist(pts))
 
 
+@pytest.mark.parametrize("n", [31, 32, 2001])
+def test_gpu_knn_in_one_cell(n):
+    """Points that one outlier puts into a single cell of the Morton order, so that every box
+    overlaps every other: the oracle's values."""
+    pts = np.random.default_rng(n).uniform(0, 1, (n, 3)).astype(np.float32)
+    pts[n // 2] = 1e4
+    np.testing.assert_array_equal(_core._gpu_knn3_mean_dist(pts), Oracle("restatement").knn3_mean_dist(pts))
+
+
 def _f32_ulps(a, b):
     ia = np.asarray(a, np.float32).view(np.int32).astype(np.int64)
     ib = np.asarray(b, np.float32).view(np.int32).astype(np.int64)
