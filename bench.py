@@ -748,11 +748,11 @@ class TargetPrefetch:
 
 def launches_per_step(n_gauss: float = 1e5) -> float:
     """Kernels one plain training step launches: project, the depth sort (one cluster
-    launch up to 65,536 Gaussians, else 4 passes of hist + scatter, plus a 3-kernel scan
+    launch up to 20,480 Gaussians, else 4 passes of hist + scatter, plus a 3-kernel scan
     per pass above 131,072), tile rectangles, the scan of their counts (3 kernels, one up
     to 16,384 Gaussians), the binning's count, prefix, list starts and emission, raster
     forward, SSIM, loss finalize, raster backward, backward/Adam."""
-    depth_sort = 1 if n_gauss <= 65536 else 4 * (2 if n_gauss <= 131072 else 5)
+    depth_sort = 1 if n_gauss <= 20480 else 4 * (2 if n_gauss <= 131072 else 5)
     scan = 1 if n_gauss <= 16384 else 3
     return 1 + depth_sort + 1 + scan + 4 + 1 + 1 + 1 + 1 + 1
 

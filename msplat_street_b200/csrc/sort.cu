@@ -357,9 +357,11 @@ __global__ void __launch_bounds__(THREADS, sizeof(K) == 8 ? 1024 / THREADS : 512
 // all the passes. A block ranks its part as the scatter does, the blocks exchange their
 // digit counts, and every key goes straight to its place in the shared memory of the
 // block that holds it next. In place; one launch where the histogram and scatter kernels
-// take two a pass, few blocks each: 10 k keys of 32 bits, 30 -> 21 us.
+// take two a pass, few blocks each. The cluster's time grows with the keys, theirs does
+// not while their blocks find SMs free: 10 k keys of 32 bits 30 -> 20 us, 17 k 31 -> 28, 20 k
+// 31 -> 30; but 24 k 31 -> 33, 40 k 33 -> 50 and 65 k 47 -> 69, so it ends at 20,480.
 constexpr int CLUSTER_BLOCKS = 8, CLUSTER_THREADS = 1024;
-constexpr int CLUSTER_MAX_ITEMS = 8, CLUSTER_SORT = CLUSTER_BLOCKS * CLUSTER_THREADS * CLUSTER_MAX_ITEMS;
+constexpr int CLUSTER_SORT = CLUSTER_BLOCKS * CLUSTER_THREADS * 5 / 2;
 
 // per: keys a block holds, a multiple of 32, at most CLUSTER_THREADS * KEYS.
 template <int KEYS>
@@ -476,8 +478,7 @@ void radix_cluster_launch(uint32_t *keys, uint32_t *vals, int n, int key_bits, i
 void radix_cluster_sort(uint32_t *keys, uint32_t *vals, int n, int key_bits, cudaStream_t st) {
     const int per = ((n + CLUSTER_BLOCKS - 1) / CLUSTER_BLOCKS + 31) / 32 * 32;
     if (per <= CLUSTER_THREADS * 2) radix_cluster_launch<2>(keys, vals, n, key_bits, per, st);
-    else if (per <= CLUSTER_THREADS * 4) radix_cluster_launch<4>(keys, vals, n, key_bits, per, st);
-    else radix_cluster_launch<CLUSTER_MAX_ITEMS>(keys, vals, n, key_bits, per, st);
+    else radix_cluster_launch<4>(keys, vals, n, key_bits, per, st);  // CLUSTER_SORT's at most
 }
 
 template <typename K, int THREADS, int ITEMS>

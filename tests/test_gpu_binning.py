@@ -64,11 +64,11 @@ def test_lists_match_the_rectangles(n, w, h, scale):
     assert torch.equal(batch[0], img)
 
 
-@pytest.mark.parametrize("n", [33, 2049, 16_384, 16_385, 32_800, 65_536, 65_537, 300_000])
+@pytest.mark.parametrize("n", [33, 2049, 16_384, 16_385, 20_480, 20_481, 32_800, 65_536, 65_537, 300_000])
 def test_equal_depths_keep_index_order(n):
     """Five distinct depths, so that nearly every neighbour in the depth order is a tie,
-    at the sizes where the depth sort changes form (one cluster of blocks, with two, four
-    and eight keys a thread, up to 65,536; several launches a digit beyond)."""
+    at the sizes where the depth sort changes form (one cluster of blocks, with two and
+    four keys a thread, up to 20,480; several launches a digit beyond)."""
     rng = np.random.default_rng(n)
     g = scenes.random_gaussians(n, n, log_scale_mean=-4.5)
     g.means[:, 2] = rng.integers(0, 5, n).astype(np.float32) * 0.25
