@@ -190,9 +190,13 @@ __device__ __forceinline__ bool list_instances(VisibleList<NB> &L, int64_t g0, i
 // in L2), about a microsecond. A Gaussian of up to SLOT_LANE_MAX tiles is one lane's; of
 // up to SLOT_SERIAL, four neighbouring lanes', which share out its values (two or three
 // each) and fetch SLOT_AHEAD slots before they add any; of up to SLOT_WARP_MAX, a warp's,
-// and of more the block's, whose warps share out the values. One lane walking its
-// Gaussian's slots alone (34 on average in an early street view) and one warp walking the
-// 2000 of a Gaussian in front of the camera were most of the kernel's time.
+// and of more a warp's too where there is one for every warp, the rest the block's, whose
+// warps share out the values. One lane walking its Gaussian's slots alone (34 on average
+// in an early street view) and one warp walking the 2000 of a single Gaussian in front of
+// the camera were most of the kernel's time; but blocks full of large Gaussians are bound
+// by the slots' sectors, which warps that share out the values read four times: 4000
+// Gaussians of 2700 tiles each 2.80 -> 1.64 ms (2.22 with one thread a Gaussian), 300 of
+// 5300 3.63 -> 2.04 (3.02), an early street view 66 -> 60 us.
 constexpr int SLOT_LANE_MAX = 8, SLOT_SERIAL = 64, SLOT_WARP_MAX = 256, SLOT_AHEAD = 8;
 
 // All values of the slots first, first + step, ... of cnt, two slots fetched at a time.
@@ -287,8 +291,9 @@ __device__ __forceinline__ void sum_slots(VisibleList<NB> &L, const int32_t *inv
         L.store_share(i, part, p);
     }
     __syncwarp();
-    for (int li = warp; li < L.n_wide; li += NB / 32) {  // warp-uniform
-        const int i = L.wide[li];
+    const int whole = L.n_large / (NB / 32) * (NB / 32);  // large ones that keep every warp busy alone
+    for (int li = warp; li < L.n_wide + whole; li += NB / 32) {  // warp-uniform
+        const int i = li < whole ? L.large[li] : L.wide[li - whole];
         add_slots(lane, 32, inv + L.first[i], L.tiles[i], slots, slots_depth, p, pd);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -298,7 +303,7 @@ __device__ __forceinline__ void sum_slots(VisibleList<NB> &L, const int32_t *inv
         }
         if (lane == 0) L.store(i, p, pd);
     }
-    for (int q = 0; q < L.n_large; q++) {  // block-uniform
+    for (int q = whole; q < L.n_large; q++) {  // block-uniform
         const int i = L.large[q];
         add_share(warp, lane, 32, inv + L.first[i], L.tiles[i], slots, slots_depth, p);
 #pragma unroll
