@@ -313,56 +313,114 @@ __device__ __forceinline__ int lower_bound_u32(const uint32_t *keys, int n, uint
     return lo;
 }
 
-// One warp per texel: its contributions summed in sorted (= pixel, tap) order, then
-// Adam on its three channels (the reference's Adam runs over the whole texture,
-// :959-963). A texel in view collects hundreds of contributions, each two gathers away;
-// the lanes fetch SKY_CHUNK of them at a time and leave their products in shared
-// memory, where lane c adds channel c's in order. One thread a texel took 714 us for a
-// 256 x 128 texture behind a 1000 x 500 view (two thousand texels in view, a thousand
-// contributions each, one dependent load after another); 56 us now.
+// A texel's contributions summed in sorted (= pixel, tap) order, then Adam on its three
+// channels (the reference's Adam runs over the whole texture, :959-963). A block takes PER
+// texels.
+//
+// Where the texture is coarse next to the image (PER = SKY_WARPS), a texel in view
+// collects hundreds of contributions, each two gathers away: it is a warp's, whose lanes
+// fetch SKY_CHUNK of them at a time and leave their products in shared memory, where lane
+// c adds channel c's in order. One thread a texel took 714 us for a 256 x 128 texture
+// behind a 1000 x 500 view (two thousand texels in view, a thousand contributions each,
+// one dependent load after another); 56 us now. Where it is fine (PER = SKY_TEXELS), most
+// texels have none or a few: each is a thread's, and the block's warps share out those of
+// more than SKY_LIGHT.
 constexpr int SKY_WARPS = 8, SKY_CHUNK = 128, SKY_PITCH = SKY_CHUNK + 1;
+constexpr int SKY_TEXELS = 32 * SKY_WARPS, SKY_LIGHT = 32;
 
-__global__ void __launch_bounds__(32 * SKY_WARPS) sky_texel_adam_kernel(const uint32_t *keys, const uint32_t *vals,
-                                                                        const int32_t *d_n, int n_texels,
-                                                                        const float4 *tap_w, const float4 *tap_g,
-                                                                        SkyAdamArgs a) {
-    __shared__ float buf[SKY_WARPS][3 * SKY_PITCH];
-    __shared__ int first[SKY_WARPS + 1];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x <= SKY_WARPS)
-        first[threadIdx.x] = lower_bound_u32(keys, *d_n, (uint32_t)(blockIdx.x * SKY_WARPS + threadIdx.x));
-    __syncthreads();
-    const int t = blockIdx.x * SKY_WARPS + warp;
-    if (t >= n_texels) return;  // warp-uniform; no block barrier below
-    float s = 0.f;              // lane c < 3: channel c's sum
-    const int hi = first[warp + 1];
-    for (int e0 = first[warp]; e0 < hi; e0 += SKY_CHUNK) {  // warp-uniform
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < SKY_CHUNK / 32; u++) {
-            const int e = e0 + u * 32 + lane;
-            if (e >= hi) continue;
-            const uint32_t v = vals[e];
-            const uint32_t pix = v >> 2, k = v & 3u;
-            const float4 w4 = tap_w[pix];
-            const float w = k == 0 ? w4.x : (k == 1 ? w4.y : (k == 2 ? w4.z : w4.w));
-            const float4 g = tap_g[pix];
-            buf[warp][u * 32 + lane] = w * g.x;
-            buf[warp][SKY_PITCH + u * 32 + lane] = w * g.y;
-            buf[warp][2 * SKY_PITCH + u * 32 + lane] = w * g.z;
-        }
-        __syncwarp();
-        if (lane < 3) {
-            const float *b = buf[warp] + lane * SKY_PITCH;
-            const int cnt = min(SKY_CHUNK, hi - e0);
-#pragma unroll 16
-            for (int j = 0; j < cnt; j++) s += b[j];
-        }
-    }
-    if (lane >= 3) return;
-    const size_t i = 3 * (size_t)t + lane;
+__device__ __forceinline__ Raw3 sky_contribution(uint32_t v, const float4 *tap_w, const float4 *tap_g) {
+    const uint32_t pix = v >> 2, k = v & 3u;
+    const float4 w4 = tap_w[pix];
+    const float w = k == 0 ? w4.x : (k == 1 ? w4.y : (k == 2 ? w4.z : w4.w));
+    const float4 g = tap_g[pix];
+    return Raw3{{w * g.x, w * g.y, w * g.z}};
+}
+
+__device__ __forceinline__ void sky_adam(const SkyAdamArgs &a, size_t i, float s) {
     a.grad[i] = s;
     adam_step(a.tex[i], a.exp_avg[i], a.exp_avg_sq[i], s, a.step_size, a.beta1, a.beta2, a.bc2, a.eps);
+}
+
+// With SKY_TEXELS texels a block has a warp more, whose first thread finds where the last
+// texel's contributions end.
+template <int PER>
+constexpr int SKY_THREADS = 32 * SKY_WARPS + (PER > SKY_WARPS ? 32 : 0);
+
+template <int PER>
+__global__ void __launch_bounds__(SKY_THREADS<PER>) sky_texel_adam_kernel(const uint32_t *keys, const uint32_t *vals,
+                                                                          const int32_t *d_n, int n_texels,
+                                                                          const float4 *tap_w, const float4 *tap_g,
+                                                                          SkyAdamArgs a) {
+    constexpr bool FINE = PER > SKY_WARPS;
+    static_assert(PER == SKY_WARPS || PER == SKY_TEXELS, "a warp or a thread a texel");
+    __shared__ float buf[SKY_WARPS][3 * SKY_PITCH];
+    __shared__ int first[PER + 1];
+    __shared__ int n_heavy;
+    __shared__ uint16_t heavy[FINE ? PER : 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = blockIdx.x * PER;
+    if (threadIdx.x <= PER) first[threadIdx.x] = lower_bound_u32(keys, *d_n, (uint32_t)(t0 + threadIdx.x));
+    if (threadIdx.x == 0) n_heavy = 0;
+    __syncthreads();
+    if constexpr (FINE) {
+        const int t = t0 + threadIdx.x;
+        if (threadIdx.x < PER && t < n_texels) {
+            const int lo = first[threadIdx.x], hi = first[threadIdx.x + 1];
+            if (hi - lo > SKY_LIGHT) {
+                heavy[atomicAdd(&n_heavy, 1)] = (uint16_t)threadIdx.x;
+            } else {
+                float s[3] = {0.f, 0.f, 0.f};
+                for (int e = lo; e < hi; e++) {
+                    const Raw3 r = sky_contribution(vals[e], tap_w, tap_g);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) s[c] += r.v[c];
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) sky_adam(a, 3 * (size_t)t + c, s[c]);
+            }
+        }
+        __syncthreads();
+    }
+    if (warp >= SKY_WARPS) return;  // no block barrier below
+    const int items = FINE ? n_heavy : min(PER, n_texels - t0);
+    for (int li = warp; li < items; li += SKY_WARPS) {  // warp-uniform
+        const int q = FINE ? heavy[li] : li, hi = first[q + 1];
+        float s = 0.f;  // lane c < 3: channel c's sum
+        for (int e0 = first[q]; e0 < hi; e0 += SKY_CHUNK) {  // warp-uniform
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < SKY_CHUNK / 32; u++) {
+                const int e = e0 + u * 32 + lane;
+                if (e >= hi) continue;
+                const Raw3 r = sky_contribution(vals[e], tap_w, tap_g);
+#pragma unroll
+                for (int c = 0; c < 3; c++) buf[warp][c * SKY_PITCH + u * 32 + lane] = r.v[c];
+            }
+            __syncwarp();
+            if (lane < 3) {
+                const float *b = buf[warp] + lane * SKY_PITCH;
+                const int cnt = min(SKY_CHUNK, hi - e0);
+#pragma unroll 16
+                for (int j = 0; j < cnt; j++) s += b[j];
+            }
+        }
+        if (lane < 3) sky_adam(a, 3 * (size_t)(t0 + q) + lane, s);
+    }
+}
+
+// Whether a texture of n_texels is fine next to an image of taps / 4 pixels. A warp a texel
+// costs 0.41 us a thousand texels whether they are seen or not, a thread a texel the
+// contributions of the ones that are; the two meet at a texel count that grows with the
+// square root of the taps: behind 500 x 250 at 131 k texels (54 and 55 us; 245 k: 92 and 43),
+// behind 1000 x 500 at 250 k (245 k: 110 and 104; 524 k: 217 and 84; 131 k: 66 and 124),
+// behind 1920 x 1080 above 245 k (156 and 384) and below 524 k (281 and 204). A texture of
+// 2048 x 1024 behind 1000 x 500 took 810 us with a warp a texel, 79 now.
+inline bool sky_fine(int64_t n_texels, int64_t taps) { return n_texels * n_texels > taps * 32768; }
+
+template <int PER>
+void sky_texel_adam(const uint32_t *keys, const uint32_t *vals, int n_texels, const SkyScratch &sc,
+                    const SkyAdamArgs &a, cudaStream_t st) {
+    sky_texel_adam_kernel<PER><<<(n_texels + PER - 1) / PER, SKY_THREADS<PER>, 0, st>>>(keys, vals, sc.d_total, n_texels,
+                                                                                       sc.tap_w, sc.tap_g, a);
 }
 
 }  // namespace
@@ -418,8 +476,8 @@ void launch_sky_backward_adam(const SkyArgs &s, int W, int H, const float *final
     while ((1 << bits) < n_texels) bits++;
     const int cur = radix_sort_pairs32(kk, vv, (int)std::max<int64_t>(4 * npix, 1), std::max(bits, 1),
                                        sc.radix_scratch, st, sc.d_total);
-    sky_texel_adam_kernel<<<(n_texels + SKY_WARPS - 1) / SKY_WARPS, 32 * SKY_WARPS, 0, st>>>(kk[cur], vv[cur], sc.d_total, n_texels, sc.tap_w,
-                                                                   sc.tap_g, a);
+    if (sky_fine(n_texels, 4 * npix)) sky_texel_adam<SKY_TEXELS>(kk[cur], vv[cur], n_texels, sc, a, st);
+    else sky_texel_adam<SKY_WARPS>(kk[cur], vv[cur], n_texels, sc, a, st);
 }
 
 __global__ void needle_cap_kernel(float *scales, int n, float log_max) {

@@ -144,11 +144,11 @@ def test_train_step_with_prior(oracle, modes):
     set_prior(oracle, None)
 
 
-@pytest.mark.parametrize("sky_w,sky_h", [(5, 3), (4, 2), (9, 7), (130, 33)])
+@pytest.mark.parametrize("sky_w,sky_h", [(5, 3), (4, 2), (9, 7), (130, 33), (248, 187), (250, 187), (811, 400)])
 def test_sky_gradient_texture_sizes(oracle, sky_w, sky_h):
-    """Textures whose texel counts are no multiple of a block's eight, from a few texels
-    with thousands of contributions each to texels with a handful, against the oracle
-    with the tolerances of the other sky tests."""
+    """Textures whose texel counts are no multiple of a block's eight or 256, from a few texels
+    with thousands of contributions each to texels with a handful or none, against the
+    oracle with the tolerances of the other sky tests."""
     g, cam = _scene(), _camera()
     set_prior(oracle, None)
     gt = oracle.render(scenes.random_gaussians(3000, 51, sh_degree=2), cam, BACKGROUND)
