@@ -288,17 +288,11 @@ constexpr int SCAN_THREADS = 1024, SCAN_PER = 8;
 // length of their lists, the longest first, so that the last blocks to start are short
 // ones (a tile of the frame's last rows may hold its longest list). A counting sort over
 // eighths of each power of two; tiles of one step in no particular order, which changes
-// no tile's result. It costs 2.5 to 5 us and pays where lists are short: forward and
-// backward of 50 k to 200 k Gaussians at 512 x 512 to 1920 x 1080 (220 to 440 entries a
-// tile on average) gain 8 to 60 us of 250 to 680, 500 k of a street at 1024 x 512 4 to 48
-// of 240 to 450. Where lists are long and opaque, pixels are done before their lists' ends,
-// length no longer measures a tile's work, and neighbouring tiles, whose splats a cache
-// holds, are torn apart: of ball views those of 560 entries a tile gained 16 to -5 us, of
-// 730 to 870 26 to -29, of 1100 to 1750 20 to -67, of 3800 -6 to -107; early street steps
-// of 570 to 800, nearly transparent, gain 1 to 3 % of the step all the same. So a frame of
-// more than ORDER_MAX_LIST entries a tile on average is not ordered (tile_ordered; the
-// host decides by the same rule once it knows the count). Frames of up to BIN_ORDER_MIN
-// tiles start them all at once: ordering them made a 256 x 256 step 1.5 % slower.
+// no tile's result. It costs 2.6 us for 2048 tiles; ball views at 1024 x 768 composite in
+// 120 instead of 132 us and their backward in 222 instead of 267 where the long lists come
+// late. Street steps at 1024 x 512 gain 3 % (852 -> 824 us), renders there 2.5 %; at 1600 x
+// 1060, eight rounds of blocks, nothing either way. Frames of up to BIN_ORDER_MIN tiles
+// start them all at once: ordering them made a 256 x 256 step 1.5 % slower.
 constexpr int ORDER_STEPS = 256;
 static_assert(BIN_ORDER_MAX <= SCAN_THREADS * SCAN_PER, "one round");
 
@@ -308,7 +302,7 @@ __device__ __forceinline__ int order_step(int len) {
 
 template <bool ORDER>
 __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(int T, int32_t *tile_start, int32_t *tile_end,
-                                                                  int32_t *order, const int64_t *total) {
+                                                                  int32_t *order) {
     __shared__ long long ws[32];
     __shared__ int step[ORDER ? ORDER_STEPS : 1], wsum[ORDER_STEPS / 32];
     if (ORDER && threadIdx.x < ORDER_STEPS) step[threadIdx.x] = 0;  // read after the scan's barriers
@@ -369,7 +363,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(int T, int32_t
         }
         carry += all;
         __syncthreads();
-        if (!ORDER || !tile_ordered(*total, T)) continue;  // block-uniform
+        if constexpr (!ORDER) continue;
 #pragma unroll
         for (int j = 0; j < SCAN_PER; j++) {
             v[j] = i0 + j < T ? order_step(v[j] - first[j]) : -1;
@@ -628,8 +622,8 @@ void launch_bin_count(const BinArgs &a, int64_t *offsets, cudaStream_t st) {
     const int blocks = (a.tile_cap + 31) / 32;
     if (batch) bin_prefix_kernel<true><<<blocks, BIN_THREADS, 0, st>>>(a);
     else bin_prefix_kernel<false><<<blocks, BIN_THREADS, 0, st>>>(a);
-    if (a.tile_order) bin_starts_kernel<true><<<1, SCAN_THREADS, 0, st>>>(a.tile_cap, a.tile_start, a.tile_end, a.tile_order, a.total);
-    else bin_starts_kernel<false><<<1, SCAN_THREADS, 0, st>>>(a.tile_cap, a.tile_start, a.tile_end, nullptr, nullptr);
+    if (a.tile_order) bin_starts_kernel<true><<<1, SCAN_THREADS, 0, st>>>(a.tile_cap, a.tile_start, a.tile_end, a.tile_order);
+    else bin_starts_kernel<false><<<1, SCAN_THREADS, 0, st>>>(a.tile_cap, a.tile_start, a.tile_end, nullptr);
 }
 
 void launch_bin_emit(const BinArgs &a, int32_t *gids, int32_t *inv, int64_t cap, cudaStream_t st) {

@@ -231,7 +231,6 @@ int forward(msplat_cuda_ctx *ctx, int n, const float *means, const float *scales
     ENSURE(ctx->isect_gid, n_isect, int32_t, isect_gid);
     ENSURE(ctx->inv, n_isect, int32_t, inv);
     if (!emitted) launch_bin_emit(ba, isect_gid, inv, n_isect, st);
-    if (!tile_ordered(n_isect, T)) tile_order = nullptr;
 
     RasterArgs ra{};
     ra.W = (int)cam.width;

@@ -181,17 +181,14 @@ struct BinArgs {
     int2 *bounds;             // per chunk: its positions
     int32_t *counts;          // per chunk, the tiles of its view
     int32_t *tile_start, *tile_end;
-    int32_t *tile_order;  // single views, may be null: the tiles, longest lists first (tile_ordered)
+    int32_t *tile_order;  // single views, may be null: the tiles, longest lists first
 };
 // Four blocks on each of the 148 SMs: whole-tile blocks of the rasterizers that run at a
 // time.
 constexpr int GPU_PLACES = 4 * 148;
-// A frame of more tiles than that, of no more than the scan of the list starts takes in one
-// round, and of lists that are not long, has its tiles ordered.
-constexpr int BIN_ORDER_MIN = GPU_PLACES, BIN_ORDER_MAX = 8192, ORDER_MAX_LIST = 1024;
-__host__ __device__ inline bool tile_ordered(int64_t entries, int tiles) {
-    return tiles > BIN_ORDER_MIN && tiles <= BIN_ORDER_MAX && entries <= (int64_t)ORDER_MAX_LIST * tiles;
-}
+// A frame of more tiles than that, and of no more than the scan of the list starts takes
+// in one round, has its tiles ordered.
+constexpr int BIN_ORDER_MIN = GPU_PLACES, BIN_ORDER_MAX = 8192;
 int bin_chunk_len(int64_t n, int64_t tiles);
 int bin_chunks(int n, int len);
 void bin_plan(BinArgs &a);
