@@ -44,6 +44,33 @@ def test_failed_allocation_leaves_no_frame():
         assert counts == 0 and launched == [], k
 
 
+def _batch_fails_at_every_allocation(cuda):
+    """The same with a batch of two larger views after the frame."""
+    k, seen = 0, []
+    while True:
+        ctx = cuda.context()
+        cuda.allocs_left(-1)
+        cuda.readback(5000)
+        assert cuda.render(ctx, N, W, H) == 0
+        cuda.readback(50_000_000)
+        cuda.allocs_left(k)
+        status = cuda.render_batch(ctx, 2, 20 * N, 2 * W, 2 * H)
+        cuda.allocs_left(-1)
+        cuda.launches()
+        seen.append((status, cuda.render_backward(ctx, N, W, H), cuda.pair_counts(ctx), _frame_kernels(cuda)))
+        cuda.lib.msplat_cuda_ctx_destroy(ctx)
+        if status == 0:
+            return seen
+        k += 1
+
+
+def test_failed_batch_leaves_no_frame():
+    seen = fake_cuda.run(_batch_fails_at_every_allocation)
+    assert len(seen) > 10 and seen[-1][0] == 0
+    for k, (_, after, counts, launched) in enumerate(seen):
+        assert (after, counts, launched) == (1, 0, []), k
+
+
 def _too_many_entries(cuda, w, h):
     ctx = cuda.context()
     cuda.readback(5000)
