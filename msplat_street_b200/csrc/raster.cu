@@ -120,8 +120,8 @@ __device__ __forceinline__ float sigma_cut(float o) { return fminf(logf(255.f * 
 //
 // Measured and not kept: each splat's terms of sigma per column and per row of the tile
 // in place of its centre and conic (three operations and two loads a visit for sigma
-// instead of eleven and one, 42 more stores a splat and 47 KB a block). Against these
-// blocks it lost in every frame and batch tried, from 300 to 14400 tiles and 120 to 6500
+// instead of eleven and one, 32 more pairs to stage a splat and 47 KB a block). Against
+// these blocks it won in no frame or batch tried, from 300 to 14400 tiles and 120 to 6500
 // entries a tile: 100 k to 3 M Gaussians at 1024 x 768 2 to 5 %, 580 to 700 tiles 2 to 8 %,
 // an early street step 0.1 %, batches 1 to 3 %.
 template <int FB>
