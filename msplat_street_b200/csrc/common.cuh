@@ -6,8 +6,9 @@
 // depth keys and the alpha / transmittance cut-offs. To that end
 //  * the translation units that compute them are compiled with -fmad=false, so every
 //    a*b+c stays two rounded operations, in the reference's order;
-//  * exponentials use exp_ref(): exp evaluated in double and rounded once to float,
-//    which agrees with a correctly rounded expf except in rare near-halfway cases;
+//  * exponentials are evaluated in double and rounded once to float: exp_ref(), which
+//    agrees with a correctly rounded expf except in rare near-halfway cases, and the
+//    table methods below, which are correctly rounded;
 //  * division and square root are IEEE (nvcc's default -prec-div / -prec-sqrt).
 // Matrices are column-major (c[col] is a column) because the reference's helper
 // types follow MSL conventions (core/cpu/cpu_math.hpp:1-4).
